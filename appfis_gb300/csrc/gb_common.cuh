@@ -27,6 +27,16 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // that use the same slot on the same device must not overlap on the GPU.
 enum Slot { WS_REDUCE = 0, WS_JOB_A, WS_JOB_B, WS_JOB_C, WS_JOB_D, WS_JOB_E, WS_JOB_F, WS_LIFE_C, WS_LIFE_D, WS_LIFE_E, WS_LIFE_F, WS_FLOOD_Z, WS_FLOOD_SRC, WS_F64_PARTIALS, WS_FLOOD_MAPS, WS_SLOTS };
 int workspace(int slot, size_t bytes, void** out);
+// True if that slot holds at least `bytes` already, so that workspace() will not allocate.
+bool workspace_holds(int slot, size_t bytes);
+// Device memory for one call, ordered on `st` (allocated and freed by the stream, so calls on other
+// streams and threads never share it): from a pool per device that keeps up to 256 MB between
+// calls and gives back what is over that when the device is next synchronised.  False, with no error
+// left behind, if there is none (the caller then takes a path without it).
+bool scratch_alloc(size_t bytes, cudaStream_t st, void** out);
+void scratch_free(void* p, cudaStream_t st);
+// True while `st` records a graph (or cannot tell): a call then allocates nothing of its own.
+bool capturing(cudaStream_t st);
 // Pinned host staging buffer, grow-only, per slot (0..1).
 int pinned(int slot, size_t bytes, void** out);
 

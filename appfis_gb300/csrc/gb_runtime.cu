@@ -60,6 +60,7 @@ Buf g_pinned[2];
 std::vector<int> g_sms;
 std::vector<unsigned*> g_status;  // [device]
 std::vector<cudaStream_t> g_job_streams;  // [device]
+std::vector<cudaMemPool_t> g_pools;  // [device]
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 std::once_flag g_encode_once;
 }  // namespace
@@ -85,6 +86,49 @@ int workspace(int slot, size_t bytes, void** out)
     }
     *out = b.p;
     return APPFIS_GB_OK;
+}
+
+bool workspace_holds(int slot, size_t bytes)
+{
+    int dev = 0;
+    if (slot < 0 || slot >= WS_SLOTS || cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(g_mu);
+    return (int)g_dev.size() > dev && g_dev[dev][slot].n >= bytes;
+}
+
+bool scratch_alloc(size_t bytes, cudaStream_t st, void** out)
+{
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if ((int)g_pools.size() <= dev) g_pools.resize(dev + 1, nullptr);
+        if (!g_pools[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            uint64_t keep = 256ull << 20;
+            if (cudaMemPoolCreate(&g_pools[dev], &props) == cudaSuccess)
+                cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            else
+                g_pools[dev] = nullptr;
+        }
+        pool = g_pools[dev];
+    }
+    if (pool && cudaMallocFromPoolAsync(out, bytes, pool, st) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+void scratch_free(void* p, cudaStream_t st) { cudaFreeAsync(p, st); }
+
+bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
 }
 
 int pinned(int slot, size_t bytes, void** out)

@@ -41,7 +41,8 @@ __device__ __forceinline__ uint32_t rule_bytes(uint32_t cnt, uint32_t c, uint32_
 
 
 // ------------------------------------------------------------------------------ generic form
-// One thread per cell, any nx, ny (used when nx is not a multiple of 16).
+// One thread per cell, any nx, ny (a few generations of rows that are not whole 16-byte vectors, or of
+// a small grid).
 template <int RULE>
 __global__ void life_u8_generic(const uint8_t* __restrict__ cur, uint8_t* __restrict__ out, int nx, int ny)
 {
@@ -250,7 +251,7 @@ __device__ __forceinline__ RowBits finish_row_bits(const RawBits& raw, int xw, i
 // Warp tasks: 32 words (1024 cells) per row over LIFE_ROWS rows, grid-stride, one row prefetched.
 template <int RULE>
 __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restrict__ cur, uint32_t* __restrict__ out,
-                                                        int nw, int ny, int strips, int tasks)
+                                                        int nw, int ny, int strips, int rows, int tasks)
 {
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restric
         const int strip = task % strips, seg = task / strips;
         const int xw = strip * 32 + lane;
         const bool active = xw < nw;
-        const int j0 = seg * LIFE_ROWS, j1 = min(j0 + LIFE_ROWS, ny);
+        const int j0 = seg * rows, j1 = min(j0 + rows, ny);
         RowBits up = finish_row_bits(load_raw_bits(cur, nw, j0 == 0 ? ny - 1 : j0 - 1, xw, active, lane), xw, nw, lane);
         RowBits mid = finish_row_bits(load_raw_bits(cur, nw, j0, xw, active, lane), xw, nw, lane);
         RawBits rdn = load_raw_bits(cur, nw, j0 == ny - 1 ? 0 : j0 + 1, xw, active, lane);
@@ -282,20 +283,46 @@ __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restric
 }
 
 // ------------------------------------------------------------------------------ bit-packed, time-blocked
-// TB_STEPS generations per launch on a tile held in shared memory.  A CTA owns output words
-// [30*tx, 30*tx + 30) x rows [R*ty, R*ty + R) and loads a 32-word x (R + 2*TB_STEPS)-row region
+// Up to TB_STEPS generations per launch on a tile held in shared memory.  A CTA owns output words
+// [30*tx, 30*tx + 30) x rows [R*ty, R*ty + R) and loads a 32-word x (R + 2*steps)-row region
 // around it (periodic wrap at load time, so the region is a consistent periodic window even on
 // the grid's last tiles).  Lane 0 / 31 hold the halo words: their outer bits go stale by one
 // cell per generation, which never reaches the output words for up to 31 generations; rows go
 // stale from the region's top/bottom by one row per generation, which never reaches the R
-// output rows for up to TB_STEPS generations.  Both states (t and t-1) are kept: each
+// output rows for up to `steps` generations.  Both states (t and t-1) are kept: each
 // generation writes the new state in place over the t-1 plane (new(x) reads only old(x) and
 // the current plane), then the planes swap.  The launch reads two planes and writes two planes
 // (the next launch needs both), so global traffic per generation drops by ~TB_STEPS/1.5.
-constexpr int TB_ROWS = 256;  // output rows per tile (72 KB of dynamic shared memory, 3 CTAs per SM)
+//
+// RAGGED: rows of nw words whose last word holds only v = nx - 32*(nw - 1) cells (the rest of its
+// bits 0).  Interior words are loaded as they are; the words past a row's end are put together
+// from the two words that hold their 32 cells after the periodic wrap.  Needs nx >= 64.
 constexpr int TB_STEPS = 16;  // generations per launch (max)
 constexpr int TB_WARPS = 8;
-constexpr int TB_RR = TB_ROWS + 2 * TB_STEPS;
+constexpr int tb_smem(int rows) { return 2 * (rows + 2 * TB_STEPS) * 32 * 4; }
+
+// One lane's words of a region: word `q` of every row, or (general) the 32 cells that start r bits
+// into word q, of which only `cnt` lie before the row's end and the others are the row's first.
+struct WordSource {
+    int q, r, cnt, nw;
+    __device__ __forceinline__ void at(int word, int nx, int nwords)
+    {
+        nw = nwords;
+        long long s = (32LL * word) % nx;
+        if (s < 0) s += nx;
+        q = (int)(s >> 5);
+        r = (int)(s & 31);
+        cnt = nx - (int)s;
+    }
+    __device__ __forceinline__ uint32_t load(const uint32_t* __restrict__ row) const
+    {
+        const uint32_t lo = __ldg(row + q);
+        if (r == 0 && cnt >= 32) return lo;
+        const uint32_t hi = q + 1 < nw ? __ldg(row + q + 1) : 0u;
+        const uint32_t w = __funnelshift_r(lo, hi, r);
+        return cnt >= 32 ? w : (w & ((1u << cnt) - 1u)) | (__ldg(row) << cnt);
+    }
+};
 
 // Row summary of one word for the bit-sliced neighbour count.  Lanes 0 / 31 get their own word
 // back from the shuffles, so their outer bit is wrong; those lanes are the stale halo, whose
@@ -312,34 +339,43 @@ __device__ __forceinline__ RowBits tile_row(uint32_t w)
     return r;
 }
 
-template <int RULE>
+template <int RULE, int ROWS, bool RAGGED>
 __global__ void __launch_bounds__(TB_WARPS * 32) life_bits_tb(const uint32_t* __restrict__ curG, const uint32_t* __restrict__ oldG,
                                                                uint32_t* __restrict__ outCur, uint32_t* __restrict__ outOld,
-                                                               int nw, int ny, int tiles_x, int tiles, int steps)
+                                                               int nx, int nw, int ny, int tiles_x, int tiles, int steps)
 {
-    extern __shared__ uint32_t tbsm[];  // two (TB_RR x 32)-word planes
+    constexpr int RRMAX = ROWS + 2 * TB_STEPS;
+    extern __shared__ uint32_t tbsm[];  // two (RRMAX x 32)-word planes
     uint32_t(*sA)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm);
-    uint32_t(*sB)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm + TB_RR * 32);
+    uint32_t(*sB)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm + RRMAX * 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rr = ROWS + 2 * steps;  // rows of the region
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int tx = tile % tiles_x, ty = tile / tiles_x;
         int wx = (tx * 30 - 1 + lane) % nw;
         if (wx < 0) wx += nw;
-        const int row0 = ty * TB_ROWS - TB_STEPS;
-        for (int r = warp; r < TB_RR; r += TB_WARPS) {
+        WordSource src;
+        if (RAGGED) src.at(tx * 30 - 1 + lane, nx, nw);
+        const int row0 = ty * ROWS - steps;
+        for (int r = warp; r < rr; r += TB_WARPS) {
             int gy = (row0 + r) % ny;
             if (gy < 0) gy += ny;
             const size_t g = (size_t)gy * nw + wx;
-            sA[r][lane] = __ldg(curG + g);
-            sB[r][lane] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(oldG + g) : 0u;
+            if (RAGGED) {
+                sA[r][lane] = src.load(curG + (size_t)gy * nw);
+                sB[r][lane] = RULE == APPFIS_GB_LIFE_REFERENCE ? src.load(oldG + (size_t)gy * nw) : 0u;
+            } else {
+                sA[r][lane] = __ldg(curG + g);
+                sB[r][lane] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(oldG + g) : 0u;
+            }
         }
         __syncthreads();
         uint32_t(*cur)[32] = sA;
         uint32_t(*old)[32] = sB;
         for (int t = 1; t <= steps; t++) {
-            // rows valid after generation t: [t, TB_RR - t), split evenly over the warps; each warp
+            // rows valid after generation t: [t, rr - t), split evenly over the warps; each warp
             // marches its chunk carrying the row summaries (one new row summary per output row)
-            const int lo = t, n = TB_RR - 2 * t, chunk = (n + TB_WARPS - 1) / TB_WARPS;
+            const int lo = t, n = rr - 2 * t, chunk = (n + TB_WARPS - 1) / TB_WARPS;
             const int r0 = lo + warp * chunk, r1 = min(lo + n, r0 + chunk);
             if (r0 < r1) {
                 RowBits up = tile_row(cur[r0 - 1][lane]);
@@ -359,13 +395,14 @@ __global__ void __launch_bounds__(TB_WARPS * 32) life_bits_tb(const uint32_t* __
             old = tmp;
         }
         const int wout = tx * 30 - 1 + lane;
+        const uint32_t keep = RAGGED && wout == nw - 1 && (nx & 31) ? (1u << (nx & 31)) - 1u : FULL;
         if (lane >= 1 && lane <= 30 && wout < nw) {
-            for (int r = TB_STEPS + warp; r < TB_STEPS + TB_ROWS; r += TB_WARPS) {
-                const int gy = ty * TB_ROWS + (r - TB_STEPS);
+            for (int r = steps + warp; r < steps + ROWS; r += TB_WARPS) {
+                const int gy = ty * ROWS + (r - steps);
                 if (gy < ny) {
                     const size_t g = (size_t)gy * nw + wout;
-                    outCur[g] = cur[r][lane];
-                    outOld[g] = old[r][lane];
+                    outCur[g] = RAGGED ? cur[r][lane] & keep : cur[r][lane];
+                    outOld[g] = RAGGED ? old[r][lane] & keep : old[r][lane];
                 }
             }
         }
@@ -373,38 +410,130 @@ __global__ void __launch_bounds__(TB_WARPS * 32) life_bits_tb(const uint32_t* __
     }
 }
 
-__global__ void life_pack(const uint8_t* __restrict__ cells, uint32_t* __restrict__ bits, size_t nwords)
+// ------------------------------------------------------------------------------ bytes <-> words
+__device__ __forceinline__ uint32_t four_bits(uint32_t v)  // bit 0 of bytes 0..3 -> bits 0..3
 {
+    uint32_t x = v & LSB;
+    x = (x | (x >> 7)) & 0x00030003u;  // bytes 0,1 -> bits 0,1 ; bytes 2,3 -> bits 16,17
+    return (x | (x >> 14)) & 0x0000000fu;
+}
+
+__device__ __forceinline__ uint32_t four_bytes(uint32_t b)  // bits 0..3 -> bytes 0..3
+{
+    uint32_t x = b & 0xfu;
+    x = (x | (x << 14)) & 0x00030003u;
+    return (x | (x << 7)) & LSB;
+}
+
+// Whole words (nx a multiple of 32), one or two planes per launch (blockIdx.y).
+__global__ void life_pack(const uint8_t* __restrict__ cellsA, const uint8_t* __restrict__ cellsB, uint32_t* __restrict__ bitsA,
+                          uint32_t* __restrict__ bitsB, size_t nwords)
+{
+    const uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
+    uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
     size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= nwords) return;
     const uint4* p = reinterpret_cast<const uint4*>(cells + w * 32);
     uint4 a = __ldg(p), b = __ldg(p + 1);
     uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, out = 0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        uint32_t x = v[k] & LSB;                 // bit 0 of bytes 0..3 -> bits 0, 8, 16, 24
-        x = (x | (x >> 7)) & 0x00030003u;        // bytes 0,1 -> bits 0,1 ; bytes 2,3 -> bits 16,17
-        x = (x | (x >> 14)) & 0x0000000fu;       // -> bits 0..3
-        out |= x << (4 * k);
-    }
+    for (int k = 0; k < 8; k++) out |= four_bits(v[k]) << (4 * k);
     bits[w] = out;
 }
 
-__global__ void life_unpack(const uint32_t* __restrict__ bits, uint8_t* __restrict__ cells, size_t nwords)
+__global__ void life_unpack(const uint32_t* __restrict__ bitsA, const uint32_t* __restrict__ bitsB, uint8_t* __restrict__ cellsA,
+                            uint8_t* __restrict__ cellsB, size_t nwords)
 {
+    const uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
+    uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
     size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= nwords) return;
     uint32_t b = __ldg(bits + w), v[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        uint32_t x = (b >> (4 * k)) & 0xfu;
-        x = (x | (x << 14)) & 0x00030003u;
-        x = (x | (x << 7)) & LSB;
-        v[k] = x;
-    }
+    for (int k = 0; k < 8; k++) v[k] = four_bytes(b >> (4 * k));
     uint4* p = reinterpret_cast<uint4*>(cells + w * 32);
     p[0] = make_uint4(v[0], v[1], v[2], v[3]);
     p[1] = make_uint4(v[4], v[5], v[6], v[7]);
+}
+
+// Byte rows of any length (nx >= 64) to and from rows of nw = ceil(nx / 32) words, two planes per
+// launch (blockIdx.y).  Bytes move as aligned words whatever the rows' alignment: packing, a thread
+// puts its 32 cells together from nine aligned words; unpacking, a thread writes one aligned
+// 16-byte piece of the plane, which may hold the end of a row and the start of the next.
+// Row and column of the block's first item, items numbered along rows of `per`; the threads then
+// need no 64-bit division.
+__device__ __forceinline__ size_t block_origin(size_t first, int per, int* col)
+{
+    __shared__ size_t row;
+    __shared__ int c;
+    if (threadIdx.x == 0) {
+        row = first / per;
+        c = (int)(first - row * per);
+    }
+    __syncthreads();
+    *col = c;
+    return row;
+}
+
+__global__ void __launch_bounds__(256) life_pack_rows(const uint8_t* __restrict__ cellsA, const uint8_t* __restrict__ cellsB,
+                                                      uint32_t* __restrict__ bitsA, uint32_t* __restrict__ bitsB, int nx, int nw,
+                                                      size_t nwords, size_t ncells)
+{
+    const uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
+    uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
+    int col;
+    const size_t first = (size_t)blockIdx.x * 256, row0 = block_origin(first, nw, &col);
+    const size_t id = first + threadIdx.x;
+    if (id >= nwords) return;
+    const unsigned q = (unsigned)(col + threadIdx.x) / (unsigned)nw, w = (unsigned)(col + threadIdx.x) - q * (unsigned)nw;
+    const size_t at = (row0 + q) * (size_t)nx + 32 * (size_t)w;
+    const int n = min(32, nx - (int)(32 * w));
+    const uint8_t* p = cells + at;
+    const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(p) & 3u);
+    uint32_t out = 0u;
+    if (at >= off && at - off + 36 <= ncells) {  // the nine words lie inside the plane
+        const uint32_t* a = reinterpret_cast<const uint32_t*>(p - off);
+        uint32_t u[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) u[k] = __ldg(a + k);
+#pragma unroll
+        for (int k = 0; k < 8; k++) out |= four_bits(__funnelshift_r(u[k], u[k + 1], 8 * off)) << (4 * k);
+        if (n < 32) out &= (1u << n) - 1u;
+    } else {
+        for (int k = 0; k < n; k++) out |= (uint32_t)(__ldg(p + k) & 1u) << k;
+    }
+    bits[id] = out;
+}
+
+__global__ void __launch_bounds__(256) life_unpack_rows(const uint32_t* __restrict__ bitsA, const uint32_t* __restrict__ bitsB,
+                                                        uint8_t* __restrict__ cellsA, uint8_t* __restrict__ cellsB, int nx, int nw,
+                                                        size_t ncells)
+{
+    const uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
+    uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
+    // the block's 4096 cells start at the plane's byte 4096 * blockIdx.x - lead, a 16-byte boundary
+    const int lead = (int)(reinterpret_cast<uintptr_t>(cells) & 15u);
+    const size_t begin = (size_t)blockIdx.x * 4096;
+    const int skip = begin == 0 ? lead : 0;  // bytes of the first block that lie before the plane
+    int col;
+    const size_t row0 = block_origin(begin + skip - lead, nx, &col);
+    const int from = max(16 * (int)threadIdx.x, skip);  // this thread's cells of the block: from .. to
+    const size_t cell = begin + from - lead;
+    if (cell >= ncells) return;
+    const int to = (int)min((size_t)(16 * (threadIdx.x + 1)), ncells + lead - begin);
+    if (from >= to) return;
+    const unsigned x0 = (unsigned)(col + from - skip), q = x0 / (unsigned)nx, x = x0 - q * (unsigned)nx;
+    const uint32_t* row = bits + (row0 + q) * (size_t)nw;
+    const unsigned w = x >> 5;
+    uint32_t v = __funnelshift_r(__ldg(row + w), (int)w + 1 < nw ? __ldg(row + w + 1) : 0u, x & 31u);
+    const int here = nx - (int)x;  // cells of this row from x on
+    if (here < to - from) v = (v & ((1u << here) - 1u)) | (__ldg(row + nw) << here);
+    uint8_t* d = cells + cell;
+    if (to - from == 16) {
+        *reinterpret_cast<uint4*>(d) = make_uint4(four_bytes(v), four_bytes(v >> 4), four_bytes(v >> 8), four_bytes(v >> 12));
+    } else {
+        for (int k = 0; k < to - from; k++) d[k] = (uint8_t)((v >> k) & 1u);
+    }
 }
 
 // The reference's layout: int cells 0/1 on a (nx + 2g) x (ny + 2g) grid with a periodic ghost
@@ -468,11 +597,112 @@ unsigned resident_grid(K kernel, int tasks)
     return (unsigned)std::max<size_t>(1, std::min<size_t>(need, (size_t)per_sm * gb::sm_count()));
 }
 
+// ------------------------------------------------------------------------------ time-blocked runs
+struct TbPair {
+    uint32_t* p[2];  // state at t, state at t-1
+};
+
+template <int RULE, int ROWS, bool RAGGED>
+int launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+{
+    const int tiles_x = (nw + 29) / 30, tiles = tiles_x * ((ny + ROWS - 1) / ROWS);
+    constexpr int smem = tb_smem(ROWS);
+    auto kern = life_bits_tb<RULE, ROWS, RAGGED>;
+    if (smem > 48 * 1024) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TB_WARPS * 32, smem) != cudaSuccess || per_sm < 1) per_sm = 3;
+    const int grid = std::max(1, std::min(tiles, per_sm * gb::sm_count()));
+    kern<<<grid, TB_WARPS * 32, smem, st>>>(in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, tiles, steps);
+    return APPFIS_GB_OK;
+}
+
+// Output rows per tile: the most whose tiles still number 1.5 per SM.  Tall tiles recompute less halo
+// (256 rows: 9% at 16 generations, 32 rows: 50%) but a warp marches rows / 8 of them one after another, and
+// a small grid has too few to go round.  Measured, us per 64 generations with 256 / 128 / 64 / 32
+// rows: 1024 x 1000 172 / 98 / 66 / 49; 2048^2 172 / 98 / 66 / 66; 4096^2 172 / 123 / 107 / 123;
+// 512 x 16384 164 / 98 / 82 / 98; 8192^2 211 / 213 / 238 / 337; 16384^2 706 / 811 / 935 / 1279.
+int tb_rows(int nw, int ny)
+{
+    const int tiles_x = (nw + 29) / 30;
+    for (int rows : {256, 128, 64})
+        if ((long long)tiles_x * ((ny + rows - 1) / rows) * 2 >= 3LL * gb::sm_count()) return rows;
+    return 32;
+}
+
+template <int RULE, bool RAGGED>
+int tb_step(int rows, TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+{
+    switch (rows) {
+    case 256: return launch_tb<RULE, 256, RAGGED>(in, out, nx, nw, ny, steps, st);
+    case 128: return launch_tb<RULE, 128, RAGGED>(in, out, nx, nw, ny, steps, st);
+    case 64: return launch_tb<RULE, 64, RAGGED>(in, out, nx, nw, ny, steps, st);
+    default: return launch_tb<RULE, 32, RAGGED>(in, out, nx, nw, ny, steps, st);
+    }
+}
+
+// `gens` generations in `launches` launches of nearly equal length, from pair[0] and back into
+// `last`; a launch cannot write the pair it reads (its tiles read their neighbours' halo rows).
+// An odd number of launches goes round three pairs once, so it needs pair[2].
+template <int RULE, bool RAGGED>
+int run_tb(const TbPair (&pair)[3], TbPair last, int nx, int ny, int gens, int launches, cudaStream_t st)
+{
+    const int nw = (nx + 31) / 32, rows = tb_rows(nw, ny);
+    int at = 0, done = 0;
+    for (int n = 0; n < launches; n++) {
+        const int next = (pair[2].p[0] && n < 3) ? (n + 1) % 3 : 1 - at;
+        const int upto = (int)((long long)gens * (n + 1) / launches);
+        GB_TRY((tb_step<RULE, RAGGED>(rows, pair[at], n + 1 == launches ? last : pair[next], nx, nw, ny, upto - done, st)));
+        done = upto;
+        at = next;
+    }
+    return gb::launched("life_bits_tb");
+}
+
 template <int RULE>
 int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream_t st)
 {
     int ci = 0;
-    if (nx % 16 == 0) {
+    const size_t cells = (size_t)nx * ny;
+    // bulk: rows of whole 16-byte vectors and enough of them; 64 x 32-row CTAs at 4 M cells take the
+    // 18.4 us of one CTA's march, which the one-thread-per-cell form takes there too (701 x 700: 5.4)
+    const bool bulk = nx % 16 == 0 && cells >= ((size_t)1 << 22);
+    // Packed: bytes to words, the time-blocked kernel, words to bytes.  The conversions and launches cost
+    // 14 us and 1.1-1.5 us per M cells, a generation next to nothing; a sweep costs 3.4 us (0.1 M cells),
+    // 18 (4 M, either form), 60 / 23 (17 M, one thread per cell / bulk), 244 / 35-47 (67 M).  So packed
+    // wins from 4 generations on, sooner where one thread per cell is slow, and from 3 on over the
+    // bulk form.  Us for 20 generations, sweeps -> packed: 301 x 300 82 -> 33, 2050 x 1999 366 -> 43,
+    // 8192^2 697 -> 131, 8200 x 8192 4878 -> 186.
+    const bool packed = bulk ? gens >= 3 : gens >= 4 || (size_t)gens * cells >= ((size_t)1 << 23);
+    if (nx >= 64 && packed && !gb::capturing(st)) {
+        const int nw = (nx + 31) / 32;
+        const size_t words = (size_t)nw * ny, plane = (words + 63) / 64 * 64;
+        void* ws = nullptr;
+        if (gb::scratch_alloc(4 * sizeof(uint32_t) * plane, st, &ws)) {
+            uint32_t* w = reinterpret_cast<uint32_t*>(ws);
+            const TbPair pair[3] = {{{w, w + plane}}, {{w + 2 * plane, w + 3 * plane}}, {{nullptr, nullptr}}};
+            const unsigned planes = RULE == APPFIS_GB_LIFE_REFERENCE ? 2 : 1;  // B3/S23 does not read the state at t-1
+            const int launches = (gens + TB_STEPS - 1) / TB_STEPS;
+            const TbPair last = pair[launches & 1];
+            const dim3 wgrid(gb::ceil_div(words, 256), planes);
+            ci = gens & 1;
+            int rc;
+            if (nx % 32) {
+                life_pack_rows<<<wgrid, 256, 0, st>>>(buf[0], buf[1], w, w + plane, nx, nw, words, cells);
+                rc = run_tb<RULE, true>(pair, last, nx, ny, gens, launches, st);
+                life_unpack_rows<<<dim3(gb::ceil_div(cells + 15, 4096), 2), 256, 0, st>>>(last.p[0], last.p[1], buf[ci], buf[1 - ci], nx, nw, cells);
+            } else {
+                life_pack<<<wgrid, 256, 0, st>>>(buf[0], buf[1], w, w + plane, words);
+                rc = run_tb<RULE, false>(pair, last, nx, ny, gens, launches, st);
+                life_unpack<<<dim3(wgrid.x, 2), 256, 0, st>>>(last.p[0], last.p[1], buf[ci], buf[1 - ci], words);
+            }
+            gb::scratch_free(ws, st);
+            GB_TRY(rc);
+            GB_TRY(gb::launched("life_u8 (packed)"));
+            if (cur_index) *cur_index = ci;
+            return APPFIS_GB_OK;
+        }
+    }
+    if (bulk) {
         unsigned* status;
         GB_TRY(gb::status_word(&status));
         GB_CUDA(cudaFuncSetAttribute(life_u8_bulk<RULE>, cudaFuncAttributeMaxDynamicSharedMemorySize, UB_SMEM));
@@ -494,63 +724,50 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
     return APPFIS_GB_OK;
 }
 
-// Time-blocked launches for whole blocks of TB_STEPS generations, single-generation sweeps for
-// the remainder.  A launch reads a (cur, old) pair and writes another pair (its tiles read
-// neighbours' halo rows, so it cannot write in place).  An even number of launches ping-pongs
-// between (a, b) and a workspace pair; an odd number of three or more first goes round three
-// pairs once ((a, b) -> W1 -> W2 -> (a, b)) and then ping-pongs, so the newest state ends in
-// (a, b) without a copy; a single launch copies its pair back.  cur_index tells which of a, b
-// holds the newest state.
+// Bit-packed run.  Four or more generations take the time-blocked kernel, at least two launches so that
+// the state comes back into (a, b): 2 / 4 / 8 generations as sweeps against tiles, us: 1024 x 1000 8.2 / 16.4 /
+// 32.8 against 10.8 / 12.3 / 14.3; 4096^2 12.3 / 24.6 / 49.2 against 14.7 / 17.0 / 22.6; 16384^2 61 / 123 / 246
+// against 89 / 102 / 131.  The newest state is in a after an even number of generations, else in b,
+// as it is when every generation is a sweep.
 template <int RULE>
 int run_bits(uint32_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream_t st)
 {
-    const int nw = nx / 32;
-    int ci = 0;
-    const size_t plane = (size_t)nw * ny;
-    if (gens >= TB_STEPS) {
-        const int launches = gens / TB_STEPS;
-        void *wc, *wd, *we = nullptr, *wf = nullptr;
-        GB_TRY(gb::workspace(gb::WS_LIFE_C, sizeof(uint32_t) * plane, &wc));
-        GB_TRY(gb::workspace(gb::WS_LIFE_D, sizeof(uint32_t) * plane, &wd));
-        if (launches % 2 == 1 && launches >= 3) {
-            GB_TRY(gb::workspace(gb::WS_LIFE_E, sizeof(uint32_t) * plane, &we));
-            GB_TRY(gb::workspace(gb::WS_LIFE_F, sizeof(uint32_t) * plane, &wf));
-        }
-        uint32_t* P[3][2] = {{buf[0], buf[1]}, {(uint32_t*)wc, (uint32_t*)wd}, {(uint32_t*)we, (uint32_t*)wf}};  // [pair][cur/old]
-        const int tiles_x = (nw + 29) / 30, tiles = tiles_x * ((ny + TB_ROWS - 1) / TB_ROWS);
-        int per_sm = 0;
-        const int tsm = 2 * TB_RR * 32 * 4;
-        GB_CUDA(cudaFuncSetAttribute(life_bits_tb<RULE>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm));
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, life_bits_tb<RULE>, TB_WARPS * 32, tsm) != cudaSuccess ||
-            per_sm < 1)
-            per_sm = 4;
-        const int grid = std::max(1, std::min(tiles, per_sm * gb::sm_count()));
-        int pair = 0;
-        for (int n = 0; n < launches; n++) {
-            const int next = (we && n < 3) ? (n + 1) % 3 : 1 - pair;  // the three-pair round first, then ping-pong
-            life_bits_tb<RULE><<<grid, TB_WARPS * 32, tsm, st>>>(P[pair][0], P[pair][1], P[next][0], P[next][1], nw, ny, tiles_x,
-                                                               tiles, TB_STEPS);
-            pair = next;
-        }
-        GB_TRY(gb::launched("life_bits_tb"));
-        if (pair != 0) {  // one launch: bring the (cur, old) pair back into (a, b)
-            GB_CUDA(cudaMemcpyAsync(buf[0], P[pair][0], sizeof(uint32_t) * plane, cudaMemcpyDeviceToDevice, st));
-            GB_CUDA(cudaMemcpyAsync(buf[1], P[pair][1], sizeof(uint32_t) * plane, cudaMemcpyDeviceToDevice, st));
-        }
-        gens -= launches * TB_STEPS;
-    }
-    if (gens > 0) {
-        const int strips = (nw + 31) / 32;
-        const int tasks = strips * ((ny + LIFE_ROWS - 1) / LIFE_ROWS);
-        const unsigned grid = resident_grid(life_bits_sweep<RULE>, tasks);
-        for (int g = 0; g < gens; g++) {
-            life_bits_sweep<RULE><<<grid, 256, 0, st>>>(buf[ci], buf[1 - ci], nw, ny, strips, tasks);
-            ci = 1 - ci;
-        }
-        GB_TRY(gb::launched("life_bits sweep"));
-    }
+    const int nw = nx / 32, ci = gens & 1;
+    const size_t plane = (size_t)nw * ny, bytes = sizeof(uint32_t) * plane;
+    const TbPair own = {{buf[0], buf[1]}}, last = {{buf[ci], buf[1 - ci]}};
     if (cur_index) *cur_index = ci;
-    return APPFIS_GB_OK;
+    if (gens >= TB_STEPS) {
+        // the long runs' pairs stay in the workspace, so that a run can be recorded in a graph after a
+        // first one has sized them; a recording that would need more takes one more, shorter, launch
+        int launches = std::max(2, (gens + TB_STEPS - 1) / TB_STEPS);
+        void *wc, *wd, *we = nullptr, *wf = nullptr;
+        GB_TRY(gb::workspace(gb::WS_LIFE_C, bytes, &wc));
+        GB_TRY(gb::workspace(gb::WS_LIFE_D, bytes, &wd));
+        if (launches % 2 && gb::capturing(st) && !(gb::workspace_holds(gb::WS_LIFE_E, bytes) && gb::workspace_holds(gb::WS_LIFE_F, bytes)))
+            launches++;
+        if (launches % 2) {
+            GB_TRY(gb::workspace(gb::WS_LIFE_E, bytes, &we));
+            GB_TRY(gb::workspace(gb::WS_LIFE_F, bytes, &wf));
+        }
+        const TbPair pair[3] = {own, {{(uint32_t*)wc, (uint32_t*)wd}}, {{(uint32_t*)we, (uint32_t*)wf}}};
+        return run_tb<RULE, false>(pair, last, nx, ny, gens, launches, st);
+    }
+    void* ws = nullptr;
+    if (gens >= 4 && !gb::capturing(st) && gb::scratch_alloc(2 * bytes, st, &ws)) {
+        const TbPair pair[3] = {own, {{(uint32_t*)ws, (uint32_t*)ws + plane}}, {{nullptr, nullptr}}};
+        const int rc = run_tb<RULE, false>(pair, last, nx, ny, gens, 2, st);
+        gb::scratch_free(ws, st);
+        return rc;
+    }
+    // one launch per generation; rows per warp so that every SM has 24 warps' work if the grid has it
+    // (1024 x 1000: 4.1 us with 4 rows, 10.3 with 32; 16384^2: 37.9 and 30.7)
+    const int strips = (nw + 31) / 32;
+    int srows = LIFE_ROWS;
+    while (srows > 4 && (long long)strips * ((ny + srows - 1) / srows) < 24LL * gb::sm_count()) srows /= 2;
+    const int tasks = strips * ((ny + srows - 1) / srows);
+    const unsigned grid = resident_grid(life_bits_sweep<RULE>, tasks);
+    for (int g = 0; g < gens; g++) life_bits_sweep<RULE><<<grid, 256, 0, st>>>(buf[g & 1], buf[1 - (g & 1)], nw, ny, strips, srows, tasks);
+    return gb::launched("life_bits sweep");
 }
 
 int check_life(const void* a, const void* b, int nx, int ny, int gens, int rule)
@@ -609,7 +826,7 @@ int appfis_gb_life_pack(const uint8_t* cells, uint32_t* bits, int nx, int ny, vo
     if (!cells || !bits || nx < 1 || ny < 1 || nx % 32) return gb::fail(APPFIS_GB_EINVAL, "life_pack: bad arguments");
     if (reinterpret_cast<uintptr_t>(cells) & 15) return gb::fail(APPFIS_GB_EINVAL, "life_pack: cells must be 16-byte aligned");
     size_t nw = (size_t)nx * ny / 32;
-    life_pack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(cells, bits, nw);
+    life_pack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(cells, cells, bits, bits, nw);
     return gb::launched("life_pack");
 }
 
@@ -618,7 +835,7 @@ int appfis_gb_life_unpack(const uint32_t* bits, uint8_t* cells, int nx, int ny, 
     if (!cells || !bits || nx < 1 || ny < 1 || nx % 32) return gb::fail(APPFIS_GB_EINVAL, "life_unpack: bad arguments");
     if (reinterpret_cast<uintptr_t>(cells) & 15) return gb::fail(APPFIS_GB_EINVAL, "life_unpack: cells must be 16-byte aligned");
     size_t nw = (size_t)nx * ny / 32;
-    life_unpack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(bits, cells, nw);
+    life_unpack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(bits, bits, cells, cells, nw);
     return gb::launched("life_unpack");
 }
 
