@@ -20,7 +20,8 @@ constexpr int BX = 32, BY = 8;
 __global__ void __launch_bounds__(BX * BY) heat2d_f64(const double* __restrict__ cur, double* __restrict__ nxt, int nx, int ny,
                                                       int px, double cx, double cy)
 {
-    const int i = 1 + blockIdx.x * BX + threadIdx.x, j = 1 + blockIdx.y * BY + threadIdx.y;
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = 1 + bid.x * BX + threadIdx.x, j = 1 + bid.y * BY + threadIdx.y;
     if (i > nx || j > ny) return;
     const size_t c = (size_t)j * px + i;
     const double v = __ldg(cur + c), two_c = __dmul_rn(2.0, v);
@@ -38,7 +39,8 @@ struct CoefF64 {
 __global__ void __launch_bounds__(BX * BY) himeno_f64(CoefF64 cf, const double* __restrict__ p, double* __restrict__ w2, int nx,
                                                       int ny, int nz, int px, int py, double omega, double* __restrict__ partials)
 {
-    const int i = 1 + blockIdx.x * BX + threadIdx.x, j = 1 + blockIdx.y * BY + threadIdx.y, k = 1 + blockIdx.z;
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = 1 + bid.x * BX + threadIdx.x, j = 1 + bid.y * BY + threadIdx.y, k = 1 + bid.z;
     double g = 0.0;
     if (i <= nx && j <= ny) {
         const size_t sx = 1, sy = (size_t)px, sz = (size_t)px * py, c = (size_t)k * sz + (size_t)j * sy + i;
@@ -69,13 +71,14 @@ __global__ void __launch_bounds__(BX * BY) himeno_f64(CoefF64 cf, const double* 
     if (t == 0 && partials) {
         double s = 0.0;
         for (int n = 0; n < BY; n++) s = __dadd_rn(s, ws[n]);
-        partials[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = s;
+        partials[((size_t)bid.z * gridDim.y + bid.y) * gridDim.x + bid.x] = s;
     }
 }
 
 // One block folds n partials: each thread a contiguous run in order, then the runs in thread order.
 __global__ void __launch_bounds__(1024) fold_f64(const double* __restrict__ part, size_t n, double* __restrict__ out)
 {
+    gb::grid_wait();
     __shared__ double sh[1024];
     const size_t per = (n + 1023) / 1024, b = (size_t)threadIdx.x * per, e = b + per < n ? b + per : n;
     double s = 0.0;
@@ -98,8 +101,9 @@ template <int MODE>
 __global__ void __launch_bounds__(BX * BY) star_r4_f64(const double* __restrict__ cur, double* __restrict__ nxt, int nx, int ny,
                                                        int px, int py, double coeff, StarWeightsF64 wt)
 {
+    const gb::BlockId bid = gb::grid_wait();
     constexpr int R = 4;
-    const int i = R + blockIdx.x * BX + threadIdx.x, j = R + blockIdx.y * BY + threadIdx.y, k = R + blockIdx.z;
+    const int i = R + bid.x * BX + threadIdx.x, j = R + bid.y * BY + threadIdx.y, k = R + bid.z;
     if (i >= nx + R || j >= ny + R) return;
     const long long sy = px, sz = (long long)px * py;
     const size_t c = (size_t)k * sz + (size_t)j * sy + i;
@@ -129,7 +133,7 @@ int appfis_gb_heat2d_f64(double* a, double* b, int nx, int ny, int pitch, int it
     double* buf[2] = {a, b};
     dim3 blk(BX, BY), grd(gb::ceil_div(nx, BX), gb::ceil_div(ny, BY));
     int ci = 0;
-    for (int it = 0; it < iters; it++, ci = 1 - ci) heat2d_f64<<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny, pitch, cx, cy);
+    for (int it = 0; it < iters; it++, ci = 1 - ci) gb::launch(heat2d_f64, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny, pitch, cx, cy);
     GB_TRY(gb::launched("heat2d_f64"));
     if (cur_index) *cur_index = ci;
     return APPFIS_GB_OK;
@@ -155,8 +159,8 @@ int appfis_gb_himeno_f64(const double* const* coef, double* p, double* wrk2, int
     double* buf[2] = {p, wrk2};
     int ci = 0;
     for (int it = 0; it < iters; it++, ci = 1 - ci) {
-        himeno_f64<<<grd, blk, 0, st>>>(cf, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, omega, part);
-        if (dev_gosa) fold_f64<<<1, 1024, 0, st>>>(part, nblk, dev_gosa + it);
+        gb::launch(himeno_f64, grd, blk, 0, st, cf, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, omega, part);
+        if (dev_gosa) gb::launch(fold_f64, 1, 1024, 0, st, part, nblk, dev_gosa + it);
     }
     GB_TRY(gb::launched("himeno_f64"));
     if (cur_index) *cur_index = ci;
@@ -179,8 +183,8 @@ int appfis_gb_star_r4_f64(double* a, double* b, int nx, int ny, int nz, int pitc
     dim3 blk(BX, BY), grd(gb::ceil_div(nx, BX), gb::ceil_div(ny, BY), nz);
     int ci = 0;
     for (int it = 0; it < iters; it++, ci = 1 - ci) {
-        if (mode == 0) star_r4_f64<0><<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny, pitch, ny + 8, coeff, w);
-        else star_r4_f64<1><<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny, pitch, ny + 8, coeff, w);
+        if (mode == 0) gb::launch(star_r4_f64<0>, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny, pitch, ny + 8, coeff, w);
+        else gb::launch(star_r4_f64<1>, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny, pitch, ny + 8, coeff, w);
     }
     GB_TRY(gb::launched("star_r4_f64"));
     if (cur_index) *cur_index = ci;

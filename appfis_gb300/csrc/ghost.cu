@@ -14,12 +14,13 @@ namespace {
 template <class E>
 __global__ void periodic_axis(E* __restrict__ f, int dx, int dy, int dz, int axis, int G)
 {
+    const gb::BlockId bid = gb::grid_wait();
     // slab: 2G layers along `axis` times the full extent of the two other axes
     const int dims[3] = {dx, dy, dz};
     const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
     const long long n1 = dims[a1], n2 = dims[a2];
     const long long total = (long long)2 * G * n1 * n2;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+    for (long long t = (long long)bid.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int u = (int)(t % n1);
         const long long r = t / n1;
         const int v = (int)(r % n2);
@@ -51,7 +52,7 @@ int fill(void* field, int ndim, const int* pd, int G, cudaStream_t st)
         const long long other = (long long)dims[axis == 0 ? 1 : 0] * dims[axis == 2 ? 1 : 2];
         const long long total = 2LL * G * other;
         const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((total + 255) / 256, 4LL * gb::sm_count()));
-        periodic_axis<E><<<grid, 256, 0, st>>>(reinterpret_cast<E*>(field), dx, dy, dz, axis, G);
+        gb::launch(periodic_axis<E>, grid, 256, 0, st, reinterpret_cast<E*>(field), dx, dy, dz, axis, G);
     }
     return gb::launched("periodic_axis");
 }

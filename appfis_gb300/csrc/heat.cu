@@ -26,8 +26,9 @@ __device__ __forceinline__ float heat_point(float c, float l, float r, float u, 
 __global__ void __launch_bounds__(256) heat2d_sweep_k(const float* __restrict__ cur, float* __restrict__ nxt, int nx,
                                                        int ny, int pitch, float cx, float cy)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = 1 + bid.x * blockDim.x + threadIdx.x;
+    const int j = 1 + bid.y * blockDim.y + threadIdx.y;
     if (i > nx || j > ny) return;
     const size_t c = (size_t)j * pitch + i;
     nxt[c] = heat_point(__ldg(cur + c), __ldg(cur + c - 1), __ldg(cur + c + 1), __ldg(cur + c - pitch), __ldg(cur + c + pitch),
@@ -57,12 +58,12 @@ struct HeatEdges {  // block edges, by sweep parity
 // cells are updated; tiles whose whole region is interior take the unmasked form.
 template <int TX, int TY, int SMAX, int S, bool MASK>
 __device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch,
-                                          float cx, float cy, HeatEdges<(TX + 2 * SMAX) / RBS, (TY + 2 * SMAX) / RBS>& e)
+                                          float cx, float cy, HeatEdges<(TX + 2 * SMAX) / RBS, (TY + 2 * SMAX) / RBS>& e, gb::BlockId bid)
 {
     constexpr int BX = (TX + 2 * SMAX) / RBS, BY = (TY + 2 * SMAX) / RBS;
     constexpr int rw = TX + 2 * S, rh = TY + 2 * S;  // region in use
     const int t = threadIdx.x, bx = t % BX, by = t / BX;
-    const int ox = 1 + blockIdx.x * TX - S, oy = 1 + blockIdx.y * TY - S;  // padded coords of region (0,0)
+    const int ox = 1 + bid.x * TX - S, oy = 1 + bid.y * TY - S;  // padded coords of region (0,0)
     float v[RBS][RBS];
     unsigned upd = 0;  // MASK: bit 4r+c set for an interior cell of the region in use
 #pragma unroll
@@ -115,7 +116,7 @@ __device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* 
 #pragma unroll
         for (int c = 0; c < RBS; c++) {
             const int x = RBS * bx + c - S, y = RBS * by + r - S;  // output tile coordinates
-            const int gx = 1 + blockIdx.x * TX + x, gy = 1 + blockIdx.y * TY + y;
+            const int gx = 1 + bid.x * TX + x, gy = 1 + bid.y * TY + y;
             if (x >= 0 && x < TX && y >= 0 && y < TY && (!MASK || (gx <= nx && gy <= ny))) nxt[(size_t)gy * pitch + gx] = v[r][c];
         }
 }
@@ -124,17 +125,18 @@ template <int TX, int TY, int SMAX, int S>
 __global__ void __launch_bounds__(((TX + 2 * SMAX) / RBS) * ((TY + 2 * SMAX) / RBS))
     heat2d_regs(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch, float cx, float cy)
 {
+    const gb::BlockId bid = gb::grid_wait();
     constexpr int BX = (TX + 2 * SMAX) / RBS, BY = (TY + 2 * SMAX) / RBS;
     static_assert(BX * RBS == TX + 2 * SMAX && BY * RBS == TY + 2 * SMAX, "region in whole blocks");
     static_assert(S >= 1 && S <= SMAX, "sweeps per launch");
     __shared__ HeatEdges<BX, BY> e;
     // the whole region (TX + 2 SMAX wide, loaded in full) lies on interior cells
-    const bool inner = S == SMAX && (int)blockIdx.x * TX >= S && (int)blockIdx.y * TY >= S &&
-                       ((int)blockIdx.x + 1) * TX + S <= nx && ((int)blockIdx.y + 1) * TY + S <= ny;
+    const bool inner = S == SMAX && (int)bid.x * TX >= S && (int)bid.y * TY >= S &&
+                       ((int)bid.x + 1) * TX + S <= nx && ((int)bid.y + 1) * TY + S <= ny;
     if (inner)
-        heat_tile<TX, TY, SMAX, S, false>(cur, nxt, nx, ny, pitch, cx, cy, e);
+        heat_tile<TX, TY, SMAX, S, false>(cur, nxt, nx, ny, pitch, cx, cy, e, bid);
     else
-        heat_tile<TX, TY, SMAX, S, true>(cur, nxt, nx, ny, pitch, cx, cy, e);
+        heat_tile<TX, TY, SMAX, S, true>(cur, nxt, nx, ny, pitch, cx, cy, e, bid);
 }
 
 template <int TX, int TY, int SMAX, int S = SMAX>
@@ -145,7 +147,7 @@ void launch_heat_regs(int s, dim3 grd, const float* cur, float* nxt, int nx, int
         if (s < S) return launch_heat_regs<TX, TY, SMAX, S - 1>(s, grd, cur, nxt, nx, ny, pitch, cx, cy, st);
     }
     constexpr int threads = ((TX + 2 * SMAX) / RBS) * ((TY + 2 * SMAX) / RBS);
-    heat2d_regs<TX, TY, SMAX, S><<<grd, threads, 0, st>>>(cur, nxt, nx, ny, pitch, cx, cy);
+    gb::launch(heat2d_regs<TX, TY, SMAX, S>, grd, threads, 0, st, cur, nxt, nx, ny, pitch, cx, cy);
 }
 
 // 48 x 32 output tiles: a 64 x 48 region, 16 x 12 blocks, 192 threads of at most 96 registers,
@@ -168,7 +170,7 @@ int appfis_gb_heat2d_sweep(const float* cur, float* next, int nx, int ny, int pi
 {
     GB_TRY(check_heat(cur, next, nx, ny, pitch));
     dim3 blk(64, 4), grd(gb::ceil_div(nx, 64), gb::ceil_div(ny, 4));
-    heat2d_sweep_k<<<grd, blk, 0, gb::as_stream(stream)>>>(cur, next, nx, ny, pitch, cx, cy);
+    gb::launch(heat2d_sweep_k, grd, blk, 0, gb::as_stream(stream), cur, next, nx, ny, pitch, cx, cy);
     return gb::launched("heat2d_sweep");
 }
 

@@ -103,7 +103,7 @@ __device__ __forceinline__ void gosa_end(const double (&v)[NV], const GosaIO& g)
     if (g.prev && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) gosa_fold(g);
 }
 
-__global__ void himeno_gosa_fold(GosaIO g) { gosa_fold(g); }
+__global__ void himeno_gosa_fold(GosaIO g) { gb::grid_wait(); gosa_fold(g); }
 
 // Per-thread sum of squares in two floats (hi + lo, ~48 significant bits): the square is split
 // exactly with an FMA and added with an exact two-sum, so a thread's few dozen terms stay within
@@ -157,9 +157,10 @@ __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float*
                                                           __half* __restrict__ enext, int nx, int ny, int nz, int px,
                                                           int py, int kz, float omega, float inv_omega, int prime, GosaIO gz)
 {
-    const int i = 1 + blockIdx.x * BX + threadIdx.x;
-    const int j = 1 + blockIdx.y * BY + threadIdx.y;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = 1 + bid.x * BX + threadIdx.x;
+    const int j = 1 + bid.y * BY + threadIdx.y;
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const bool act = i <= nx && j <= ny;
     const ptrdiff_t plane = (ptrdiff_t)px * py;
     ptrdiff_t c = ((ptrdiff_t)k0 * py + j) * px + i;
@@ -239,18 +240,19 @@ __global__ void __launch_bounds__(RX* RY) himeno_ring(Coef12 cf, H10 hf, const v
                                                        const __half* __restrict__ D, int nx, int ny, int nz, int px, int py,
                                                        int kz, float omega, float inv_omega, GosaIO gz)
 {
+    const gb::BlockId bid = gb::grid_wait();
     __shared__ float ring[4][RSLOT];
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * RX + tx;
-    const int i = 1 + blockIdx.x * RX + tx, j = 1 + blockIdx.y * RY + ty;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const int i = 1 + bid.x * RX + tx, j = 1 + bid.y * RY + ty;
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const size_t plane = (size_t)px * py;
     const bool act = i <= nx && j <= ny;
     // this thread's halo cell (fixed for all planes)
     int hs = 0, hi = 0, hj = 0;
     if (t < RHALO) {
         hs = halo_slot(t);
-        hi = blockIdx.x * RX + hs % RW;  // padded coords: slot (0,0) is (i0-1, j0-1)
-        hj = blockIdx.y * RY + hs / RW;
+        hi = bid.x * RX + hs % RW;  // padded coords: slot (0,0) is (i0-1, j0-1)
+        hj = bid.y * RY + hs / RW;
     }
     typedef typename std::conditional<MODE == 0, float, __half>::type L;
     const L* f = reinterpret_cast<const L*>(pin);
@@ -363,6 +365,7 @@ __global__ void __launch_bounds__(RX* RY) himeno_tma(const __grid_constant__ Til
                                                       int nz, int pitch, int py, int kz, float omega,
                                                       GosaIO gz, unsigned* __restrict__ status)
 {
+    const gb::BlockId bid = gb::grid_wait();
     typedef TmaLayout Lay;
     typedef float L;
     constexpr int P = S + 2;  // ring slots: planes k-1 .. k+S
@@ -372,9 +375,9 @@ __global__ void __launch_bounds__(RX* RY) himeno_tma(const __grid_constant__ Til
     uint64_t* bar = reinterpret_cast<uint64_t*>(tsm + S * Lay::CT + P * Lay::PB);
 
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * RX + tx;
-    const int x0 = blockIdx.x * RX, y0 = 1 + blockIdx.y * RY;
+    const int x0 = bid.x * RX, y0 = 1 + bid.y * RY;
     const int i = x0 + tx, j = y0 + ty;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const bool act = i >= 1 && i <= nx && j <= ny;
     if (gb::tma::smem_u32(tsm) & 127u) {  // uniform: the copies need 128-byte aligned destinations
         if (t == 0) atomicOr(status, (unsigned)gb::ST_SMEM_ALIGN);
@@ -548,6 +551,7 @@ __global__ void __launch_bounds__(TW / 2 * MY) himeno_mixed2(const __grid_consta
                                                              int nx, int ny, int nz, int pitch, int py, int kz, float omega,
                                                              float inv_omega, GosaIO gz, unsigned* __restrict__ status)
 {
+    const gb::BlockId bid = gb::grid_wait();
     namespace f2 = gb::f2;
     typedef MixTile<TW> L;
     constexpr int MX = L::X, MW = L::W, MEB = L::EB, MES = L::ES, MCT = L::CT, MSTG = L::STG, MR32 = L::R32;
@@ -560,9 +564,9 @@ __global__ void __launch_bounds__(TW / 2 * MY) himeno_mixed2(const __grid_consta
     // the copies are issued by the last warp's first thread: the e box conversion leaves that
     // warp the fewest pairs, so the issue work does not delay the plane's slowest warp
     const int issuer = MX / 2 * MY - 32;
-    const int x0 = blockIdx.x * MX, y0 = 1 + blockIdx.y * MY;
+    const int x0 = bid.x * MX, y0 = 1 + bid.y * MY;
     const int xa = x0 + 2 * tx, j = y0 + ty;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const bool acta = xa >= 1 && xa <= nx && j <= ny, actb = xa + 1 <= nx && j <= ny;
     if (gb::tma::smem_u32(tsm) & 127u) {
         if (t == 0) atomicOr(status, (unsigned)gb::ST_SMEM_ALIGN);
@@ -689,6 +693,7 @@ __global__ void __launch_bounds__(T2NT, 2) himeno_mixed_tb2(const __grid_constan
                                                             int ny, int nz, int pitch, int py, int kz, float omega, float inv_omega,
                                                             GosaIO gz, unsigned* __restrict__ status)
 {
+    const gb::BlockId bid = gb::grid_wait();
     namespace f2 = gb::f2;
     extern __shared__ __align__(128) unsigned char tsm[];
     unsigned char* stages = tsm;
@@ -697,8 +702,8 @@ __global__ void __launch_bounds__(T2NT, 2) himeno_mixed_tb2(const __grid_constan
     unsigned char* pro = tsm + T2S * T2STG + T2R0B + T2R1B;
     uint64_t* bar = reinterpret_cast<uint64_t*>(pro + 2 * T2EB);
     const int t = threadIdx.x, issuer = T2NT - 32;  // the copies: the last warp (no sweep-2 pairs)
-    const int x0 = blockIdx.x * T2X, y0 = 1 + blockIdx.y * T2Y;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const int x0 = bid.x * T2X, y0 = 1 + bid.y * T2Y;
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const int qlo = k0 - 1, nst = k1 - k0 + 2;  // sweep 1 runs on planes qlo .. k1
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (gb::tma::smem_u32(tsm) & 127u) {
@@ -854,6 +859,7 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
                                                               int nz, int pitch, int py, int kz, float omega, float inv_omega,
                                                               int prime, GosaIO gz, unsigned* __restrict__ status)
 {
+    const gb::BlockId bid = gb::grid_wait();
     typedef TmaLayout Lay;
     extern __shared__ __align__(128) unsigned char tsm[];
     unsigned char* stages = tsm;
@@ -861,9 +867,9 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
     unsigned char* pro = tsm + S * CSTG + 4 * CQ * 4;
     uint64_t* bar = reinterpret_cast<uint64_t*>(pro + 3 * (CPB + CES));
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * RX + tx;
-    const int x0 = blockIdx.x * RX, y0 = 1 + blockIdx.y * RY;
+    const int x0 = bid.x * RX, y0 = 1 + bid.y * RY;
     const int i = x0 + tx, j = y0 + ty;
-    const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, nz + 1);
+    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
     const bool act = i >= 1 && i <= nx && j <= ny;
     if (gb::tma::smem_u32(tsm) & 127u) {
         if (t == 0) atomicOr(status, (unsigned)gb::ST_SMEM_ALIGN);
@@ -1010,7 +1016,7 @@ struct GosaSeq {
     int flush(cudaStream_t st)
     {
         if (!pend.prev) return APPFIS_GB_OK;
-        himeno_gosa_fold<<<1, 256, 0, st>>>(pend);
+        gb::launch(himeno_gosa_fold, 1, 256, 0, st, pend);
         pend = {};
         return gb::launched("himeno_gosa_fold");
     }
@@ -1057,7 +1063,7 @@ int appfis_gb_himeno(const float* const* coef, float* p, float* wrk2, int nx, in
         dim3 tgrd(nx / RX + 1, gb::ceil_div(ny, RY), gb::ceil_div(nz, kz));
         GB_TRY(gs.init(dev_gosa, (size_t)tgrd.x * tgrd.y * tgrd.z, 1));
         for (int it = 0; it < iters; it++) {
-            himeno_tma<TMA_S_PLAIN><<<tgrd, blk, smem, st>>>(maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, kz, omega,
+            gb::launch(himeno_tma<TMA_S_PLAIN>, tgrd, blk, smem, st, maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, kz, omega,
                                                             gs.next(tgrd, 1, dev_gosa ? dev_gosa + it : nullptr), status);
             ci = 1 - ci;
         }
@@ -1069,7 +1075,7 @@ int appfis_gb_himeno(const float* const* coef, float* p, float* wrk2, int nx, in
     GB_TRY(gs.init(dev_gosa, (size_t)grd.x * grd.y * grd.z, 1));
     H10 none = {};
     for (int it = 0; it < iters; it++) {
-        himeno_ring<0><<<grd, blk, 0, st>>>(cf, none, buf[ci], buf[1 - ci], nullptr, nx, ny, nz, pitch, ny + 2, HKZ, omega, 0.0f,
+        gb::launch(himeno_ring<0>, grd, blk, 0, st, cf, none, buf[ci], buf[1 - ci], nullptr, nx, ny, nz, pitch, ny + 2, HKZ, omega, 0.0f,
                                             gs.next(grd, 1, dev_gosa ? dev_gosa + it : nullptr));
         ci = 1 - ci;
     }
@@ -1221,10 +1227,10 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     auto correct = [&](bool prime, double* g) {
         const GosaIO gz = gs.next(use_tma ? cgrd : grd, 1, prime ? g : nullptr);
         if (use_tma)
-            himeno_correct_tma<CORR_S><<<cgrd, rblk, csmem, st>>>(cmaps[pc][ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
+            gb::launch(himeno_correct_tma<CORR_S>, cgrd, rblk, csmem, st, cmaps[pc][ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
                                                                  ckz, omega, inv_omega, prime ? 1 : 0, gz, status);
         else
-            himeno_correct<HBX, HBY><<<grd, blk, 0, st>>>(cf, P[pc], E[ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
+            gb::launch(himeno_correct<HBX, HBY>, grd, blk, 0, st, cf, P[pc], E[ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
                                                           HKZ, omega, inv_omega, prime ? 1 : 0, gz);
         pc = 1 - pc;
         ec = 1 - ec;
@@ -1239,15 +1245,15 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
         it += 1;
         while (it < end) {
             if (two && end - it >= 2) {
-                himeno_mixed_tb2<<<t2grd, T2NT, t2_smem(), st>>>(t2maps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, t2kz, omega, inv_omega,
+                gb::launch(himeno_mixed_tb2, t2grd, T2NT, t2_smem(), st, t2maps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, t2kz, omega, inv_omega,
                                                                gs.next(t2grd, 2, dev_gosa ? dev_gosa + it : nullptr), status);
                 it += 2;
             } else {
                 if (use_tma)
-                    tkern<<<tgrd, tblk, tsmem, st>>>(tmaps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, tkz, omega, inv_omega,
+                    gb::launch(tkern, tgrd, tblk, tsmem, st, tmaps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, tkz, omega, inv_omega,
                                                      gs.next(tgrd, 1, dev_gosa ? dev_gosa + it : nullptr), status);
                 else
-                    himeno_ring<1><<<rgrd, rblk, 0, st>>>(cf, hf, E[ec], E[1 - ec], Dd, nx, ny, nz, pitch, ny + 2, HKZ, omega,
+                    gb::launch(himeno_ring<1>, rgrd, rblk, 0, st, cf, hf, E[ec], E[1 - ec], Dd, nx, ny, nz, pitch, ny + 2, HKZ, omega,
                                                           inv_omega, gs.next(rgrd, 1, dev_gosa ? dev_gosa + it : nullptr));
                 it += 1;
             }

@@ -46,8 +46,9 @@ __device__ __forceinline__ uint32_t rule_bytes(uint32_t cnt, uint32_t c, uint32_
 template <int RULE>
 __global__ void life_u8_generic(const uint8_t* __restrict__ cur, uint8_t* __restrict__ out, int nx, int ny)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const gb::BlockId bid = gb::grid_wait();
+    int i = bid.x * blockDim.x + threadIdx.x;
+    int j = bid.y * blockDim.y + threadIdx.y;
     if (i >= nx || j >= ny) return;
     int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
     size_t rm = (size_t)(j == 0 ? ny - 1 : j - 1) * nx, r0 = (size_t)j * nx, rp = (size_t)(j == ny - 1 ? 0 : j + 1) * nx;
@@ -103,10 +104,11 @@ template <int RULE>
 __global__ void __launch_bounds__(256) life_u8_bulk(const uint8_t* __restrict__ cur, uint8_t* __restrict__ out, int nx, int ny,
                                                      int strips, unsigned* __restrict__ status)
 {
+    const gb::BlockId bid = gb::grid_wait();
     extern __shared__ __align__(128) unsigned char ub[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(ub + UB_RING * UB_SLOT);
     const int t = threadIdx.x;
-    const int strip = blockIdx.x % strips, band = blockIdx.x / strips;
+    const int strip = bid.x % strips, band = bid.x / strips;
     const int x0 = strip * UB_W, w = min(UB_W, nx - x0);
     const int j0 = band * UB_ROWS, j1 = min(j0 + UB_ROWS, ny);
     const int rbase = j0 - 1;  // row of slot 0, first use
@@ -253,9 +255,10 @@ template <int RULE>
 __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restrict__ cur, uint32_t* __restrict__ out,
                                                         int nw, int ny, int strips, int rows, int tasks)
 {
+    const gb::BlockId bid = gb::grid_wait();
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += nwarps) {
+    for (int task = (bid.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += nwarps) {
         const int strip = task % strips, seg = task / strips;
         const int xw = strip * 32 + lane;
         const bool active = xw < nw;
@@ -344,13 +347,14 @@ __global__ void __launch_bounds__(TB_WARPS * 32) life_bits_tb(const uint32_t* __
                                                                uint32_t* __restrict__ outCur, uint32_t* __restrict__ outOld,
                                                                int nx, int nw, int ny, int tiles_x, int tiles, int steps)
 {
+    const gb::BlockId bid = gb::grid_wait();
     constexpr int RRMAX = ROWS + 2 * TB_STEPS;
     extern __shared__ uint32_t tbsm[];  // two (RRMAX x 32)-word planes
     uint32_t(*sA)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm);
     uint32_t(*sB)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm + RRMAX * 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rr = ROWS + 2 * steps;  // rows of the region
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (int tile = bid.x; tile < tiles; tile += gridDim.x) {
         const int tx = tile % tiles_x, ty = tile / tiles_x;
         int wx = (tx * 30 - 1 + lane) % nw;
         if (wx < 0) wx += nw;
@@ -429,9 +433,10 @@ __device__ __forceinline__ uint32_t four_bytes(uint32_t b)  // bits 0..3 -> byte
 __global__ void life_pack(const uint8_t* __restrict__ cellsA, const uint8_t* __restrict__ cellsB, uint32_t* __restrict__ bitsA,
                           uint32_t* __restrict__ bitsB, size_t nwords)
 {
-    const uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
-    uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
-    size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const gb::BlockId bid = gb::grid_wait();
+    const uint8_t* __restrict__ cells = bid.y ? cellsB : cellsA;
+    uint32_t* __restrict__ bits = bid.y ? bitsB : bitsA;
+    size_t w = (size_t)bid.x * blockDim.x + threadIdx.x;
     if (w >= nwords) return;
     const uint4* p = reinterpret_cast<const uint4*>(cells + w * 32);
     uint4 a = __ldg(p), b = __ldg(p + 1);
@@ -444,9 +449,10 @@ __global__ void life_pack(const uint8_t* __restrict__ cellsA, const uint8_t* __r
 __global__ void life_unpack(const uint32_t* __restrict__ bitsA, const uint32_t* __restrict__ bitsB, uint8_t* __restrict__ cellsA,
                             uint8_t* __restrict__ cellsB, size_t nwords)
 {
-    const uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
-    uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
-    size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const gb::BlockId bid = gb::grid_wait();
+    const uint32_t* __restrict__ bits = bid.y ? bitsB : bitsA;
+    uint8_t* __restrict__ cells = bid.y ? cellsB : cellsA;
+    size_t w = (size_t)bid.x * blockDim.x + threadIdx.x;
     if (w >= nwords) return;
     uint32_t b = __ldg(bits + w), v[8];
 #pragma unroll
@@ -479,10 +485,11 @@ __global__ void __launch_bounds__(256) life_pack_rows(const uint8_t* __restrict_
                                                       uint32_t* __restrict__ bitsA, uint32_t* __restrict__ bitsB, int nx, int nw,
                                                       size_t nwords, size_t ncells)
 {
-    const uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
-    uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
+    const gb::BlockId bid = gb::grid_wait();
+    const uint8_t* __restrict__ cells = bid.y ? cellsB : cellsA;
+    uint32_t* __restrict__ bits = bid.y ? bitsB : bitsA;
     int col;
-    const size_t first = (size_t)blockIdx.x * 256, row0 = block_origin(first, nw, &col);
+    const size_t first = (size_t)bid.x * 256, row0 = block_origin(first, nw, &col);
     const size_t id = first + threadIdx.x;
     if (id >= nwords) return;
     const unsigned q = (unsigned)(col + threadIdx.x) / (unsigned)nw, w = (unsigned)(col + threadIdx.x) - q * (unsigned)nw;
@@ -509,11 +516,12 @@ __global__ void __launch_bounds__(256) life_unpack_rows(const uint32_t* __restri
                                                         uint8_t* __restrict__ cellsA, uint8_t* __restrict__ cellsB, int nx, int nw,
                                                         size_t ncells)
 {
-    const uint32_t* __restrict__ bits = blockIdx.y ? bitsB : bitsA;
-    uint8_t* __restrict__ cells = blockIdx.y ? cellsB : cellsA;
-    // the block's 4096 cells start at the plane's byte 4096 * blockIdx.x - lead, a 16-byte boundary
+    const gb::BlockId bid = gb::grid_wait();
+    const uint32_t* __restrict__ bits = bid.y ? bitsB : bitsA;
+    uint8_t* __restrict__ cells = bid.y ? cellsB : cellsA;
+    // the block's 4096 cells start at the plane's byte 4096 * bid.x - lead, a 16-byte boundary
     const int lead = (int)(reinterpret_cast<uintptr_t>(cells) & 15u);
-    const size_t begin = (size_t)blockIdx.x * 4096;
+    const size_t begin = (size_t)bid.x * 4096;
     const int skip = begin == 0 ? lead : 0;  // bytes of the first block that lie before the plane
     int col;
     const size_t row0 = block_origin(begin + skip - lead, nx, &col);
@@ -542,18 +550,20 @@ __global__ void __launch_bounds__(256) life_unpack_rows(const uint32_t* __restri
 // leaves it, corners included).
 __global__ void life_from_i32(const int32_t* __restrict__ f, int px, int g, uint8_t* __restrict__ cells, int nx, int ny)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = bid.x * blockDim.x + threadIdx.x;
     if (i >= nx) return;
-    for (int j = blockIdx.y; j < ny; j += gridDim.y) cells[(size_t)j * nx + i] = __ldg(f + (size_t)(j + g) * px + i + g) != 0;
+    for (int j = bid.y; j < ny; j += gridDim.y) cells[(size_t)j * nx + i] = __ldg(f + (size_t)(j + g) * px + i + g) != 0;
 }
 
 __global__ void life_to_i32(const uint8_t* __restrict__ cells, int nx, int ny, int32_t* __restrict__ f, int px, int g)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const gb::BlockId bid = gb::grid_wait();
+    const int i = bid.x * blockDim.x + threadIdx.x;
     if (i >= nx + 2 * g) return;
     int si = (i - g) % nx;
     if (si < 0) si += nx;
-    for (int j = blockIdx.y; j < ny + 2 * g; j += gridDim.y) {
+    for (int j = bid.y; j < ny + 2 * g; j += gridDim.y) {
         int sj = (j - g) % ny;
         if (sj < 0) sj += ny;
         f[(size_t)j * px + i] = __ldg(cells + (size_t)sj * nx + si);
@@ -563,8 +573,9 @@ __global__ void life_to_i32(const uint8_t* __restrict__ cells, int nx, int ny, i
 // Population: popcount over 32-bit words (u8 cells are 0/1, so popc of 4 bytes = live bytes).
 __global__ void popcount_words(const uint32_t* __restrict__ words, size_t n, unsigned long long* __restrict__ out)
 {
+    const gb::BlockId bid = gb::grid_wait();
     unsigned long long s = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    for (size_t i = (size_t)bid.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         s += __popc(__ldg(words + i));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o);
@@ -582,6 +593,7 @@ __global__ void popcount_words(const uint32_t* __restrict__ words, size_t n, uns
 // tail of a byte array whose length is not a multiple of 4
 __global__ void popcount_tail(const uint8_t* __restrict__ p, int n, unsigned long long* __restrict__ out)
 {
+    gb::grid_wait();
     unsigned long long s = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) s += p[i];
     if (s) atomicAdd(out, s);
@@ -612,7 +624,7 @@ int launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStre
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TB_WARPS * 32, smem) != cudaSuccess || per_sm < 1) per_sm = 3;
     const int grid = std::max(1, std::min(tiles, per_sm * gb::sm_count()));
-    kern<<<grid, TB_WARPS * 32, smem, st>>>(in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, tiles, steps);
+    gb::launch(kern, grid, TB_WARPS * 32, smem, st, in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, tiles, steps);
     return APPFIS_GB_OK;
 }
 
@@ -687,13 +699,13 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
             ci = gens & 1;
             int rc;
             if (nx % 32) {
-                life_pack_rows<<<wgrid, 256, 0, st>>>(buf[0], buf[1], w, w + plane, nx, nw, words, cells);
+                gb::launch(life_pack_rows, wgrid, 256, 0, st, buf[0], buf[1], w, w + plane, nx, nw, words, cells);
                 rc = run_tb<RULE, true>(pair, last, nx, ny, gens, launches, st);
-                life_unpack_rows<<<dim3(gb::ceil_div(cells + 15, 4096), 2), 256, 0, st>>>(last.p[0], last.p[1], buf[ci], buf[1 - ci], nx, nw, cells);
+                gb::launch(life_unpack_rows, dim3(gb::ceil_div(cells + 15, 4096), 2), 256, 0, st, last.p[0], last.p[1], buf[ci], buf[1 - ci], nx, nw, cells);
             } else {
-                life_pack<<<wgrid, 256, 0, st>>>(buf[0], buf[1], w, w + plane, words);
+                gb::launch(life_pack, wgrid, 256, 0, st, buf[0], buf[1], w, w + plane, words);
                 rc = run_tb<RULE, false>(pair, last, nx, ny, gens, launches, st);
-                life_unpack<<<dim3(wgrid.x, 2), 256, 0, st>>>(last.p[0], last.p[1], buf[ci], buf[1 - ci], words);
+                gb::launch(life_unpack, dim3(wgrid.x, 2), 256, 0, st, last.p[0], last.p[1], buf[ci], buf[1 - ci], words);
             }
             gb::scratch_free(ws, st);
             GB_TRY(rc);
@@ -709,13 +721,13 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
         const int strips = (nx + UB_W - 1) / UB_W;
         const unsigned grid = (unsigned)strips * gb::ceil_div(ny, UB_ROWS);
         for (int g = 0; g < gens; g++) {
-            life_u8_bulk<RULE><<<grid, 256, UB_SMEM, st>>>(buf[ci], buf[1 - ci], nx, ny, strips, status);
+            gb::launch(life_u8_bulk<RULE>, grid, 256, UB_SMEM, st, buf[ci], buf[1 - ci], nx, ny, strips, status);
             ci = 1 - ci;
         }
     } else {
         dim3 blk(32, 8), grd(gb::ceil_div(nx, 32), gb::ceil_div(ny, 8));
         for (int g = 0; g < gens; g++) {
-            life_u8_generic<RULE><<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny);
+            gb::launch(life_u8_generic<RULE>, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny);
             ci = 1 - ci;
         }
     }
@@ -766,7 +778,7 @@ int run_bits(uint32_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStr
     while (srows > 4 && (long long)strips * ((ny + srows - 1) / srows) < 24LL * gb::sm_count()) srows /= 2;
     const int tasks = strips * ((ny + srows - 1) / srows);
     const unsigned grid = resident_grid(life_bits_sweep<RULE>, tasks);
-    for (int g = 0; g < gens; g++) life_bits_sweep<RULE><<<grid, 256, 0, st>>>(buf[g & 1], buf[1 - (g & 1)], nw, ny, strips, srows, tasks);
+    for (int g = 0; g < gens; g++) gb::launch(life_bits_sweep<RULE>, grid, 256, 0, st, buf[g & 1], buf[1 - (g & 1)], nw, ny, strips, srows, tasks);
     return gb::launched("life_bits sweep");
 }
 
@@ -788,11 +800,11 @@ int population_u8(const uint8_t* cells, int64_t n, int64_t* dev_count, cudaStrea
     size_t nw = (size_t)n / 4;
     if (nw) {
         unsigned grid = (unsigned)std::min<size_t>(gb::ceil_div(nw, 256), (size_t)gb::sm_count() * 8);
-        popcount_words<<<grid, 256, 0, st>>>(reinterpret_cast<const uint32_t*>(cells), nw,
+        gb::launch(popcount_words, grid, 256, 0, st, reinterpret_cast<const uint32_t*>(cells), nw,
                                              reinterpret_cast<unsigned long long*>(dev_count));
     }
     if (n % 4)
-        popcount_tail<<<1, 32, 0, st>>>(cells + nw * 4, (int)(n % 4), reinterpret_cast<unsigned long long*>(dev_count));
+        gb::launch(popcount_tail, 1, 32, 0, st, cells + nw * 4, (int)(n % 4), reinterpret_cast<unsigned long long*>(dev_count));
     return gb::launched("life population");
 }
 
@@ -826,7 +838,7 @@ int appfis_gb_life_pack(const uint8_t* cells, uint32_t* bits, int nx, int ny, vo
     if (!cells || !bits || nx < 1 || ny < 1 || nx % 32) return gb::fail(APPFIS_GB_EINVAL, "life_pack: bad arguments");
     if (reinterpret_cast<uintptr_t>(cells) & 15) return gb::fail(APPFIS_GB_EINVAL, "life_pack: cells must be 16-byte aligned");
     size_t nw = (size_t)nx * ny / 32;
-    life_pack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(cells, cells, bits, bits, nw);
+    gb::launch(life_pack, gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream), cells, cells, bits, bits, nw);
     return gb::launched("life_pack");
 }
 
@@ -835,7 +847,7 @@ int appfis_gb_life_unpack(const uint32_t* bits, uint8_t* cells, int nx, int ny, 
     if (!cells || !bits || nx < 1 || ny < 1 || nx % 32) return gb::fail(APPFIS_GB_EINVAL, "life_unpack: bad arguments");
     if (reinterpret_cast<uintptr_t>(cells) & 15) return gb::fail(APPFIS_GB_EINVAL, "life_unpack: cells must be 16-byte aligned");
     size_t nw = (size_t)nx * ny / 32;
-    life_unpack<<<gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream)>>>(bits, bits, cells, cells, nw);
+    gb::launch(life_unpack, gb::ceil_div(nw, 256), 256, 0, gb::as_stream(stream), bits, bits, cells, cells, nw);
     return gb::launched("life_unpack");
 }
 
@@ -844,7 +856,7 @@ int appfis_gb_life_from_i32(const int32_t* padded, int px, int ghost, uint8_t* c
     if (!padded || !cells || nx < 1 || ny < 1 || ghost < 0 || ghost > nx || ghost > ny || px < nx + 2 * ghost)
         return gb::fail(APPFIS_GB_EINVAL, "life_from_i32: bad arguments");
     dim3 grd(gb::ceil_div(nx, 256), std::min(ny, 65535));
-    life_from_i32<<<grd, 256, 0, gb::as_stream(stream)>>>(padded, px, ghost, cells, nx, ny);
+    gb::launch(life_from_i32, grd, 256, 0, gb::as_stream(stream), padded, px, ghost, cells, nx, ny);
     return gb::launched("life_from_i32");
 }
 
@@ -853,7 +865,7 @@ int appfis_gb_life_to_i32(const uint8_t* cells, int nx, int ny, int32_t* padded,
     if (!padded || !cells || nx < 1 || ny < 1 || ghost < 0 || ghost > nx || ghost > ny || px < nx + 2 * ghost)
         return gb::fail(APPFIS_GB_EINVAL, "life_to_i32: bad arguments");
     dim3 grd(gb::ceil_div(nx + 2 * ghost, 256), std::min(ny + 2 * ghost, 65535));
-    life_to_i32<<<grd, 256, 0, gb::as_stream(stream)>>>(cells, nx, ny, padded, px, ghost);
+    gb::launch(life_to_i32, grd, 256, 0, gb::as_stream(stream), cells, nx, ny, padded, px, ghost);
     return gb::launched("life_to_i32");
 }
 
@@ -871,7 +883,7 @@ int appfis_gb_life_population_bits(const uint32_t* bits, int64_t nwords, int64_t
     GB_CUDA(cudaMemsetAsync(dev_count, 0, sizeof(int64_t), st));
     if (nwords) {
         unsigned grid = (unsigned)std::min<size_t>(gb::ceil_div((size_t)nwords, 256), (size_t)gb::sm_count() * 8);
-        popcount_words<<<grid, 256, 0, st>>>(bits, (size_t)nwords, reinterpret_cast<unsigned long long*>(dev_count));
+        gb::launch(popcount_words, grid, 256, 0, st, bits, (size_t)nwords, reinterpret_cast<unsigned long long*>(dev_count));
     }
     return gb::launched("life_population_bits");
 }

@@ -65,20 +65,21 @@ __global__ void __launch_bounds__(256) reduce_box(const T* __restrict__ f, int p
                                                   int z0, int z1, typename Acc<T>::type* __restrict__ partials,
                                                   unsigned* __restrict__ ticket, void* __restrict__ result)
 {
+    const gb::BlockId bid = gb::grid_wait();
     typedef typename Acc<T>::type A;
     __shared__ A sh[32];
     __shared__ bool last;
     A v = seed<T, OP>();
     const int nyb = y1 - y0;
     const long long rows = (long long)nyb * (z1 - z0);
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
+    for (long long r = bid.x; r < rows; r += gridDim.x) {
         const int j = y0 + (int)(r % nyb), k = z0 + (int)(r / nyb);
         const T* row = f + ((size_t)k * py + j) * (size_t)px;
         for (int i = x0 + threadIdx.x; i < x1; i += blockDim.x) v = combine<OP>(v, (A)__ldg(row + i));
     }
     v = block_reduce<OP>(v, seed<T, OP>(), sh);
     if (threadIdx.x == 0) {
-        partials[blockIdx.x] = v;
+        partials[bid.x] = v;
         __threadfence();
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
@@ -112,13 +113,13 @@ int launch_reduce(const void* field, int px, int py, const int* b, int op, void*
     const T* f = reinterpret_cast<const T*>(field);
     switch (op) {
     case APPFIS_GB_MAX:
-        reduce_box<T, APPFIS_GB_MAX><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_MAX>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
         break;
     case APPFIS_GB_MIN:
-        reduce_box<T, APPFIS_GB_MIN><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_MIN>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
         break;
     default:
-        reduce_box<T, APPFIS_GB_SUM><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_SUM>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
     }
     return gb::launched("reduce_box");
 }
@@ -177,13 +178,13 @@ int launch_reduce_noalloc(const void* field, int px, int py, const int* b, int o
     const T* f = reinterpret_cast<const T*>(field);
     switch (op) {
     case APPFIS_GB_MAX:
-        reduce_box<T, APPFIS_GB_MAX><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_MAX>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
         break;
     case APPFIS_GB_MIN:
-        reduce_box<T, APPFIS_GB_MIN><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_MIN>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
         break;
     default:
-        reduce_box<T, APPFIS_GB_SUM><<<grid, RED_THREADS, 0, st>>>(f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+        gb::launch(reduce_box<T, APPFIS_GB_SUM>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
     }
     return gb::launched("reduce_box (fixed scratch)");
 }

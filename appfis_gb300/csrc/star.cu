@@ -54,6 +54,7 @@ template <class T, int MODE, int RY>
 __global__ void __launch_bounds__(256) star_r4_sweep(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz,
                                                       int px, int py, int kz, float coeff, StarW wt)
 {
+    const gb::BlockId bid = gb::grid_wait();
     constexpr int NTY = 8;          // thread rows of the block (32 x 8 threads)
     constexpr int TY = NTY * RY;    // tile rows: each thread owns RY consecutive rows
     constexpr int SW = TX + 2 * R;  // shared plane width
@@ -62,8 +63,8 @@ __global__ void __launch_bounds__(256) star_r4_sweep(const T* __restrict__ in, T
     constexpr int HPT = (NHALO + 255) / 256;        // halo values per thread per plane
     __shared__ float tile[2][SH * SW];
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * TX + tx;
-    const int x0 = R + blockIdx.x * TX, y0 = R + blockIdx.y * TY;
-    const int k0 = R + blockIdx.z * kz, k1 = min(k0 + kz, nz + R);
+    const int x0 = R + bid.x * TX, y0 = R + bid.y * TY;
+    const int k0 = R + bid.z * kz, k1 = min(k0 + kz, nz + R);
     const int xe = nx + 2 * R, ye = ny + 2 * R;  // padded extents
     const size_t plane = (size_t)px * py;
     const int x = x0 + tx, yb = y0 + ty * RY;
@@ -205,10 +206,11 @@ template <class T, int MODE>
 __global__ void __launch_bounds__(256) star_r4_vec(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz, int px,
                                                     int py, int kz, float coeff, StarW wt)
 {
+    const gb::BlockId bid = gb::grid_wait();
     __shared__ __align__(16) float tile[2][VSH * VSW];
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 16 + tx;
-    const int x0 = R + blockIdx.x * VTX, y0 = R + blockIdx.y * VTY;
-    const int k0 = R + blockIdx.z * kz, k1 = min(k0 + kz, nz + R);
+    const int x0 = R + bid.x * VTX, y0 = R + bid.y * VTY;
+    const int k0 = R + bid.z * kz, k1 = min(k0 + kz, nz + R);
     const int xe = nx + 2 * R, ye = ny + 2 * R;
     const size_t plane = (size_t)px * py;
     const int x = x0 + VX * tx, y = y0 + ty;
@@ -394,15 +396,16 @@ __global__ void __launch_bounds__(128, VXT == 4 ? (TRY == 2 ? 4 : 2) : 6) star_r
                                                                      StarW wt, unsigned* __restrict__ status,
                                                                      unsigned long long wait_ns, unsigned shortfall)
 {
+    const gb::BlockId bid = gb::grid_wait();
     namespace f2 = gb::f2;
     typedef TmaStar<T, VXT, TRY> Lay;
     constexpr int SW = Lay::SW, TTY = Lay::TTY;
     extern __shared__ __align__(128) unsigned char tsm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(tsm + TNS * Lay::SLOT);
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 16 + tx;
-    const int bx0 = blockIdx.x * Lay::TX, by0 = blockIdx.y * TTY;  // box origin (padded coordinates)
+    const int bx0 = bid.x * Lay::TX, by0 = bid.y * TTY;  // box origin (padded coordinates)
     const int x = R + bx0 + VXT * tx, y = R + by0 + TRY * ty;       // this thread's first point
-    const int k0 = R + blockIdx.z * kz, k1 = min(k0 + kz, nz + R);
+    const int k0 = R + bid.z * kz, k1 = min(k0 + kz, nz + R);
     const int plast = k1 + R - 1;                                   // last plane the chunk reads
     const size_t plane = (size_t)px * py;
     if (gb::tma::smem_u32(tsm) & 127u) {
@@ -620,15 +623,16 @@ __global__ void __launch_bounds__(TbStar<T, TY>::NT, 1) star_r4_tb2(const __grid
                                                                     int ny, int nz, int px, int py, int kz, float coeff, StarW wt,
                                                                     unsigned* __restrict__ status, unsigned long long wait_ns)
 {
+    const gb::BlockId bid = gb::grid_wait();
     typedef TbStar<T, TY> Lay;
     extern __shared__ __align__(128) unsigned char tsm[];
     float* l1 = reinterpret_cast<float*>(tsm + TB_NS * Lay::SLOT);
     uint64_t* bar = reinterpret_cast<uint64_t*>(tsm + TB_NS * Lay::SLOT + TB_L1 * Lay::L1S);
     const int t = threadIdx.x, tx = t % (Lay::RX / 4), ty = t / (Lay::RX / 4);
-    const int rx0 = blockIdx.x * Lay::OX, ry0 = blockIdx.y * TY;     // region origin (padded coordinates)
+    const int rx0 = bid.x * Lay::OX, ry0 = bid.y * TY;     // region origin (padded coordinates)
     const int bx0 = rx0 - 2 * R, by0 = ry0 - R;                       // box origin
     const int x = rx0 + 4 * tx, y = ry0 + ty;                         // this thread's first point, its row
-    const int k0 = R + blockIdx.z * kz, k1 = min(k0 + kz, nz + R);
+    const int k0 = R + bid.z * kz, k1 = min(k0 + kz, nz + R);
     const int pbase = k0 - 2 * R, plast = k1 + 2 * R - 1;             // input planes of the chunk
     const bool out_thread = tx >= 1 && tx <= Lay::OX / 4 && ty >= R && ty < R + TY;
     const size_t plane = (size_t)px * py;
@@ -769,7 +773,7 @@ int run_star_tb2(T** buf, int nx, int ny, int nz, int pitch, int pairs, int mode
     dim3 blk(Lay::NT), grd(gb::ceil_div(nx, Lay::OX), gb::ceil_div(ny, TY), gb::ceil_div(nz, tkz));
     int ci = 0;
     for (int it = 0; it < pairs; it++) {
-        kern<<<grd, blk, smem, st>>>(maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, tkz, coeff, w, status, 1000000000ull);
+        gb::launch(kern, grd, blk, smem, st, maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, tkz, coeff, w, status, 1000000000ull);
         ci = 1 - ci;
     }
     return gb::launched("star_r4_tb2");
@@ -780,7 +784,7 @@ void launch_star(const T* in, T* out, int nx, int ny, int nz, int px, int kz, fl
 {
     dim3 blk(TX, 8), grd(gb::ceil_div(nx, TX), gb::ceil_div(ny, 8 * RY), gb::ceil_div(nz, kz));
     static_assert(RY >= 1, "rows per thread");
-    star_r4_sweep<T, MODE, RY><<<grd, blk, 0, st>>>(in, out, nx, ny, nz, px, ny + 2 * R, kz, coeff, w);
+    gb::launch(star_r4_sweep<T, MODE, RY>, grd, blk, 0, st, in, out, nx, ny, nz, px, ny + 2 * R, kz, coeff, w);
 }
 
 template <class T, int VXT, int TRY = 2>
@@ -819,7 +823,7 @@ int run_star_tma(T** buf, int nx, int ny, int nz, int pitch, int iters, int mode
     }
     int ci = 0;
     for (int it = 0; it < iters; it++) {
-        kern<<<grd, blk, smem, st>>>(maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, tkz, coeff, w, status, wait_ns, shortfall);
+        gb::launch(kern, grd, blk, smem, st, maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, tkz, coeff, w, status, wait_ns, shortfall);
         wait_ns = 1000000000ull;
         shortfall = 0;
         ci = 1 - ci;
@@ -1015,8 +1019,8 @@ int run_star(T* a, T* b, int nx, int ny, int nz, int pitch, int iters, int mode,
     for (int it = 0; it < iters; it++) {
         if (tile == APPFIS_GB_STAR_VEC) {
             dim3 blk(16, 16), grd(gb::ceil_div(nx, VTX), gb::ceil_div(ny, VTY), gb::ceil_div(nz, kz));
-            if (mode == 0) star_r4_vec<T, 0><<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, kz, coeff, w);
-            else star_r4_vec<T, 1><<<grd, blk, 0, st>>>(buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, kz, coeff, w);
+            if (mode == 0) gb::launch(star_r4_vec<T, 0>, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, kz, coeff, w);
+            else gb::launch(star_r4_vec<T, 1>, grd, blk, 0, st, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, kz, coeff, w);
         } else if (mode == 0) {
             if (tile == APPFIS_GB_STAR_SCALAR2) launch_star<T, 0, 2>(buf[ci], buf[1 - ci], nx, ny, nz, pitch, kz, coeff, w, st);
             else launch_star<T, 0, 4>(buf[ci], buf[1 - ci], nx, ny, nz, pitch, kz, coeff, w, st);
