@@ -3,7 +3,7 @@
 // for the per-face / per-cell arithmetic and the reference it follows.
 //
 // One cooperative launch advances a batch of independent domains of uneven sizes to t_end.
-// Work items are strips (SCOLS interior columns x ROWS rows) of all domains; in each phase a warp
+// Work items are strips (SCOLS interior columns x Params::rows rows) of all domains; in each phase a warp
 // takes its first strip by index and the rest one at a time from a counter (a strip's cost
 // follows the water, so a fixed stride leaves some warps with far more wet strips than others).
 // Each step is phase A (wet/dry fix of the previous step + CFL dt, min per domain) and phase B
@@ -54,6 +54,7 @@ struct Params {
     double dx, cn, hextra, t_end, print_interval, time_step;
     float fdx, fcn, fhextra;  // dx, cn, hextra rounded to float once on the host (float kernel)
     int max_steps, ndom;
+    int rows;  // rows per strip
     long long total_strips;
     double* dtlog;  // [ndom][max_steps] or null
     unsigned char* zc;  // [2][total_strips] dry-step counters (null: every strip every step)
@@ -143,6 +144,25 @@ __device__ __forceinline__ bool is_active(const Ctl* ctl, int cur, int d, const 
     return ctl->simtime[cur][d] < p.t_end && ctl->steps[cur][d] < p.max_steps;
 }
 
+// Commits domain d's scalars of the step that starts now (dt, or what it was for a domain that takes
+// no step) into the other half, and resets dtbits[slot], which the steps around this one do not use.
+// Block 0 does it at the step's start, one thread per domain: nobody reads that half before the next
+// grid barrier (in one thread at the step's end, domain after domain, it held up every step:
+// about 1 us a domain).
+__device__ __forceinline__ void commit(Ctl* ctl, int cur, int slot, int d, bool active, double dt, const Params& p, double big)
+{
+    const double t = ctl->simtime[cur][d];
+    const int id = ctl->pid[cur][d], n = ctl->steps[cur][d];
+    // a collapsed (below 1e-9 of the step scale) or NaN time step stops the run
+    if (active && !(dt > 1e-9 * p.time_step)) atomicExch(&ctl->error, 2);
+    const double st = active ? t + dt : t;
+    if (active && p.dtlog) p.dtlog[(size_t)d * p.max_steps + n] = dt;
+    ctl->simtime[1 - cur][d] = st;
+    ctl->pid[1 - cur][d] = active && st >= p.print_interval * (id + 1) ? id + 1 : id;
+    ctl->steps[1 - cur][d] = active ? n + 1 : n;
+    ctl->dtbits[slot][d] = (unsigned long long)__double_as_longlong(big);
+}
+
 // ---------------------------------------------------------------- phase A: fix + dt
 // The domain descriptor arrives by value (registers): read through the shared-memory copy, every
 // field would be reloaded after each global store, which the compiler cannot prove disjoint.
@@ -159,7 +179,7 @@ __device__ void phase_a(const Dom<T> D, Ctl* ctl, int slot, int d, long long loc
     const int lane = threadIdx.x & 31;
     const int loc = (int)local, sy = loc / D.strips_x, sx = loc - sy * D.strips_x;  // 32-bit: a domain has < 2^31 strips
     const int i = sx * SC + lane - LO + 1;  // lanes LO..LO+SC-1: the strip's interior columns
-    const int j0 = 1 + sy * ROWS, j1 = min(j0 + ROWS, D.ny + 1);
+    const int j0 = 1 + sy * p.rows, j1 = min(j0 + p.rows, D.ny + 1);
     const T* __restrict__ h = D.h[b];
     T* __restrict__ qx = D.qx[b];
     T* __restrict__ qy = D.qy[b];
@@ -249,7 +269,7 @@ __device__ bool phase_b(const Dom<T> D, long long local, int b, T dt, const Para
     const int lane = threadIdx.x & 31;
     const int loc = (int)local, sy = loc / D.strips_x, sx = loc - sy * D.strips_x;  // 32-bit: a domain has < 2^31 strips
     const int i = sx * SCOLS + lane;
-    const int j0 = 1 + sy * ROWS, j1 = min(j0 + ROWS, D.ny + 1);
+    const int j0 = 1 + sy * p.rows, j1 = min(j0 + p.rows, D.ny + 1);
     const bool own = lane >= 1 && lane <= SCOLS && i <= D.nx;  // cells this lane updates
     const bool xface = lane <= SCOLS && i <= D.nx;             // face i|i+1 is needed
     const T dx = typed<T>(p.dx, p.fdx), hextra = typed<T>(p.hextra, p.fhextra);
@@ -324,12 +344,12 @@ __device__ bool phase_b(const Dom<T> D, long long local, int b, T dt, const Para
 // dry for two steps (both state buffers hold zeros there) and its four neighbour strips of the
 // same domain are dry in the step's input.
 template <class T>
-__device__ __forceinline__ bool strip_idle(const Dom<T>& D, const unsigned char* zin, long long s)
+__device__ __forceinline__ bool strip_idle(const Dom<T>& D, const unsigned char* zin, long long s, int rows)
 {
     if (zin[s] < 2) return false;
     const long long local = s - D.strip0;
     const int loc = (int)local, sy = loc / D.strips_x, sx = loc - sy * D.strips_x;  // 32-bit: a domain has < 2^31 strips
-    const int sy_n = (D.ny + ROWS - 1) / ROWS;
+    const int sy_n = (D.ny + rows - 1) / rows;
     if (sx > 0 && zin[s - 1] == 0) return false;
     if (sx + 1 < D.strips_x && zin[s + 1] == 0) return false;
     if (sy > 0 && zin[s - D.strips_x] == 0) return false;
@@ -400,7 +420,7 @@ __device__ void apply_sources(const Dom<T>& D, const SrcDev& S, Ctl* ctl, int cu
         const int j = S.cells[s] / (D.nx + 2), i = S.cells[s] - j * (D.nx + 2);
         T* c = h + (size_t)j * D.px + i;
         *c = (T)((double)*c + hs);
-        if (zwet) zwet[D.strip0 + (long long)((j - 1) / ROWS) * D.strips_x + (i - 1) / SCOLS] = 0;
+        if (zwet) zwet[D.strip0 + (long long)((j - 1) / p.rows) * D.strips_x + (i - 1) / SCOLS] = 0;
     }
 }
 
@@ -450,16 +470,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             const bool run = active && dt > 1e-9 * p.time_step;
             dc.dt[d] = (T)dt;
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (run ? 4 : 0));
+            if (blockIdx.x == 0) commit(ctl, cur, 1 - cur, d, active, dt, p, big);
         }
-        if (!__syncthreads_or(active)) {
-            if (blockIdx.x == 0 && threadIdx.x == 0)  // leave the final scalars in both halves
-                for (int d = 0; d < p.ndom; d++) {
-                    ctl->simtime[1 - cur][d] = ctl->simtime[cur][d];
-                    ctl->pid[1 - cur][d] = ctl->pid[cur][d];
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d];
-                }
-            return;
-        }
+        if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
         // phase B
         for_strips(&ctl->ticketb[cur], warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
@@ -468,7 +481,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
                 const unsigned char* zin = p.zc + (size_t)cur * p.total_strips;
                 unsigned char* zout = p.zc + (size_t)(1 - cur) * p.total_strips;
                 const unsigned char z = zin[s];
-                if (!(f & 4) || strip_idle(doms[d], zin, s)) {  // unchanged state
+                if (!(f & 4) || strip_idle(doms[d], zin, s, p.rows)) {  // unchanged state
                     if (lane == 0) zout[s] = z;
                     return;
                 }
@@ -478,27 +491,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
                 phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
             }
         });
-        if (blockIdx.x == 0 && threadIdx.x == 0) {  // commit the per-domain scalars of step n
-            for (int d = 0; d < p.ndom; d++) {
-                if (is_active(ctl, cur, d, p)) {
-                    const double dt = step_dt(ctl, cur, d, p, big);
-                    // a collapsed (below 1e-9 of the step scale) or NaN time step stops the run
-                    if (!(dt > 1e-9 * p.time_step)) atomicExch(&ctl->error, 2);
-                    const double st = ctl->simtime[cur][d] + dt;
-                    int pid = ctl->pid[cur][d];
-                    if (st >= p.print_interval * (pid + 1)) pid++;
-                    if (p.dtlog) p.dtlog[(size_t)d * p.max_steps + ctl->steps[cur][d]] = dt;
-                    ctl->simtime[1 - cur][d] = st;
-                    ctl->pid[1 - cur][d] = pid;
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d] + 1;
-                } else {
-                    ctl->simtime[1 - cur][d] = ctl->simtime[cur][d];
-                    ctl->pid[1 - cur][d] = ctl->pid[cur][d];
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d];
-                }
-                ctl->dtbits[1 - cur][d] = (unsigned long long)__double_as_longlong(big);
-            }
-        }
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ticketb[cur] = 0;  // next used two steps later, past a barrier
         if (p.srcs) {  // the point sources of step n, seen by the next step's wet/dry fix and dt
@@ -556,7 +548,7 @@ __device__ bool phase_bf(const Dom<T>& D, long long local, int b, T dt, const Pa
     const int lane = threadIdx.x & 31;
     const int loc = (int)local, sy = loc / D.strips_x, sx = loc - sy * D.strips_x;  // 32-bit: a domain has < 2^31 strips
     const int i = sx * FCOLS + lane - 1;
-    const int j0 = 1 + sy * ROWS, j1 = min(j0 + ROWS, D.ny + 1);  // owned rows j0 .. j1-1
+    const int j0 = 1 + sy * p.rows, j1 = min(j0 + p.rows, D.ny + 1);  // owned rows j0 .. j1-1
     const int nx = D.nx, ny = D.ny, px = D.px;
     const bool col = i >= 0 && i <= nx + 1;                            // a column of the padded domain
     const bool upd = lane >= 1 && lane <= 30 && i >= 1 && i <= nx;     // updates its cell
@@ -812,16 +804,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             const bool run = active && dt > 1e-9 * p.time_step;
             dc.dt[d] = (T)dt;
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (run ? 4 : 0));
+            if (blockIdx.x == 0) commit(ctl, cur, (n + 2) % 3, d, active, dt, p, big);
         }
-        if (!__syncthreads_or(active)) {
-            if (blockIdx.x == 0 && threadIdx.x == 0)  // leave the final scalars in both halves
-                for (int d = 0; d < p.ndom; d++) {
-                    ctl->simtime[1 - cur][d] = ctl->simtime[cur][d];
-                    ctl->pid[1 - cur][d] = ctl->pid[cur][d];
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d];
-                }
-            return;
-        }
+        if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
         const int dn = (n + 1) % 3;
         for_strips(&ctl->ticketb[cur], warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
@@ -830,7 +815,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
                 const unsigned char* zin = p.zc + (size_t)cur * p.total_strips;
                 unsigned char* zout = p.zc + (size_t)(1 - cur) * p.total_strips;
                 const unsigned char z = zin[s];
-                if (!(f & 4) || strip_idle(doms[d], zin, s)) {  // unchanged state, no fix, no dt
+                if (!(f & 4) || strip_idle(doms[d], zin, s, p.rows)) {  // unchanged state, no fix, no dt
                     if (lane == 0) zout[s] = z;
                     return;
                 }
@@ -841,26 +826,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
                 phase_bf<T, STAGED>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p, &ctl->dtbits[dn][d], &ring, d, ctl);
             }
         });
-        if (blockIdx.x == 0 && threadIdx.x == 0) {  // commit the per-domain scalars of step n
-            for (int d = 0; d < p.ndom; d++) {
-                if (is_active(ctl, cur, d, p)) {
-                    const double dt = step_dt_at(ctl, ds, cur, d, p, big);
-                    if (!(dt > 1e-9 * p.time_step)) atomicExch(&ctl->error, 2);
-                    const double st = ctl->simtime[cur][d] + dt;
-                    int pid = ctl->pid[cur][d];
-                    if (st >= p.print_interval * (pid + 1)) pid++;
-                    if (p.dtlog) p.dtlog[(size_t)d * p.max_steps + ctl->steps[cur][d]] = dt;
-                    ctl->simtime[1 - cur][d] = st;
-                    ctl->pid[1 - cur][d] = pid;
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d] + 1;
-                } else {
-                    ctl->simtime[1 - cur][d] = ctl->simtime[cur][d];
-                    ctl->pid[1 - cur][d] = ctl->pid[cur][d];
-                    ctl->steps[1 - cur][d] = ctl->steps[cur][d];
-                }
-                ctl->dtbits[(n + 2) % 3][d] = (unsigned long long)__double_as_longlong(big);
-            }
-        }
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ticketb[cur] = 0;  // next used two steps later, past a barrier
     }
@@ -868,7 +833,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
 
 static __global__ void flood_init_ctl(Ctl* ctl, int ndom, double big, double t0)
 {
-    const int d = threadIdx.x + blockIdx.x * blockDim.x;
+    gb::grid_wait();
+    const int d = threadIdx.x;  // one block
     if (d == 0) {
         ctl->bar_count = 0;
         ctl->bar_gen = 0;

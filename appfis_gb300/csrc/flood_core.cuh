@@ -11,7 +11,7 @@
 //   wet/dry momentum fix on the updated depth                           (:1095-1112)
 // seven kernel launches over five to sixteen arrays, plus a host round trip for dt.
 //
-// Here a step is two phases over strips of 32 columns x FLOOD_ROWS rows (one warp each):
+// Here a step is two phases over strips of 32 columns x 2 to 32 rows (one warp each):
 //   phase A: wet/dry fix of the previous step (in place on q), then the CFL dt of every wet
 //            cell, min-reduced per domain in double (atomicMin on the ordered bits);
 //   phase B: every face flux computed once (a lane's X face i|i+1 feeds its own rhs0 and, by
@@ -33,7 +33,6 @@
 
 namespace flood {
 
-constexpr int ROWS = 32;        // rows per strip
 constexpr int SCOLS = 30;       // interior columns per strip (a warp's lanes 1..30; lanes 0 and 31 hold the halo)
 constexpr int MAXD = 64;        // domains per batch
 

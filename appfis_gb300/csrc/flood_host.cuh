@@ -51,6 +51,7 @@ __global__ void flood_extract(Dom<T> D, int b, double* __restrict__ h, double* _
 
 static __global__ void flood_results(const Ctl* __restrict__ ctl, int ndom, int* steps, double* simtime, int* status)
 {
+    gb::grid_wait();
     const int d = threadIdx.x;
     if (d < ndom) {
         if (steps) steps[d] = ctl->steps[0][d];
@@ -65,7 +66,8 @@ static __global__ void flood_results(const Ctl* __restrict__ ctl, int ndom, int*
 
 // scols: interior columns per strip (SCOLS for the two-phase kernel, FCOLS for the fused one).
 template <class T>
-int make_table(const appfis_gb_flood_domain* doms, int ndom, std::vector<Dom<T>>& tab, long long& total, int scols = SCOLS)
+int make_table(const appfis_gb_flood_domain* doms, int ndom, std::vector<Dom<T>>& tab, long long& total, int scols = SCOLS,
+               int rows = 32)
 {
     total = 0;
     tab.resize(ndom);
@@ -88,7 +90,7 @@ int make_table(const appfis_gb_flood_domain* doms, int ndom, std::vector<Dom<T>>
         D.px = s.pitch;
         D.strips_x = (s.nx + scols - 1) / scols;
         D.strip0 = total;
-        total += (long long)D.strips_x * ((s.ny + ROWS - 1) / ROWS);
+        total += (long long)D.strips_x * ((s.ny + rows - 1) / rows);
     }
     return APPFIS_GB_OK;
 }
@@ -165,6 +167,30 @@ inline int upload_sources(const appfis_gb_flood_domain* doms, const appfis_gb_fl
     return APPFIS_GB_OK;
 }
 
+// Rows per strip for a batch on `warps` resident warps: the most that still leave each warp enough
+// strips.  A strip recomputes the faces (fused: the rows) around it, so tall strips do the least work;
+// but a step lasts as long as the slowest warp's wet strips, and a small batch has fewer strips
+// than the chip has warps.  Us per step with 32 / 16 / 8 / 4 / 2 rows:
+//   FP32 fused: 100^2 50 / 30 / 19 / 14 / 11; 300 x 1100 55 / 32 / 21 / 17 / 21; 1024^2 55 / 34 / 30 / 31 / 32;
+//     six domains of 3.6 M cells 101 / 73 / 63 / 64 / 88; 2 x 3000^2 180 / 174 / 187 / 241; 32 domains of 80 M cells 671 / 708 / 828 / 1085
+//   FP64: 100^2 1442 / 778 / 412 / 223 / 127; 1024^2 2377 / 1621 / 653 / 476 / 347; six 3090 / 1691 / 1141 / 1014 / 1025;
+//     2 x 3000^2 4224 / 3411 / 3214 / 3282 / 3874; 32 domains 14.87 / 14.23 / 14.34 / 15.40 / 18.13 ms
+// FP64 asks for more strips per warp: it has a third of the warps, and each is bound by the FP64 pipe.
+template <class T>
+int strip_rows(const appfis_gb_flood_domain* doms, int ndom, int scols, long long warps)
+{
+    constexpr bool f32 = std::is_same<T, float>::value;
+    const int rows[4] = {32, 16, 8, 4};
+    const double per_warp[4] = {f32 ? 8.0 : 512.0, f32 ? 8.0 : 64.0, f32 ? 4.0 : 48.0, f32 ? 0.8 : 24.0};
+    for (int k = 0; k < 4; k++) {
+        long long strips = 0;
+        for (int d = 0; d < ndom; d++)
+            strips += ((long long)doms[d].nx + scols - 1) / scols * (((long long)doms[d].ny + rows[k] - 1) / rows[k]);
+        if ((double)strips >= per_warp[k] * (double)warps) return rows[k];
+    }
+    return 2;
+}
+
 // Uploads the table, initialises the control block and launches the persistent kernel.
 template <class T>
 int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_params* prm, double* dev_dtlog, int* dev_steps,
@@ -182,9 +208,32 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     // form is faster (full sweep 21.2 against 22.9 s on the 32-domain batch)
     const bool fused = !any_src && !(prm->flags & APPFIS_GB_FLOOD_TWO_PHASE) &&
                        ((prm->flags & APPFIS_GB_FLOOD_FUSED) || std::is_same<T, float>::value);
+    const bool skip = (prm->flags & APPFIS_GB_FLOOD_SKIP_DRY) != 0;
+    const int scols = fused ? FCOLS : SCOLS;
     std::vector<Dom<T>> tab;
     long long total = 0;
-    GB_TRY(make_table<T>(doms, ndom, tab, total, fused ? FCOLS : SCOLS));
+    GB_TRY(make_table<T>(doms, ndom, tab, total, scols));  // checks the domains
+    // the fused FP32 full sweep stages its rows by TMA when every domain's arrays and rows are
+    // 16-byte aligned: 112.5 against 97.4 G cell-steps/s on the 32-domain batch.  With dry strips
+    // left out it loads them directly (324 against 319: a warp's strips are then scattered, and
+    // each one starts its ring from empty); so does UNSTAGED, or any other layout (same fields).
+    bool staged = fused && std::is_same<T, float>::value && !(prm->flags & APPFIS_GB_FLOOD_UNSTAGED) && !skip;
+    for (int d = 0; staged && d < ndom; d++) {
+        const appfis_gb_flood_domain& D = doms[d];
+        const void* a[8] = {D.h[0], D.h[1], D.qx[0], D.qx[1], D.qy[0], D.qy[1], D.dem, D.n2};
+        for (int k = 0; k < 8; k++) staged = staged && gb::aligned16(a[k]);
+        staged = staged && (D.pitch * sizeof(T)) % 16 == 0;
+    }
+    int per_sm = 0;
+    auto kern = staged  ? flood_fused<T, false, true>
+                : fused ? (skip ? flood_fused<T, true> : flood_fused<T, false>)
+                        : (skip ? flood_persistent<T, true> : flood_persistent<T, false>);
+    const int smem = staged ? FS_SMEM : 0;
+    if (staged) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+    if (per_sm < 1) return gb::fail(APPFIS_GB_ECUDA, "flood: kernel cannot be resident");
+    const int rows = strip_rows<T>(doms, ndom, scols, 8LL * per_sm * gb::sm_count());
+    GB_TRY(make_table<T>(doms, ndom, tab, total, scols, rows));
     void *wt, *hs;
     GB_TRY(gb::workspace(gb::WS_REDUCE, sizeof(Ctl) + sizeof(Dom<T>) * MAXD + 256, &wt));
     Ctl* ctl = reinterpret_cast<Ctl*>(wt);
@@ -194,7 +243,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     std::memcpy(hs, tab.data(), sizeof(Dom<T>) * ndom);
     GB_CUDA(cudaMemcpyAsync(dtab, hs, sizeof(Dom<T>) * ndom, cudaMemcpyHostToDevice, st));
     const double big = std::is_same<T, float>::value ? 3.402823466e38 : 1.7976931348623157e308;
-    flood_init_ctl<<<1, MAXD, 0, st>>>(ctl, ndom, big, prm->t_start);
+    gb::launch(flood_init_ctl, 1, MAXD, 0, st, ctl, ndom, big, prm->t_start);
     GB_TRY(gb::launched("flood_init_ctl"));
 
     Params p;
@@ -209,6 +258,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     p.time_step = prm->time_step;
     p.max_steps = prm->max_steps > 0 ? prm->max_steps : STEP_CAP;
     p.ndom = ndom;
+    p.rows = rows;
     p.total_strips = total;
     p.dtlog = prm->max_steps > 0 ? dev_dtlog : nullptr;
     p.zc = nullptr;
@@ -218,18 +268,6 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     p.wait_ns = 1000000000ull;
     p.tx_extra = 0;
     GB_TRY(upload_sources(doms, srcs, ndom, &p.srcs, st));
-    // the fused FP32 full sweep stages its rows by TMA when every domain's arrays and rows are
-    // 16-byte aligned: 112.5 against 97.4 G cell-steps/s on the 32-domain batch.  With dry strips
-    // left out it loads them directly (324 against 319: a warp's strips are then scattered, and
-    // each one starts its ring from empty); so does UNSTAGED, or any other layout (same fields).
-    bool staged = fused && std::is_same<T, float>::value && !(prm->flags & APPFIS_GB_FLOOD_UNSTAGED) &&
-                  !(prm->flags & APPFIS_GB_FLOOD_SKIP_DRY);
-    for (int d = 0; staged && d < ndom; d++) {
-        const Dom<T>& D = tab[d];
-        const void* a[8] = {D.h[0], D.h[1], D.qx[0], D.qx[1], D.qy[0], D.qy[1], D.dem, D.n2};
-        for (int k = 0; k < 8; k++) staged = staged && gb::aligned16(a[k]);
-        staged = staged && (D.px * sizeof(T)) % 16 == 0;
-    }
     if (staged) {
         std::vector<CUtensorMap> maps(8 * (size_t)ndom);
         for (int d = 0; d < ndom; d++) {
@@ -255,22 +293,13 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
         p.spin_limit = test_limit;
         p.stall_cta = 0;
     }
-    if (prm->flags & APPFIS_GB_FLOOD_SKIP_DRY) {
+    if (skip) {
         void* z;
         GB_TRY(gb::workspace(gb::WS_FLOOD_Z, 2 * (size_t)total, &z));
         GB_CUDA(cudaMemsetAsync(z, 0, 2 * (size_t)total, st));
         p.zc = reinterpret_cast<unsigned char*>(z);
     }
 
-    int dev = 0, per_sm = 0;
-    GB_CUDA(cudaGetDevice(&dev));
-    auto kern = staged  ? flood_fused<T, false, true>
-                : fused ? (p.zc ? flood_fused<T, true> : flood_fused<T, false>)
-                        : (p.zc ? flood_persistent<T, true> : flood_persistent<T, false>);
-    const int smem = staged ? FS_SMEM : 0;
-    if (staged) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
-    if (per_sm < 1) return gb::fail(APPFIS_GB_ECUDA, "flood: kernel cannot be resident");
     long long want = (total * 32 + 255) / 256;  // one warp per strip at most
     int grid = (int)std::min<long long>(want, (long long)per_sm * gb::sm_count());
     if (grid < 1) grid = 1;
@@ -286,7 +315,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     cfg.numAttrs = 1;
     const Dom<T>* cdt = dtab;
     GB_CUDA(cudaLaunchKernelEx(&cfg, kern, cdt, ctl, p));
-    flood_results<<<1, MAXD, 0, st>>>(ctl, ndom, dev_steps, dev_simtime, dev_status);
+    gb::launch(flood_results, 1, MAXD, 0, st, ctl, ndom, dev_steps, dev_simtime, dev_status);
     return gb::launched("flood_results");
 }
 

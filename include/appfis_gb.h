@@ -312,7 +312,7 @@ typedef struct {
     int flags;             /* APPFIS_GB_FLOOD_SKIP_DRY | APPFIS_GB_FLOOD_TWO_PHASE or _FUSED, or 0 */
 } appfis_gb_flood_params;
 
-/* flags: strips (28 or 30 x 32 cells) whose depth and momentum are exactly 0 and whose four neighbour
+/* flags: strips (28 or 30 columns x 2 to 32 rows) whose depth and momentum are exactly 0 and whose four neighbour
  * strips are dry as well are left out of a step: such cells cannot change (no face of theirs
  * has water on either side), so every field is bit-identical to the full sweep.  A strip is
  * skipped only after its output was dry for two consecutive steps (both state buffers hold the
