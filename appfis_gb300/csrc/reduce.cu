@@ -7,10 +7,16 @@
 // from numeric_limits<T>::min(), MIN from max(), SUM from 0 (kept here, including MAX's
 // smallest-positive seed for floating types).
 //
-// Here: one launch.  Each block walks whole rows of the box (coalesced along x), reduces in
-// registers + warp shuffles, writes one partial to a workspace array; the last block to finish
-// (ticket counter) folds the partials in block order.  Fixed grid size and fixed combine order
-// make the result deterministic; floating sums accumulate in double.  The input is never written.
+// Here: the box's elements are numbered along its rows and dealt to threads round robin, so a warp
+// reads 32 neighbours whatever the row length, eight loads in flight per thread; the position moves
+// by fixed steps and two carries, no division per element.  Each block leaves one partial and a
+// second launch folds them in block order (a box of up to 4096 elements is one block and one
+// launch): fixed grid, fixed order, deterministic, and nothing kept between calls.
+// This part has 2 FP64 lanes per SM and clock, so FP32 elements are compared as floats, and summed
+// as two or three floats (FloatSum) that reach a double once per 16 or 64 elements: FP32 SUM of 200 x 190 x 180
+// 38 us with a double add and conversion per element, 11.7 so (MAX 38 -> 9.8); 514^3 547 -> 129 us.
+// Bound there by the index arithmetic (a third of the instructions) and HBM (5.1 TB/s MAX); FP64 by
+// its pipe (272 us at 514^3).  The input is never written.
 #include <cfloat>
 #include <climits>
 #include <mutex>
@@ -19,9 +25,6 @@
 #include "gb_common.cuh"
 
 namespace {
-
-template <class T> struct Acc { typedef double type; };
-template <> struct Acc<int32_t> { typedef long long type; };
 
 template <class T> __device__ __forceinline__ T max_seed();
 template <> __device__ __forceinline__ float max_seed<float>() { return FLT_MIN; }
@@ -32,10 +35,18 @@ template <> __device__ __forceinline__ float min_seed<float>() { return FLT_MAX;
 template <> __device__ __forceinline__ double min_seed<double>() { return DBL_MAX; }
 template <> __device__ __forceinline__ int32_t min_seed<int32_t>() { return INT_MAX; }
 
+// The type a thread hands to its block: the element's own for MAX and MIN, double or int64 for SUM.
+template <class T, int OP> struct Acc { typedef T type; };
+template <> struct Acc<float, APPFIS_GB_SUM> { typedef double type; };
+template <> struct Acc<int32_t, APPFIS_GB_SUM> { typedef long long type; };
+// The type of a partial and of the result.
+template <class T> struct Wide { typedef double type; };
+template <> struct Wide<int32_t> { typedef long long type; };
+
 template <class T, int OP>
-__device__ __forceinline__ typename Acc<T>::type seed()
+__device__ __forceinline__ typename Acc<T, OP>::type seed()
 {
-    typedef typename Acc<T>::type A;
+    typedef typename Acc<T, OP>::type A;
     return OP == APPFIS_GB_MAX ? (A)max_seed<T>() : (OP == APPFIS_GB_MIN ? (A)min_seed<T>() : (A)0);
 }
 
@@ -60,79 +71,259 @@ __device__ __forceinline__ A block_reduce(A v, A neutral, A* sh)
     return v;
 }
 
-template <class T, int OP>
-__global__ void __launch_bounds__(256) reduce_box(const T* __restrict__ f, int px, int py, int x0, int x1, int y0, int y1,
-                                                  int z0, int z1, typename Acc<T>::type* __restrict__ partials,
-                                                  unsigned* __restrict__ ticket, void* __restrict__ result)
+// a + b == sum + err exactly, |err| at most half a unit in the last place of sum (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& err)
+{
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+
+// A thread's running sum of floats.  hi takes the element, mid what hi rounds off and (EXACT) lo what mid
+// rounds off.  EXACT: 64 elements reach the double within 2^-60 of their magnitude, so no more is
+// lost than by adding each to a double.  Otherwise 16 elements do within ~2^-47 of theirs, at half the
+// instructions: for boxes of 2^20 elements and more, where those errors, of either sign, come to
+// less than 2^-56 of the sum of magnitudes, under the rounding of the double tree that follows.
+// Infinities, NaN and sums beyond the float range leave a component that is not finite: the thread
+// then starts again in doubles.
+template <bool EXACT>
+struct FloatSum {
+    static constexpr int BATCH = EXACT ? 64 : 16;
+    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
+    double total = 0.0;
+    bool finite = true;
+    __device__ __forceinline__ void add(float v)
+    {
+        float e, r;
+        hi = two_sum(hi, v, e);
+        if (EXACT) {
+            mid = two_sum(mid, e, r);
+            lo = __fadd_rn(lo, r);
+        } else {
+            mid = __fadd_rn(mid, e);
+        }
+    }
+    __device__ __forceinline__ void flush()
+    {
+        finite = finite && fabsf(hi) <= FLT_MAX && fabsf(mid) <= FLT_MAX;
+        total += (double)hi + (EXACT ? (double)mid + (double)lo : (double)mid);
+        hi = mid = lo = 0.0f;
+    }
+};
+
+// The box: W x ny x nz elements from `first` (element offset of its corner), and what one stride of
+// all threads moves a position by.
+struct Box {
+    size_t first, n;          // elements
+    int W, ny;                // row length, rows per plane
+    int dcol, drow;           // the stride's columns, rows within a plane
+    long long step;           // and as an element offset
+    long long row_end, plane_end;  // offsets added when a row or a plane is passed
+};
+
+// A position in the box; Off: 32-bit offsets where the box spans less than 2^31 elements.
+template <class Off>
+struct Cursor {
+    Off at;
+    int col, row;
+    __device__ __forceinline__ void to(const Box& b, size_t e, int px, size_t plane)
+    {
+        const size_t r = e / (unsigned)b.W, k = r / (unsigned)b.ny;
+        col = (int)(e - r * b.W);
+        row = (int)(r - k * b.ny);
+        at = (Off)(k * plane + (size_t)row * px + col);
+    }
+    __device__ __forceinline__ void next(const Box& b)
+    {
+        at += (Off)b.step;
+        col += b.dcol;
+        row += b.drow;
+        if (col >= b.W) {
+            col -= b.W;
+            row += 1;
+            at += (Off)b.row_end;
+        }
+        if (row >= b.ny) {
+            row -= b.ny;
+            at += (Off)b.plane_end;
+        }
+    }
+};
+
+constexpr int RED_THREADS = 256;
+constexpr int RED_PER_SM = 4;        // blocks per SM (3 to 8, and 12 or 16 loads in flight, measured within 5%)
+constexpr int RED_ONE_BLOCK = 4096;  // elements up to which one block does it all
+
+template <class W>
+__device__ __forceinline__ void put_result(void* result, W w)
+{
+    *reinterpret_cast<W*>(result) = w;
+}
+
+// EXACT: see FloatSum (FP32 SUM only).
+template <class T, int OP, class Off, bool EXACT>
+__global__ void __launch_bounds__(RED_THREADS, RED_PER_SM) reduce_part(const T* __restrict__ field, Box b, int px, size_t plane,
+                                                          typename Wide<T>::type* __restrict__ partials, void* __restrict__ result)
 {
     const gb::BlockId bid = gb::grid_wait();
-    typedef typename Acc<T>::type A;
+    typedef typename Acc<T, OP>::type A;
+    typedef typename Wide<T>::type Wd;
+    constexpr int U = 8;  // loads in flight
     __shared__ A sh[32];
-    __shared__ bool last;
+    const size_t stride = (size_t)gridDim.x * RED_THREADS, e0 = (size_t)bid.x * RED_THREADS + threadIdx.x;
+    const T* __restrict__ f = field + b.first;
     A v = seed<T, OP>();
-    const int nyb = y1 - y0;
-    const long long rows = (long long)nyb * (z1 - z0);
-    for (long long r = bid.x; r < rows; r += gridDim.x) {
-        const int j = y0 + (int)(r % nyb), k = z0 + (int)(r / nyb);
-        const T* row = f + ((size_t)k * py + j) * (size_t)px;
-        for (int i = x0 + threadIdx.x; i < x1; i += blockDim.x) v = combine<OP>(v, (A)__ldg(row + i));
+    if (e0 < b.n) {
+        Cursor<Off> c;
+        c.to(b, e0, px, plane);
+        size_t left = (b.n - e0 + stride - 1) / stride;  // this thread's elements
+        if constexpr (std::is_same<T, float>::value && OP == APPFIS_GB_SUM) {
+            typedef FloatSum<EXACT> Sum;
+            Sum t;
+            int m = 0;
+            size_t q = left;
+            for (; q >= U; q -= U) {
+                float x[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    x[u] = __ldg(f + c.at);
+                    c.next(b);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) t.add(x[u]);
+                if ((m += U) == Sum::BATCH) {
+                    t.flush();
+                    m = 0;
+                }
+            }
+            for (; q > 0; q--) {
+                t.add(__ldg(f + c.at));
+                c.next(b);
+            }
+            t.flush();
+            v = t.total;
+            if (!t.finite) {
+                v = 0.0;
+                c.to(b, e0, px, plane);
+                for (; left > 0; left--) {
+                    v += (double)__ldg(f + c.at);
+                    c.next(b);
+                }
+            }
+        } else {
+            for (; left >= U; left -= U) {
+                T x[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    x[u] = __ldg(f + c.at);
+                    c.next(b);
+                }
+                A w[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) w[u] = (A)x[u];
+                if (OP == APPFIS_GB_SUM) {
+#pragma unroll
+                    for (int o = U / 2; o > 0; o /= 2)
+#pragma unroll
+                        for (int u = 0; u < o; u++) w[u] += w[u + o];
+                    v += w[0];
+                } else {
+#pragma unroll
+                    for (int u = 0; u < U; u++) v = combine<OP>(v, w[u]);
+                }
+            }
+            for (; left > 0; left--) {
+                v = combine<OP>(v, (A)__ldg(f + c.at));
+                c.next(b);
+            }
+        }
     }
     v = block_reduce<OP>(v, seed<T, OP>(), sh);
     if (threadIdx.x == 0) {
-        partials[bid.x] = v;
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    A w = seed<T, OP>();
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) w = combine<OP>(w, ((volatile A*)partials)[b]);
-    __syncthreads();
-    w = block_reduce<OP>(w, seed<T, OP>(), sh);
-    if (threadIdx.x == 0) {
-        if (std::is_floating_point<A>::value) *reinterpret_cast<double*>(result) = (double)w;
-        else *reinterpret_cast<long long*>(result) = (long long)w;
-        *ticket = 0;  // ready for the next call
+        if (result) put_result(result, (Wd)v);
+        else partials[bid.x] = (Wd)v;
     }
 }
 
-constexpr int RED_THREADS = 256;
+template <class T, int OP>
+__global__ void __launch_bounds__(RED_THREADS) reduce_fold(const typename Wide<T>::type* __restrict__ partials, int n, void* __restrict__ result)
+{
+    gb::grid_wait();
+    typedef typename Wide<T>::type Wd;
+    __shared__ Wd sh[32];
+    const volatile Wd* part = partials;  // written by the launch before: read behind the wait
+    const Wd neutral = (Wd)seed<T, OP>();
+    Wd v = neutral;
+    for (int k = threadIdx.x; k < n; k += RED_THREADS) v = combine<OP>(v, (Wd)part[k]);
+    v = block_reduce<OP>(v, neutral, sh);
+    if (threadIdx.x == 0) put_result(result, v);
+}
+
+int reduce_blocks(long long n)
+{
+    if (n <= RED_ONE_BLOCK) return 1;
+    return (int)std::min<long long>((n + RED_THREADS * 16 - 1) / (RED_THREADS * 16), (long long)RED_PER_SM * gb::sm_count());
+}
+
+// partials: one value per block, for grids of more than one
+template <class T, int OP>
+int launch_op(const T* f, int px, int py, const int* x, int grid, void* partials, void* res, cudaStream_t st)
+{
+    Box b;
+    const size_t plane = (size_t)px * py;
+    b.W = x[1] - x[0];
+    b.ny = x[3] - x[2];
+    b.first = x[4] * plane + (size_t)x[2] * px + x[0];
+    b.n = (size_t)b.W * b.ny * (x[5] - x[4]);
+    const size_t stride = (size_t)grid * RED_THREADS, srow = stride / b.W;
+    b.dcol = (int)(stride % b.W);
+    b.drow = (int)(srow % b.ny);
+    b.step = (long long)(srow / b.ny * plane) + (long long)b.drow * px + b.dcol;
+    b.row_end = px - b.W;
+    b.plane_end = (long long)plane - (long long)b.ny * px;
+    typedef typename Wide<T>::type Wd;
+    Wd* part = reinterpret_cast<Wd*>(partials);
+    // the last offset a cursor can reach: one stride past the box
+    const bool small = (double)plane * (x[5] - x[4] + 2) + (double)b.step < 2147483647.0;
+    constexpr bool fsum = std::is_same<T, float>::value && OP == APPFIS_GB_SUM;
+    const bool exact = fsum && b.n < ((size_t)1 << 20);
+    auto kern = exact ? reduce_part<T, OP, int, fsum> : (small ? reduce_part<T, OP, int, false> : reduce_part<T, OP, long long, false>);
+    if (exact && !small) kern = reduce_part<T, OP, long long, fsum>;
+    gb::launch(kern, grid, RED_THREADS, 0, st, f, b, px, plane, part, grid == 1 ? res : nullptr);
+    if (grid > 1) gb::launch(reduce_fold<T, OP>, 1, RED_THREADS, 0, st, part, grid, res);
+    return gb::launched("reduce");
+}
 
 template <class T>
-int launch_reduce(const void* field, int px, int py, const int* b, int op, void* res, cudaStream_t st)
+int launch_reduce(const void* field, int px, int py, const int* b, int op, int grid, void* partials, void* res, cudaStream_t st)
 {
-    typedef typename Acc<T>::type A;
-    const long long rows = (long long)(b[3] - b[2]) * (b[5] - b[4]);
-    const int grid = (int)std::max<long long>(1, std::min<long long>(rows, (long long)gb::sm_count() * 4));
-    void* ws;
-    GB_TRY(gb::workspace(gb::WS_REDUCE, 256 + sizeof(A) * (size_t)grid, &ws));
-    unsigned* ticket = reinterpret_cast<unsigned*>(ws);
-    A* partials = reinterpret_cast<A*>(reinterpret_cast<char*>(ws) + 256);
-    GB_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
     const T* f = reinterpret_cast<const T*>(field);
     switch (op) {
-    case APPFIS_GB_MAX:
-        gb::launch(reduce_box<T, APPFIS_GB_MAX>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
-        break;
-    case APPFIS_GB_MIN:
-        gb::launch(reduce_box<T, APPFIS_GB_MIN>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
-        break;
-    default:
-        gb::launch(reduce_box<T, APPFIS_GB_SUM>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
+    case APPFIS_GB_MAX: return launch_op<T, APPFIS_GB_MAX>(f, px, py, b, grid, partials, res, st);
+    case APPFIS_GB_MIN: return launch_op<T, APPFIS_GB_MIN>(f, px, py, b, grid, partials, res, st);
+    default: return launch_op<T, APPFIS_GB_SUM>(f, px, py, b, grid, partials, res, st);
     }
-    return gb::launched("reduce_box");
 }
+
+int launch_reduce(int dtype, const void* field, int px, int py, const int* b, int op, int grid, void* partials, void* res, cudaStream_t st)
+{
+    switch (dtype) {
+    case APPFIS_GB_F32: return launch_reduce<float>(field, px, py, b, op, grid, partials, res, st);
+    case APPFIS_GB_F64: return launch_reduce<double>(field, px, py, b, op, grid, partials, res, st);
+    default: return launch_reduce<int32_t>(field, px, py, b, op, grid, partials, res, st);
+    }
+}
+
+long long box_elements(const int* b) { return (long long)(b[1] - b[0]) * (b[3] - b[2]) * (b[5] - b[4]); }
 
 // ---------------------------------------------------------------- allocation-free variant
 // Some callers cannot allocate device memory at the moment they need a reduction: a host
 // framework whose caching allocator has reserved the device memory, a library embedded in a
 // runtime that owns every allocation, or a latency-critical loop that cannot take the implicit
 // synchronisation of a first cudaMalloc/cudaFree.  For them the same reduction kernel can take
-// its scratch (one ticket counter and one partial per block) from a fixed array that is part of
-// the library image instead of the grow-only workspace.  64 KiB holds the ticket and 8160
-// partials; the kernel uses at most 4 blocks per SM (608 on a GB300), so every box fits on
-// current GPUs.  Every device that loads the library keeps this array until the process exits
+// its scratch (one partial per block) from a fixed array that is part of the library image instead of
+// the grow-only workspace.  Of its 64 KiB 8160 partials are used; the kernel has at most 4 blocks per
+// SM (608 on a GB300), so every box fits on current GPUs.  Every device that loads the library keeps this array until the process exits
 // (under lazy module loading the runtime commits it on the first use of the module on a device).
 constexpr size_t NOALLOC_SCRATCH_BYTES = 64 * 1024;
 constexpr size_t NOALLOC_MAX_PARTIALS = (NOALLOC_SCRATCH_BYTES - 256) / sizeof(double);
@@ -161,34 +352,6 @@ int noalloc_scratch(void** out)
     return APPFIS_GB_OK;
 }
 
-template <class T>
-int launch_reduce_noalloc(const void* field, int px, int py, const int* b, int op, void* res, cudaStream_t st)
-{
-    typedef typename Acc<T>::type A;
-    const long long rows = (long long)(b[3] - b[2]) * (b[5] - b[4]);
-    const int grid = (int)std::max<long long>(1, std::min<long long>(rows, (long long)gb::sm_count() * 4));
-    if ((size_t)grid > NOALLOC_MAX_PARTIALS)
-        return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: %d partial sums needed, the fixed scratch holds %zu", grid,
-                        NOALLOC_MAX_PARTIALS);
-    void* ws = nullptr;
-    GB_TRY(noalloc_scratch(&ws));
-    unsigned* ticket = reinterpret_cast<unsigned*>(ws);
-    A* partials = reinterpret_cast<A*>(reinterpret_cast<char*>(ws) + 256);
-    GB_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));  // the array keeps the last call's contents
-    const T* f = reinterpret_cast<const T*>(field);
-    switch (op) {
-    case APPFIS_GB_MAX:
-        gb::launch(reduce_box<T, APPFIS_GB_MAX>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
-        break;
-    case APPFIS_GB_MIN:
-        gb::launch(reduce_box<T, APPFIS_GB_MIN>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
-        break;
-    default:
-        gb::launch(reduce_box<T, APPFIS_GB_SUM>, grid, RED_THREADS, 0, st, f, px, py, b[0], b[1], b[2], b[3], b[4], b[5], partials, ticket, res);
-    }
-    return gb::launched("reduce_box (fixed scratch)");
-}
-
 }  // namespace
 
 extern "C" {
@@ -202,13 +365,15 @@ int appfis_gb_reduce_noalloc(const void* field, int dtype, int px, int py, const
         if (box[2 * a] < 0 || box[2 * a + 1] < box[2 * a]) return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: bad box axis %d", a);
     if (box[1] > px || box[3] > py || px < 1 || py < 1) return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: box outside the field");
     if (box[0] == box[1] || box[2] == box[3] || box[4] == box[5]) return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: empty box");
-    cudaStream_t st = gb::as_stream(stream);
-    switch (dtype) {
-    case APPFIS_GB_F32: return launch_reduce_noalloc<float>(field, px, py, box, op, dev_result, st);
-    case APPFIS_GB_F64: return launch_reduce_noalloc<double>(field, px, py, box, op, dev_result, st);
-    case APPFIS_GB_I32: return launch_reduce_noalloc<int32_t>(field, px, py, box, op, dev_result, st);
-    default: return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: unknown dtype %d", dtype);
-    }
+    if (dtype != APPFIS_GB_F32 && dtype != APPFIS_GB_F64 && dtype != APPFIS_GB_I32)
+        return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: unknown dtype %d", dtype);
+    const int grid = reduce_blocks(box_elements(box));
+    if ((size_t)grid > NOALLOC_MAX_PARTIALS)
+        return gb::fail(APPFIS_GB_EINVAL, "reduce_noalloc: %d partial sums needed, the fixed scratch holds %zu", grid,
+                        NOALLOC_MAX_PARTIALS);
+    void* part = nullptr;
+    GB_TRY(noalloc_scratch(&part));
+    return launch_reduce(dtype, field, px, py, box, op, grid, part, dev_result, gb::as_stream(stream));
 }
 
 int appfis_gb_reduce(const void* field, int dtype, int px, int py, const int* box, int op, void* dev_result, void* stream)
@@ -220,13 +385,12 @@ int appfis_gb_reduce(const void* field, int dtype, int px, int py, const int* bo
     if (box[1] > px || box[3] > py || px < 1 || py < 1) return gb::fail(APPFIS_GB_EINVAL, "reduce: box outside the field");
     if (box[0] == box[1] || box[2] == box[3] || box[4] == box[5])
         return gb::fail(APPFIS_GB_EINVAL, "reduce: empty box");
-    cudaStream_t st = gb::as_stream(stream);
-    switch (dtype) {
-    case APPFIS_GB_F32: return launch_reduce<float>(field, px, py, box, op, dev_result, st);
-    case APPFIS_GB_F64: return launch_reduce<double>(field, px, py, box, op, dev_result, st);
-    case APPFIS_GB_I32: return launch_reduce<int32_t>(field, px, py, box, op, dev_result, st);
-    default: return gb::fail(APPFIS_GB_EINVAL, "reduce: unknown dtype %d", dtype);
-    }
+    if (dtype != APPFIS_GB_F32 && dtype != APPFIS_GB_F64 && dtype != APPFIS_GB_I32)
+        return gb::fail(APPFIS_GB_EINVAL, "reduce: unknown dtype %d", dtype);
+    const int grid = reduce_blocks(box_elements(box));
+    void* part;
+    GB_TRY(gb::workspace(gb::WS_REDUCE, sizeof(double) * (size_t)grid, &part));
+    return launch_reduce(dtype, field, px, py, box, op, grid, part, dev_result, gb::as_stream(stream));
 }
 
 int appfis_gb_reduce_host(const void* field, int dtype, int px, int py, const int* box, int op, double* result, void* stream)

@@ -90,8 +90,8 @@ APPFIS_GB_API int appfis_gb_test_stall_next(int kind, unsigned long long limit);
  * The result is written to the 8-byte device location dev_result: a double for F32/F64, an
  * int64 for I32.  MAX is seeded with std::numeric_limits<T>::min() like the reference (for
  * floating types that is the smallest positive normal, so an all-negative box returns it),
- * MIN with max(), SUM with 0.  Floating SUMs accumulate in double; every result is deterministic
- * (fixed-order tree: per-block partials, then the last block folds them in block order). */
+ * MIN with max(), SUM with 0.  Floating SUMs accumulate in double or to the same accuracy; every
+ * result is deterministic (fixed-order tree: per-block partials, folded in block order). */
 APPFIS_GB_API int appfis_gb_reduce(const void* field, int dtype, int px, int py, const int* box, int op, void* dev_result,
                      void* stream);
 /* Same reduction, same result, for callers that must not allocate device memory: a host
@@ -100,7 +100,7 @@ APPFIS_GB_API int appfis_gb_reduce(const void* field, int dtype, int px, int py,
  * every allocation, or a latency-critical loop where the implicit device synchronisation of a
  * first cudaMalloc/cudaFree would stall the pipeline.  No counterpart in the reference (its
  * reductions allocate nothing beyond the grid's own buffers).
- * The scratch (a ticket and one partial sum per block) lives in a fixed 64 KiB device array
+ * The scratch (one partial sum per block) lives in a fixed 64 KiB device array
  * inside the library, held by every device that loads it until the process exits; a box whose
  * reduction needs more than 8160 partial sums is rejected with APPFIS_GB_EINVAL (this kernel
  * uses at most 4 per SM).  The entry point calls no cudaMalloc, cudaFree or allocating library
@@ -109,9 +109,8 @@ APPFIS_GB_API int appfis_gb_reduce(const void* field, int dtype, int px, int py,
  * capture.  Under CUDA's default lazy module loading the runtime commits the array's 64 KiB and
  * loads each (dtype, op) kernel instance on first use, so warm up every dtype/op pair you will
  * use before the device memory is handed to another allocator (or set CUDA_MODULE_LOADING=EAGER,
- * which loads everything when the library's module is first used).  Every call clears the
- * ticket with an asynchronous memset on `stream`.  All calls share the array, so calls that
- * overlap on the GPU (other streams, other host threads) race: order them. */
+ * which loads everything when the library's module is first used).  All calls share the array,
+ * so calls that overlap on the GPU (other streams, other host threads) race: order them. */
 APPFIS_GB_API int appfis_gb_reduce_noalloc(const void* field, int dtype, int px, int py, const int* box, int op,
                                            void* dev_result, void* stream);
 /* Same, returning the value on the host (synchronises `stream`). */
