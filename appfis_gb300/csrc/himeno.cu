@@ -5,9 +5,9 @@
 // on a DUAL p grid and 12 SINGLE coefficient grids (:74-86, :108-114).  The reference computes
 // no gosa; ss is exactly its :195 expression.
 //
-// Plain form: one launch per sweep, a 2.5-D z-march with the p planes in a shared ring and the
-// 12 coefficient streams read once: himeno_tma (tiles moved by the tensor memory accelerator)
-// when rows and fields are 16-byte aligned, else himeno_ring<0> (register-prefetched loads).
+// Plain form: one launch per sweep.  himeno_tma: a 2.5-D z-march with the p planes in a shared ring
+// and the 12 coefficient streams read once, tiles moved by the tensor memory accelerator, for large
+// grids whose rows and fields are 16-byte aligned; else himeno_flat.
 // The sum uses round-to-nearest intrinsics in the reference's order (no FMA contraction), so p
 // is bit-identical to the reference CPU path.
 //
@@ -21,7 +21,7 @@
 // correction pass folds e into P, recomputes D from the FP32 coefficients and restarts e at 0,
 // which bounds the FP16 error to the last period's correction.  The sweep's own ss is
 // (e' - e)/w (FP32, before rounding e').  Inner sweeps: himeno_mixed2 (TMA-staged, two points
-// per thread) when the FP16 rows are 16-byte aligned, else himeno_ring<1>.
+// per thread) when the FP16 rows are 16-byte aligned, else (and on small grids without gosa) himeno_flat.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -125,6 +125,37 @@ struct SqAcc {
     __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
+// The end of a flat sweep's block: as gosa_end, for kernels whose threads have only a few points each.
+// The warps add their threads' two-float sums as such (relative error under 2^-45 for these
+// positive terms) and one warp takes the warps' sums to double: a double shuffle tree per warp costs
+// 8 FP64 instructions of 16 cycles each on this part, more than the sweep itself at few planes per
+// thread (65 x 65 x 129: see himeno_flat).
+__device__ __forceinline__ void gosa_end_flat(const SqAcc& acc, const GosaIO& g, unsigned block)
+{
+    if (g.part) {
+        __shared__ float2 sh[32];
+        float hi = acc.hi, lo = acc.lo;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float h2 = __shfl_down_sync(0xffffffffu, hi, o), l2 = __shfl_down_sync(0xffffffffu, lo, o);
+            const float s = __fadd_rn(hi, h2), bb = __fsub_rn(s, hi);
+            const float e = __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(h2, bb)), __fadd_rn(lo, l2));
+            hi = __fadd_rn(s, e);
+            lo = __fsub_rn(e, __fsub_rn(hi, s));
+        }
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_float2(hi, lo);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const float2 w = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : make_float2(0.0f, 0.0f);
+            double v = (double)w.x + (double)w.y;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);  // at most 8 warps
+            if (threadIdx.x == 0) g.part[block] = v;
+        }
+    }
+    if (g.prev && block == 0) gosa_fold(g);
+}
+
 // 19-point s0 in the reference's order, on any readable field F (F(di,dj,dk) -> float)
 #define HIMENO_S0(F, A0, A1, A2, B0, B1, B2, C0, C1, C2, W1)                                               \
     fadd(fadd(fadd(fadd(fadd(fadd(fadd(fadd(fadd(fmul(A0, F(1, 0, 0)), fmul(A1, F(0, 1, 0))), fmul(A2, F(0, 0, 1))), \
@@ -188,159 +219,153 @@ __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float*
     gosa_end<1>({(double)g}, gz);
 }
 
-// ---------------------------------------------------------------- 2.5-D forms with a shared plane ring
-// A CTA of RX x RY threads owns an (x, y) tile and marches a chunk of z.  p (or e) planes k-1,
-// k, k+1 live in a 4-slot shared ring with a one-cell x/y halo: plane k+2 is loaded into
-// registers one iteration ahead and written to its slot after the sweep of plane k, so one
-// barrier per plane suffices and every p value comes from memory once per CTA.  The point's
-// coefficients for plane k+1 are loaded while plane k is computed.  All neighbour reads are
-// shared-memory reads, so the only global traffic is the compulsory streams.
-constexpr int RX = 32, RY = 8;
-constexpr int RW = RX + 2, RH = RY + 2, RSLOT = RW * RH;
-constexpr int RHALO = RSLOT - RX * RY;  // 84 halo cells per plane
-
-// (row, col) in the slot of halo item h (0 <= h < RHALO): top row, bottom row, left col, right col
-__device__ __forceinline__ int halo_slot(int h)
-{
-    if (h < RW) return h;                                     // row 0
-    h -= RW;
-    if (h < RW) return (RH - 1) * RW + h;                     // row RH-1
-    h -= RW;
-    if (h < RY) return (h + 1) * RW;                          // col 0, rows 1..RY
-    h -= RY;
-    return (h + 1) * RW + RW - 1;                             // col RW-1
-}
+// ---------------------------------------------------------------- flat form
+// One column of FK planes per thread, the columns of a plane numbered along its rows (ghost columns
+// and padding included, so a warp reads consecutive addresses whatever the row length); neighbours
+// come through L1.  Going up a column, the five values of plane k+1 that plane k needs serve again as
+// plane k+1's own, so a point costs 9 loads of the field and 12 of the coefficients.
+//
+// It is the form for rows that are not 16-byte aligned, and for grids too small to give every SM the
+// long z-march of the TMA-staged forms.  Us per sweep against a 2.5-D march with a shared-memory plane
+// ring (which this replaced) and the TMA-staged sweep, FP32 with gosa: 65 x 65 x 129 dense 22.9 -> 6.2,
+// rows padded to 72 15.5 (TMA) -> 6.4; 129 x 129 x 257 dense 72 -> 40, rows of 136 44.7 (TMA) -> 41.9;
+// 160 x 160 x 300 77 (TMA) / 76; 200 x 210 x 400 155 (TMA) / 172; 257 x 257 x 513 dense 406 -> 329, rows of 264
+// 293 (TMA) / 336.  FP16 correction sweep: 65 x 65 x 129 dense 39 -> 6.1, 257 x 257 x 513 dense 461 -> 267.
+// Bounded by L1 and latency (0.85 of the copy rate at 257 x 257 x 513).  Columns of 1 / 2 / 4 / 8 planes
+// at 65 x 65 x 129: 7.9 / 6.6 / 6.0 / 7.2; 257 x 257 x 513: 414 / 347 / 337 / 329; 33 x 33 x 65: 4.1 / 4.2 / 4.8 / 6.3;
+// blocks of 128 threads 5-20% slower.
+constexpr int FT = 256;  // threads per block
+constexpr int RX = 32, RY = 8;  // the tile of the TMA-staged one-point forms
 
 template <class L>
-__device__ __forceinline__ float ring_load(const L* f, size_t idx, bool ok);
-template <> __device__ __forceinline__ float ring_load<float>(const float* f, size_t idx, bool ok) { return ok ? __ldg(f + idx) : 0.0f; }
-template <> __device__ __forceinline__ float ring_load<__half>(const __half* f, size_t idx, bool ok)
-{
-    return ok ? __half2float(__ldg(f + idx)) : 0.0f;
-}
+__device__ __forceinline__ float load_float(const L* f, size_t idx);
+template <> __device__ __forceinline__ float load_float<float>(const float* f, size_t idx) { return __ldg(f + idx); }
+template <> __device__ __forceinline__ float load_float<__half>(const __half* f, size_t idx) { return __half2float(__ldg(f + idx)); }
 
-// Loads plane k of field f for this thread: its centre value and (threads < RHALO) one halo value.
-template <class L>
-__device__ __forceinline__ void ring_fetch(const L* f, int k, int i, int j, int hi, int hj, int nx, int ny, int px,
-                                           size_t plane, int t, float& c, float& h)
-{
-    const size_t base = (size_t)k * plane;
-    c = ring_load<L>(f, base + (size_t)j * px + i, i <= nx + 1 && j <= ny + 1);
-    h = t < RHALO ? ring_load<L>(f, base + (size_t)hj * px + hi, hi <= nx + 1 && hj <= ny + 1) : 0.0f;
-}
-
-__device__ __forceinline__ void ring_store(float* slot, int t, int tx, int ty, int hs, float c, float h)
-{
-    slot[(ty + 1) * RW + tx + 1] = c;
-    if (t < RHALO) slot[hs] = h;
-}
-
-template <int MODE>  // 0: plain FP32 sweep of p; 1: FP16 correction sweep of e
-__global__ void __launch_bounds__(RX* RY) himeno_ring(Coef12 cf, H10 hf, const void* __restrict__ pin, void* __restrict__ pout,
-                                                       const __half* __restrict__ D, int nx, int ny, int nz, int px, int py,
-                                                       int kz, float omega, float inv_omega, GosaIO gz)
+// MODE 0: plain FP32 sweep of p; 1: FP16 correction sweep of e, in himeno_mixed2's operation order; 2: the
+// same sweep with the rounding of the sums left to the compiler, as on rows that are not 16-byte aligned.
+template <int MODE, int FK>
+__global__ void __launch_bounds__(FT, 4) himeno_flat(Coef12 cf, H10 hf, const void* __restrict__ pin, void* __restrict__ pout,
+                                                  const __half* __restrict__ D, int nx, int ny, int nz, int px, unsigned plane_blocks,
+                                                  float omega, float inv_omega, GosaIO gz)
 {
     const gb::BlockId bid = gb::grid_wait();
-    __shared__ float ring[4][RSLOT];
-    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * RX + tx;
-    const int i = 1 + bid.x * RX + tx, j = 1 + bid.y * RY + ty;
-    const int k0 = 1 + bid.z * kz, k1 = min(k0 + kz, nz + 1);
-    const size_t plane = (size_t)px * py;
-    const bool act = i <= nx && j <= ny;
-    // this thread's halo cell (fixed for all planes)
-    int hs = 0, hi = 0, hj = 0;
-    if (t < RHALO) {
-        hs = halo_slot(t);
-        hi = bid.x * RX + hs % RW;  // padded coords: slot (0,0) is (i0-1, j0-1)
-        hj = bid.y * RY + hs / RW;
-    }
     typedef typename std::conditional<MODE == 0, float, __half>::type L;
-    const L* f = reinterpret_cast<const L*>(pin);
-    float c, h;
-    // planes k0-1, k0, k0+1 into slots, k0+2 in registers
-#pragma unroll
-    for (int d = -1; d <= 1; d++) {
-        ring_fetch<L>(f, k0 + d, i, j, hi, hj, nx, ny, px, plane, t, c, h);
-        ring_store(ring[(k0 + d) & 3], t, tx, ty, hs, c, h);
+    const L* __restrict__ f = reinterpret_cast<const L*>(pin);
+    const unsigned zc = bid.x / plane_blocks, pb = bid.x - zc * plane_blocks;
+    unsigned row, col;
+    if (plane_blocks < 1u << 24) {  // uniform: a plane of fewer than 2^32 elements
+        const unsigned q = pb * FT + threadIdx.x;
+        row = q / (unsigned)px;
+        col = q - row * (unsigned)px;
+    } else {
+        const size_t q = (size_t)pb * FT + threadIdx.x;
+        row = (unsigned)(q / (unsigned)px);
+        col = (unsigned)(q - (size_t)row * px);
     }
-    float nc = 0.0f, nh = 0.0f;
-    if (k0 + 2 <= nz + 1) ring_fetch<L>(f, k0 + 2, i, j, hi, hj, nx, ny, px, plane, t, nc, nh);
-    // coefficients of plane k0
-    const size_t c0 = ((size_t)k0 * py + j) * px + i;
-    float co[12];
-    if (act) {
-        if (MODE == 0) {
-#pragma unroll
-            for (int n = 0; n < 12; n++) co[n] = __ldcs(cf.c[n] + c0);
-        } else {
-#pragma unroll
-            for (int n = 0; n < 10; n++) co[n] = __half2float(__ldcs(hf.c[n] + c0));
-            co[10] = __ldcs(hf.a3 + c0);
-            co[11] = __half2float(__ldcs(D + c0));
-        }
-    }
-    __syncthreads();
+    const int i = (int)col, j = 1 + (int)row, k0 = 1 + (int)zc * FK;
+    const size_t plane = (size_t)px * (ny + 2);
     SqAcc g;
-    for (int k = k0; k < k1; k++) {
-        const size_t cc = ((size_t)k * py + j) * px + i;
-        // prefetch the next plane's coefficients
-        float cn[12];
-        const bool more = k + 1 < k1;
-        if (act && more) {
-            const size_t c1 = cc + plane;
-            if (MODE == 0) {
+    if (i >= 1 && i <= nx && j <= ny) {
+        size_t c = (size_t)k0 * plane + (size_t)j * px + i;
+        auto ld = [&](size_t at) { return load_float<L>(f, at); };
+        float m[3][3], z[3][3], p[3][3];  // planes k-1, k, k+1; [1 + dy][1 + dx]
+        auto cross = [&](float (&v)[3][3], size_t at) {
+            v[1][1] = ld(at);
+            v[1][0] = ld(at - 1);
+            v[1][2] = ld(at + 1);
+            v[0][1] = ld(at - px);
+            v[2][1] = ld(at + px);
+        };
+        cross(m, c - plane);
+        cross(z, c);
 #pragma unroll
-                for (int n = 0; n < 12; n++) cn[n] = __ldcs(cf.c[n] + c1);
-            } else {
+        for (int u = 0; u < FK; u++) {
+            if (k0 + u <= nz) {
+                float co[12];
+                if (MODE == 0) {
 #pragma unroll
-                for (int n = 0; n < 10; n++) cn[n] = __half2float(__ldcs(hf.c[n] + c1));
-                cn[10] = __ldcs(hf.a3 + c1);
-                cn[11] = __half2float(__ldcs(D + c1));
+                    for (int n = 0; n < 12; n++) co[n] = __ldcs(cf.c[n] + c);
+                } else {
+#pragma unroll
+                    for (int n = 0; n < 10; n++) co[n] = __half2float(__ldcs(hf.c[n] + c));
+                    co[10] = __ldcs(hf.a3 + c);
+                    co[11] = __half2float(__ldcs(D + c));
+                }
+                cross(p, c + plane);
+                z[0][0] = ld(c - px - 1);
+                z[0][2] = ld(c - px + 1);
+                z[2][0] = ld(c + px - 1);
+                z[2][2] = ld(c + px + 1);
+                auto RF = [&](int di, int dj, int dk) { return dk < 0 ? m[1 + dj][1 + di] : (dk > 0 ? p[1 + dj][1 + di] : z[1 + dj][1 + di]); };
+                if (MODE == 0) {
+                    const float s0v = HIMENO_S0(RF, co[0], co[1], co[2], co[4], co[5], co[6], co[7], co[8], co[9], co[11]);
+                    const float pc = RF(0, 0, 0);
+                    const float ss = fmul(fsub(fmul(s0v, co[3]), pc), co[10]);
+                    reinterpret_cast<float*>(pout)[c] = fadd(pc, fmul(omega, ss));
+                    g.add_sq(ss);
+                } else {
+                    const float e0 = RF(0, 0, 0);
+                    const float txy = (RF(1, 1, 0) - RF(1, -1, 0)) - (RF(-1, 1, 0) - RF(-1, -1, 0));
+                    const float tyz = (RF(0, 1, 1) - RF(0, -1, 1)) - (RF(0, 1, -1) - RF(0, -1, -1));
+                    const float txz = (RF(1, 0, 1) - RF(-1, 0, 1)) - (RF(1, 0, -1) - RF(-1, 0, -1));
+                    float v;
+                    if (MODE == 1) {
+                        float ne = fmul(co[0], RF(1, 0, 0));
+                        ne = __fmaf_rn(co[1], RF(0, 1, 0), ne);
+                        ne = __fmaf_rn(co[2], RF(0, 0, 1), ne);
+                        ne = __fmaf_rn(co[3], txy, ne);
+                        ne = __fmaf_rn(co[4], tyz, ne);
+                        ne = __fmaf_rn(co[5], txz, ne);
+                        ne = __fmaf_rn(co[6], RF(-1, 0, 0), ne);
+                        ne = __fmaf_rn(co[7], RF(0, -1, 0), ne);
+                        ne = __fmaf_rn(co[8], RF(0, 0, -1), ne);
+                        v = fadd(__fmaf_rn(fmul(omega, co[9]), __fmaf_rn(co[10], ne, -e0), e0), co[11]);
+                    } else {
+                        float ne = co[0] * RF(1, 0, 0) + co[1] * RF(0, 1, 0) + co[2] * RF(0, 0, 1);
+                        ne += co[3] * txy;
+                        ne += co[4] * tyz;
+                        ne += co[5] * txz;
+                        ne += co[6] * RF(-1, 0, 0) + co[7] * RF(0, -1, 0) + co[8] * RF(0, 0, -1);
+                        v = e0 + omega * co[9] * (co[10] * ne - e0) + co[11];
+                    }
+                    reinterpret_cast<__half*>(pout)[c] = __float2half_rn(v);
+                    g.add_sq((v - e0) * inv_omega);
+                }
+#pragma unroll
+                for (int a = 0; a < 3; a++)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        m[a][d] = z[a][d];
+                        z[a][d] = p[a][d];
+                    }
+                c += plane;
             }
         }
-        if (act) {
-            const float* sm = ring[(k - 1) & 3];
-            const float* s0 = ring[k & 3];
-            const float* sp = ring[(k + 1) & 3];
-            const int q = (ty + 1) * RW + tx + 1;
-#define RF(di, dj, dk) (((dk) < 0 ? sm : ((dk) > 0 ? sp : s0))[q + (di) + (dj) * RW])
-            if (MODE == 0) {
-                const float s0v = HIMENO_S0(RF, co[0], co[1], co[2], co[4], co[5], co[6], co[7], co[8], co[9], co[11]);
-                const float pc = RF(0, 0, 0);
-                const float ss = fmul(fsub(fmul(s0v, co[3]), pc), co[10]);
-                reinterpret_cast<float*>(pout)[cc] = fadd(pc, fmul(omega, ss));
-                g.add_sq(ss);
-            } else {
-                // neighbour sum N e (no wrk1), then e' = e + w*bnd*(a3*N e - e) + D
-                float ne = co[0] * RF(1, 0, 0) + co[1] * RF(0, 1, 0) + co[2] * RF(0, 0, 1);
-                ne += co[3] * ((RF(1, 1, 0) - RF(1, -1, 0)) - (RF(-1, 1, 0) - RF(-1, -1, 0)));
-                ne += co[4] * ((RF(0, 1, 1) - RF(0, -1, 1)) - (RF(0, 1, -1) - RF(0, -1, -1)));
-                ne += co[5] * ((RF(1, 0, 1) - RF(-1, 0, 1)) - (RF(1, 0, -1) - RF(-1, 0, -1)));
-                ne += co[6] * RF(-1, 0, 0) + co[7] * RF(0, -1, 0) + co[8] * RF(0, 0, -1);
-                const float e0 = RF(0, 0, 0);
-                const float v = e0 + omega * co[9] * (co[10] * ne - e0) + co[11];
-                reinterpret_cast<__half*>(pout)[cc] = __float2half_rn(v);
-                const float ss = (v - e0) * inv_omega;
-                g.add_sq(ss);
-            }
-#undef RF
-        }
-        if (more) {
-            // plane k+2 (fetched last iteration) into its slot; its last readers (plane k-1's sweep)
-            // passed the previous barrier
-            ring_store(ring[(k + 2) & 3], t, tx, ty, hs, nc, nh);
-            if (k + 3 <= nz + 1) ring_fetch<L>(f, k + 3, i, j, hi, hj, nx, ny, px, plane, t, nc, nh);
-#pragma unroll
-            for (int n = 0; n < 12; n++) co[n] = cn[n];
-        }
-        __syncthreads();
     }
-    gosa_end<1>({g.value()}, gz);
+    gosa_end_flat(g, gz, bid.x);
 }
 
+// The kernel and grid of a flat sweep: the taller the columns the fewer loads, as long as every SM has
+// blocks.
+template <int MODE>
+struct FlatPlan {
+    decltype(&himeno_flat<MODE, 4>) kernel;
+    unsigned plane_blocks, blocks;
+    FlatPlan(int ny, int nz, int pitch)
+    {
+        plane_blocks = gb::ceil_div((size_t)ny * pitch, FT);
+        auto grid = [&](int fk) { return (size_t)plane_blocks * ((nz + fk - 1) / fk); };
+        const size_t sms = gb::sm_count();
+        const int fk = grid(8) >= 10 * sms ? 8 : (grid(4) >= 2 * sms ? 4 : 2);
+        kernel = fk == 8 ? himeno_flat<MODE, 8> : (fk == 4 ? himeno_flat<MODE, 4> : himeno_flat<MODE, 2>);
+        blocks = (unsigned)grid(fk);
+    }
+};
+
 // ---------------------------------------------------------------- TMA-staged FP32 sweep
-// Same tile, z-march and arithmetic as himeno_ring<0>, but every stream is moved by the tensor
-// memory accelerator: for plane k, one pipeline stage holds the twelve coefficient tiles of
+// A CTA of RX x RY threads owns an (x, y) tile and marches a chunk of z; every stream is moved by the
+// tensor memory accelerator: for plane k, one pipeline stage holds the twelve coefficient tiles of
 // plane k (32 x 8 each) and p's plane k+1 (40 x 10, the halo included, its x origin rounded down
 // to a 16-byte boundary).  Thread 0 keeps S stages in flight; the other threads only read
 // shared memory.  The CTA's x tile starts on a 32-point boundary of the padded row (thread tx
@@ -953,6 +978,8 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
 // HKZ: z planes per CTA (nz is split into equal chunks of at most HKZ planes)
 constexpr int HBX = 32, HBY = 4, HKZ = 32;
 constexpr int TMA_S_PLAIN = 3;
+constexpr size_t FLAT_POINTS = 6000000;        // grids up to this take the flat FP32 sweep
+constexpr size_t FLAT_MIXED_POINTS = 3000000;  // ... and the flat FP16 sweep where no gosa is asked for
 
 // Tensor maps of the plain form: the 12 FP32 coefficient fields and the iterated p buffer.
 int plain_maps(const float* const* coef, const float* pin, int nx, int ny, int nz, int pitch, TileMaps* m)
@@ -1037,49 +1064,51 @@ int appfis_gb_himeno(const float* const* coef, float* p, float* wrk2, int nx, in
     cudaStream_t st = gb::as_stream(stream);
     Coef12 cf;
     for (int n = 0; n < 12; n++) cf.c[n] = coef[n];
-    dim3 blk(RX, RY), grd(gb::ceil_div(nx, RX), gb::ceil_div(ny, RY), gb::ceil_div(nz, HKZ));
+    dim3 blk(RX, RY);
     GosaSeq gs;
     float* buf[2] = {p, wrk2};
     int ci = 0;
-    if (plain_tma_ok(coef, p, wrk2, pitch)) {
-        // TMA-staged form: tile x origins on 32-point boundaries of the padded row
-        TileMaps maps[2];
-        GB_TRY(plain_maps(coef, p, nx, ny, nz, pitch, &maps[0]));
-        maps[1] = maps[0];
-        GB_TRY(gb::tensor_map_3d(&maps[1].m[12], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, wrk2, nx + 2, ny + 2, nz + 2, pitch,
-                                 ny + 2, TmaLayout::W, RY + 2));
-        unsigned* status;
-        GB_TRY(gb::status_word(&status));
-        constexpr int smem = TmaLayout::smem(TMA_S_PLAIN);
-        GB_CUDA(cudaFuncSetAttribute(himeno_tma<TMA_S_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        // z chunks of 16-48 planes whose grid fills the resident CTAs in whole waves (each chunk
-        // re-reads 2 halo planes of p)
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, himeno_tma<TMA_S_PLAIN>, RX * RY, smem) != cudaSuccess ||
-            per_sm < 1)
-            per_sm = 1;
-        const long long cols = (long long)(nx / RX + 1) * gb::ceil_div(ny, RY);
-        const int kz = gb::wave_chunk(nz, 16, 48, cols, (long long)per_sm * gb::sm_count(), 2);
-        dim3 tgrd(nx / RX + 1, gb::ceil_div(ny, RY), gb::ceil_div(nz, kz));
-        GB_TRY(gs.init(dev_gosa, (size_t)tgrd.x * tgrd.y * tgrd.z, 1));
+    // the flat sweep below ~6 M points or without 16-byte rows (measured lines at himeno_flat)
+    if (!plain_tma_ok(coef, p, wrk2, pitch) || (size_t)nx * ny * nz <= FLAT_POINTS) {
+        const FlatPlan<0> fp(ny, nz, pitch);
+        const dim3 fgrd(fp.blocks);
+        GB_TRY(gs.init(dev_gosa, fgrd.x, 1));
+        H10 none = {};
         for (int it = 0; it < iters; it++) {
-            gb::launch(himeno_tma<TMA_S_PLAIN>, tgrd, blk, smem, st, maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, kz, omega,
-                                                            gs.next(tgrd, 1, dev_gosa ? dev_gosa + it : nullptr), status);
+            gb::launch(fp.kernel, fgrd, FT, 0, st, cf, none, buf[ci], buf[1 - ci], nullptr, nx, ny, nz, pitch, fp.plane_blocks, omega, 0.0f,
+                       gs.next(fgrd, 1, dev_gosa ? dev_gosa + it : nullptr));
             ci = 1 - ci;
         }
-        GB_TRY(gb::launched("himeno_tma<plain>"));
         GB_TRY(gs.flush(st));
         if (cur_index) *cur_index = ci;
-        return APPFIS_GB_OK;
+        return gb::launched("himeno_flat<plain>");
     }
-    GB_TRY(gs.init(dev_gosa, (size_t)grd.x * grd.y * grd.z, 1));
-    H10 none = {};
+    // TMA-staged form: tile x origins on 32-point boundaries of the padded row
+    TileMaps maps[2];
+    GB_TRY(plain_maps(coef, p, nx, ny, nz, pitch, &maps[0]));
+    maps[1] = maps[0];
+    GB_TRY(gb::tensor_map_3d(&maps[1].m[12], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, wrk2, nx + 2, ny + 2, nz + 2, pitch,
+                             ny + 2, TmaLayout::W, RY + 2));
+    unsigned* status;
+    GB_TRY(gb::status_word(&status));
+    constexpr int smem = TmaLayout::smem(TMA_S_PLAIN);
+    GB_CUDA(cudaFuncSetAttribute(himeno_tma<TMA_S_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // z chunks of 16-48 planes whose grid fills the resident CTAs in whole waves (each chunk
+    // re-reads 2 halo planes of p)
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, himeno_tma<TMA_S_PLAIN>, RX * RY, smem) != cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
+    const long long cols = (long long)(nx / RX + 1) * gb::ceil_div(ny, RY);
+    const int kz = gb::wave_chunk(nz, 16, 48, cols, (long long)per_sm * gb::sm_count(), 2);
+    dim3 tgrd(nx / RX + 1, gb::ceil_div(ny, RY), gb::ceil_div(nz, kz));
+    GB_TRY(gs.init(dev_gosa, (size_t)tgrd.x * tgrd.y * tgrd.z, 1));
     for (int it = 0; it < iters; it++) {
-        gb::launch(himeno_ring<0>, grd, blk, 0, st, cf, none, buf[ci], buf[1 - ci], nullptr, nx, ny, nz, pitch, ny + 2, HKZ, omega, 0.0f,
-                                            gs.next(grd, 1, dev_gosa ? dev_gosa + it : nullptr));
+        gb::launch(himeno_tma<TMA_S_PLAIN>, tgrd, blk, smem, st, maps[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, kz, omega,
+                                                        gs.next(tgrd, 1, dev_gosa ? dev_gosa + it : nullptr), status);
         ci = 1 - ci;
     }
-    GB_TRY(gb::launched("himeno_ring<plain>"));
+    GB_TRY(gb::launched("himeno_tma<plain>"));
     GB_TRY(gs.flush(st));
     if (cur_index) *cur_index = ci;
     return APPFIS_GB_OK;
@@ -1119,7 +1148,7 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     GB_CUDA(cudaMemsetAsync(p_work, 0, sizeof(float) * field, st));
     himeno_half_coef<<<dim3(gb::ceil_div(nx, 128), ny, nz), 128, 0, st>>>(cf, Hc, field, nx, ny, nz, pitch, ny + 2);
     dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, HKZ));
-    dim3 rblk(RX, RY), rgrd(gb::ceil_div(nx, RX), gb::ceil_div(ny, RY), gb::ceil_div(nz, HKZ));
+    dim3 rblk(RX, RY);
     // TMA-staged inner sweeps (two points per thread) when the FP16 rows are 16-byte aligned
     // (pitch a multiple of 8)
     const bool use_tma = pitch % 8 == 0 && gb::aligned16(hw) && gb::aligned16(coef[3]);
@@ -1199,9 +1228,17 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
         ckz = gb::wave_chunk(nz, 16, 64, (long long)(nx / RX + 1) * gb::ceil_div(ny, RY), (long long)per_sm * gb::sm_count(), 2);
     }
     dim3 cgrd(nx / RX + 1, gb::ceil_div(ny, RY), gb::ceil_div(nz, ckz));
+    // the flat sweep without 16-byte rows, and on small grids that ask for no gosa (the staged sweep sums
+    // its squares in single floats: a better sum would be another one, in the ninth digit).  Us per sweep,
+    // staged / flat: 65 x 65 x 129 26 / 6.2, 100 x 100 x 200 29 / 21, 129 x 129 x 257 35.9 / 35.9, 160 x 160 x 300 46 / 60
+    const bool flat = !use_tma || (!dev_gosa && !two && (size_t)nx * ny * nz <= FLAT_MIXED_POINTS);
+    const FlatPlan<1> aligned_plan(ny, nz, pitch);
+    const FlatPlan<2> fplan(ny, nz, pitch);
+    auto fkern = use_tma ? aligned_plan.kernel : fplan.kernel;
+    const dim3 fgrd(fplan.blocks);
     GosaSeq gs;  // block sums of the sweeps and of the correction passes (which do a sweep each)
     {
-        const unsigned nb1 = use_tma ? tgrd.x * tgrd.y * tgrd.z : rgrd.x * rgrd.y * rgrd.z;
+        const unsigned nb1 = flat ? fgrd.x : tgrd.x * tgrd.y * tgrd.z;
         const unsigned nb2 = two ? 2 * t2grd.x * t2grd.y * t2grd.z : 0;
         const unsigned nb3 = use_tma ? cgrd.x * cgrd.y * cgrd.z : grd.x * grd.y * grd.z;
         GB_TRY(gs.init(dev_gosa, std::max(std::max(nb1, nb2), nb3), 1));
@@ -1249,12 +1286,13 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
                                                                gs.next(t2grd, 2, dev_gosa ? dev_gosa + it : nullptr), status);
                 it += 2;
             } else {
-                if (use_tma)
-                    gb::launch(tkern, tgrd, tblk, tsmem, st, tmaps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, tkz, omega, inv_omega,
-                                                     gs.next(tgrd, 1, dev_gosa ? dev_gosa + it : nullptr), status);
+                double* out = dev_gosa ? dev_gosa + it : nullptr;
+                if (flat)
+                    gb::launch(fkern, fgrd, FT, 0, st, cf, hf, E[ec], E[1 - ec], Dd, nx, ny, nz, pitch, fplan.plane_blocks, omega, inv_omega,
+                               gs.next(fgrd, 1, out));
                 else
-                    gb::launch(himeno_ring<1>, rgrd, rblk, 0, st, cf, hf, E[ec], E[1 - ec], Dd, nx, ny, nz, pitch, ny + 2, HKZ, omega,
-                                                          inv_omega, gs.next(rgrd, 1, dev_gosa ? dev_gosa + it : nullptr));
+                    gb::launch(tkern, tgrd, tblk, tsmem, st, tmaps[ec], E[1 - ec], nx, ny, nz, pitch, ny + 2, tkz, omega, inv_omega,
+                               gs.next(tgrd, 1, out), status);
                 it += 1;
             }
             ec = 1 - ec;
