@@ -12,6 +12,7 @@
 //   star_r4_tma    (TMA_X4 / TMA_X2) planes moved by the tensor memory accelerator into an
 //                  mbarrier ring, 4 or 2 x points x 2 rows per thread, packed FP32-pair math;
 //                  needs 16-byte rows (the default whenever they are);
+//   star_r4_async  (AUTO only) the same tile for rows that are not, planes copied with cp.async;
 //   star_r4_vec    (VEC) 4 x points per thread, register-staged plane loads;
 //   star_r4_sweep  (SCALAR2 / SCALAR4) one x point, 2 or 4 rows per thread, any pitch.
 //
@@ -378,6 +379,7 @@ template <> __device__ __forceinline__ void stgv<float, 2>(float* p, const float
 {
     *reinterpret_cast<float2*>(p) = make_float2(r[0], r[1]);
 }
+template <> __device__ __forceinline__ void stgv<float, 1>(float* p, const float* r) { *p = r[0]; }
 template <> __device__ __forceinline__ void stgv<__half, 4>(__half* p, const float* r)
 {
     Vec4<__half>::st(p, make_float4(r[0], r[1], r[2], r[3]));
@@ -550,6 +552,168 @@ __global__ void __launch_bounds__(128, VXT == 4 ? (TRY == 2 ? 4 : 2) : 6) star_r
     }
 }
 
+// Four points of one row: x window xw[0..11] (x-4 .. x+7, centre xw[4..7]), y neighbours
+// ym[a-1] / yp[a-1] (rows -a / +a), z queue q (9 planes, the centre at index (P + 4) % 9).
+// CHAIN: the weighted form as w0 c rounded, then one FMA per ring; otherwise its first two terms are
+// fma(w0, c, w1 ring1).
+template <int MODE, bool CHAIN = true>
+__device__ __forceinline__ void star4(const float* xw, const VecN<4>* ym, const VecN<4>* yp, const VecN<4>* q, int P, float coeff,
+                                      const StarW& wt, float* res)
+{
+    namespace f2 = gb::f2;
+#pragma unroll
+    for (int c = 0; c < 4; c += 2) {
+        const float2 cen = make_float2(xw[R + c], xw[R + c + 1]);
+        float2 v = MODE == 0 || !CHAIN ? cen : f2::mul(f2::splat(wt.w[0]), cen);
+#pragma unroll
+        for (int a = 1; a <= R; a++) {
+            const float2 sx = (a & 1) ? make_float2(__fadd_rn(xw[R + c - a], xw[R + c + a]), __fadd_rn(xw[R + c + 1 - a], xw[R + c + 1 + a]))
+                                      : f2::add(make_float2(xw[R + c - a], xw[R + c + 1 - a]), make_float2(xw[R + c + a], xw[R + c + 1 + a]));
+            const float2 sy = f2::add(make_float2(ym[a - 1].v[c], ym[a - 1].v[c + 1]), make_float2(yp[a - 1].v[c], yp[a - 1].v[c + 1]));
+            const VecN<4>& zm = q[(P + 4 - a) % 9];
+            const VecN<4>& zp = q[(P + 4 + a) % 9];
+            const float2 sz = f2::add(make_float2(zm.v[c], zm.v[c + 1]), make_float2(zp.v[c], zp.v[c + 1]));
+            const float2 ring = f2::add(f2::add(sx, sy), sz);
+            if (MODE == 0) v = f2::add(v, ring);
+            else if (!CHAIN && a == 1) v = f2::fma(f2::splat(wt.w[0]), cen, f2::mul(f2::splat(wt.w[1]), ring));
+            else v = f2::fma(f2::splat(wt.w[a]), ring, v);
+        }
+        if (MODE == 0) v = f2::mul(v, f2::splat(coeff));
+        res[c] = v.x;
+        res[c + 1] = v.y;
+    }
+}
+
+// ---------------------------------------------------------------- the same tile with plain asynchronous copies
+// Rows that are not 16-byte aligned (the reference's dense rows of nx + 8) cannot be moved by the tensor
+// memory accelerator: here the 128 threads copy each plane's 72 x 24 box into the same ring with cp.async
+// of WB = 8 or 4 bytes, the most that rows and fields are aligned to (8: FP32 rows of an even pitch,
+// FP16 of a multiple of 4; 4: any FP32 row, FP16 of an even pitch), word by word over the whole box,
+// and store WB bytes at a time.  One barrier per plane: behind it plane k + 4 has landed and everyone
+// is done with plane k - 1, whose slot takes plane k + 7.
+template <int WB>
+__device__ __forceinline__ void cp_async(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(gb::tma::smem_u32(dst)), "l"(src), "n"(WB) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <class T, int MODE, int WB>
+__global__ void __launch_bounds__(128, 4) star_r4_async(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz, int px, int py,
+                                                        int kz, float coeff, StarW wt)
+{
+    const gb::BlockId bid = gb::grid_wait();
+    typedef TmaStar<T, 4, 2> Lay;
+    constexpr int SW = Lay::SW, TTY = Lay::TTY, TRY = 2, NT = 128;
+    constexpr int EPW = WB / (int)sizeof(T), WPR = SW / EPW;  // elements per word, words per row
+    constexpr int FULL = WPR / 32 * 32, REST = WPR - FULL;    // words of a row that whole warps take, and the others
+    extern __shared__ __align__(128) unsigned char tsm[];
+    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 16 + tx;
+    const int bx0 = bid.x * Lay::TX, by0 = bid.y * TTY;
+    const int x = R + bx0 + 4 * tx, y = R + by0 + TRY * ty;
+    const int k0 = R + bid.z * kz, k1 = min(k0 + kz, nz + R), plast = k1 + R - 1, pbase = k0 - R;
+    const size_t plane = (size_t)px * py;
+    auto slot = [&](int pl) { return reinterpret_cast<T*>(tsm + ((unsigned)(pl - pbase) % TNS) * Lay::SLOT); };
+    const int xw_end = nx + 2 * R - bx0, yr_end = ny + 2 * R - by0;  // box columns / rows inside the field
+    const bool inside = xw_end >= SW && yr_end >= Lay::SH;
+    // each warp takes every fourth row's first FULL words; the REST words of all rows follow, NT at a time
+    const int lane = t & 31, warp = t >> 5;
+    const size_t first = (size_t)by0 * px + bx0;
+    auto load = [&](int pl) {
+        unsigned char* d = reinterpret_cast<unsigned char*>(slot(pl));
+        const T* s0 = in + (size_t)pl * plane + first;
+        const T* s = s0 + (size_t)warp * px + EPW * lane;
+        unsigned char* w = d + (warp * WPR + lane) * WB;
+#pragma unroll
+        for (int n = 0; n < Lay::SH / 4; n++) {
+            if (inside || warp + 4 * n < yr_end) {
+#pragma unroll
+                for (int c = 0; c < FULL; c += 32)
+                    if (inside || EPW * (lane + c) < xw_end) cp_async<WB>(w + (4 * n * WPR + c) * WB, s + EPW * c);
+            }
+            s += 4 * (size_t)px;
+        }
+#pragma unroll
+        for (int n = 0; n < (REST * Lay::SH + NT - 1) / NT; n++) {
+            const int i = t + n * NT, r = i / REST, c = FULL + i % REST;
+            if (i < REST * Lay::SH && (inside || (r < yr_end && EPW * c < xw_end)))
+                cp_async<WB>(d + (r * WPR + c) * WB, s0 + (size_t)r * px + EPW * c);
+        }
+        cp_async_commit();
+    };
+    const int own = (TRY * ty + R) * SW + R + 4 * tx;
+    VecN<4> q[TRY][9];
+    // planes k0 - 4 .. k0 + 3, which always exist, into the queues; then k0 + 4 .. k0 + 6 on their way
+    for (int pl = pbase; pl < pbase + TNS; pl++) load(pl);
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 8; m++)
+#pragma unroll
+        for (int r = 0; r < TRY; r++) q[r][m] = ldsv<T, 4>(slot(pbase + m) + own + r * SW);
+    __syncthreads();
+    for (int pl = pbase + TNS; pl < pbase + TNS + 3; pl++) {  // one group each, also past the last plane
+        if (pl <= plast) load(pl);
+        else cp_async_commit();
+    }
+    for (int kb = k0; kb < k1; kb += 9) {
+#pragma unroll
+        for (int P = 0; P < 9; P++) {
+            const int k = kb + P;
+            if (k < k1) {
+                cp_async_wait<2>();
+                __syncthreads();
+                if (k + TNS - 1 <= plast) load(k + TNS - 1);
+                else cp_async_commit();
+#pragma unroll
+                for (int r = 0; r < TRY; r++) q[r][(P + 8) % 9] = ldsv<T, 4>(slot(k + R) + own + r * SW);
+                const T* rowp = slot(k) + own;
+                VecN<4> wv[8];
+#pragma unroll
+                for (int a = 1; a <= R; a++) {
+                    wv[a - 1] = ldsv<T, 4>(rowp - a * SW);
+                    wv[R + a - 1] = ldsv<T, 4>(rowp + (TRY - 1 + a) * SW);
+                }
+#pragma unroll
+                for (int r = 0; r < TRY; r++) {
+                    float xw[12];
+                    const VecN<4> lo = ldsv<T, 4>(rowp + r * SW - R), hi = ldsv<T, 4>(rowp + r * SW + 4);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        xw[e] = lo.v[e];
+                        xw[4 + e] = q[r][(P + 4) % 9].v[e];
+                        xw[8 + e] = hi.v[e];
+                    }
+                    VecN<4> ym[R], yp[R];
+#pragma unroll
+                    for (int a = 1; a <= R; a++) {
+                        const int mm = r - a, mp = r + a;
+                        ym[a - 1] = mm >= 0 ? q[mm < TRY ? mm : 0][(P + 4) % 9] : wv[-mm - 1 < 0 ? 0 : -mm - 1];
+                        yp[a - 1] = mp < TRY ? q[mp < TRY ? mp : 0][(P + 4) % 9] : wv[R + mp - TRY < 0 ? 0 : R + mp - TRY];
+                    }
+                    float res[4];
+                    star4<MODE, false>(xw, ym, yp, q[r], P, coeff, wt, res);
+                    if (y + r < ny + R) {
+                        T* o = out + (size_t)k * plane + (size_t)(y + r) * px + x;
+#pragma unroll
+                        for (int e = 0; e < 4; e += EPW) {
+                            if (EPW > 1 && x + e + EPW <= nx + R) {
+                                stgv<T, EPW>(o + e, res + e);
+                            } else {
+#pragma unroll
+                                for (int f = e; f < e + EPW; f++)
+                                    if (x + f < nx + R) st<T>(o + f, res[f]);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- time-blocked form: two steps per launch
 // A CTA owns a 64 x TY output tile and a chunk of z planes, and advances it by TWO time steps
 // while each input plane crosses the chip once: the output of step 1 ("level 1") is never
@@ -589,34 +753,6 @@ struct TbStar {
     static constexpr int L1S = (L1P + 127) / 128 * 128;
     static constexpr int smem() { return TB_NS * SLOT + TB_L1 * L1S + TB_NS * 8; }
 };
-
-// Four points of one row: x window xw[0..11] (x-4 .. x+7, centre xw[4..7]), y neighbours
-// ym[a-1] / yp[a-1] (rows -a / +a), z queue q (9 planes, the centre at index (P + 4) % 9).
-template <int MODE>
-__device__ __forceinline__ void star4(const float* xw, const VecN<4>* ym, const VecN<4>* yp, const VecN<4>* q, int P, float coeff,
-                                      const StarW& wt, float* res)
-{
-    namespace f2 = gb::f2;
-#pragma unroll
-    for (int c = 0; c < 4; c += 2) {
-        const float2 cen = make_float2(xw[R + c], xw[R + c + 1]);
-        float2 v = MODE == 0 ? cen : f2::mul(f2::splat(wt.w[0]), cen);
-#pragma unroll
-        for (int a = 1; a <= R; a++) {
-            const float2 sx = (a & 1) ? make_float2(__fadd_rn(xw[R + c - a], xw[R + c + a]), __fadd_rn(xw[R + c + 1 - a], xw[R + c + 1 + a]))
-                                      : f2::add(make_float2(xw[R + c - a], xw[R + c + 1 - a]), make_float2(xw[R + c + a], xw[R + c + 1 + a]));
-            const float2 sy = f2::add(make_float2(ym[a - 1].v[c], ym[a - 1].v[c + 1]), make_float2(yp[a - 1].v[c], yp[a - 1].v[c + 1]));
-            const VecN<4>& zm = q[(P + 4 - a) % 9];
-            const VecN<4>& zp = q[(P + 4 + a) % 9];
-            const float2 sz = f2::add(make_float2(zm.v[c], zm.v[c + 1]), make_float2(zp.v[c], zp.v[c + 1]));
-            if (MODE == 0) v = f2::add(v, f2::add(f2::add(sx, sy), sz));
-            else v = f2::fma(f2::splat(wt.w[a]), f2::add(f2::add(sx, sy), sz), v);
-        }
-        if (MODE == 0) v = f2::mul(v, f2::splat(coeff));
-        res[c] = v.x;
-        res[c + 1] = v.y;
-    }
-}
 
 template <class T, int MODE, int TY>
 __global__ void __launch_bounds__(TbStar<T, TY>::NT, 1) star_r4_tb2(const __grid_constant__ CUtensorMap map, T* __restrict__ out, int nx,
@@ -749,6 +885,25 @@ __global__ void __launch_bounds__(TbStar<T, TY>::NT, 1) star_r4_tb2(const __grid
     }
 }
 
+// z planes per CTA: the count that finishes in the fewest plane-times, a wave of resident CTAs taking its
+// own planes and the 2R it reads before the first of them.
+int star_chunk(int nz, long long per_chunk, long long slots)
+{
+    int best = 1;
+    double cost = 1e30;
+    for (int chunks = (nz + 63) / 64; chunks <= nz; chunks++) {
+        const int kz = (nz + chunks - 1) / chunks;
+        if (kz < 3 && chunks > 1) break;
+        const long long ctas = per_chunk * ((nz + kz - 1) / kz), waves = (ctas + slots - 1) / slots;
+        const double c = (double)waves * (kz + 2 * R);
+        if (c < cost - 1e-9) {
+            cost = c;
+            best = kz;
+        }
+    }
+    return best;
+}
+
 // Runs `pairs` double steps (a -> b in two steps per launch, ping-pong); the caller does any odd
 // step with the single-step tile.
 template <class T, int TY>
@@ -779,6 +934,26 @@ int run_star_tb2(T** buf, int nx, int ny, int nz, int pitch, int pairs, int mode
     return gb::launched("star_r4_tb2");
 }
 
+template <class T, int WB>
+int run_star_async(T** buf, int nx, int ny, int nz, int pitch, int iters, int mode, float coeff, StarW w, int kz, int* cur_index,
+                   cudaStream_t st)
+{
+    typedef TmaStar<T, 4, 2> Lay;
+    constexpr int smem = TNS * Lay::SLOT;
+    auto kern = mode == 0 ? star_r4_async<T, 0, WB> : star_r4_async<T, 1, WB>;
+    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    const int tkz = kz > 0 ? kz : star_chunk(nz, (long long)gb::ceil_div(nx, Lay::TX) * gb::ceil_div(ny, Lay::TTY), (long long)per_sm * gb::sm_count());
+    dim3 blk(16, 8), grd(gb::ceil_div(nx, Lay::TX), gb::ceil_div(ny, Lay::TTY), gb::ceil_div(nz, tkz));
+    int ci = 0;
+    for (int it = 0; it < iters; it++, ci = 1 - ci)
+        gb::launch(kern, grd, blk, smem, st, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2 * R, tkz, coeff, w);
+    GB_TRY(gb::launched("star_r4_async"));
+    if (cur_index) *cur_index = ci;
+    return APPFIS_GB_OK;
+}
+
 template <class T, int MODE, int RY>
 void launch_star(const T* in, T* out, int nx, int ny, int nz, int px, int kz, float coeff, StarW w, cudaStream_t st)
 {
@@ -803,16 +978,14 @@ int run_star_tma(T** buf, int nx, int ny, int nz, int pitch, int iters, int mode
     constexpr int smem = Lay::smem();
     auto kern = mode == 0 ? star_r4_tma<T, 0, VXT, TRY> : star_r4_tma<T, 1, VXT, TRY>;
     GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    // default z chunk: 32-64 planes per CTA, the length whose grid fills the resident CTAs in the
-    // most nearly whole waves, counting the 8 halo planes each chunk re-reads (512^3: 47 planes,
-    // 2816 CTAs in 4.6 waves of 608)
+    // default z chunk: star_chunk (512^3: 57 planes, 2304 CTAs in 3.8 waves of 608; 250 x 127 x 130: 7 planes, one
+    // wave, where chunks of 32 and more left three quarters of the slots empty: 22.0 -> 11.9 us per step)
     int tkz = kz;
     if (tkz <= 0) {
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 16 * (TTY / TRY), smem) != cudaSuccess || per_sm < 1)
             per_sm = 1;
-        tkz = gb::wave_chunk(nz, 32, 64, (long long)gb::ceil_div(nx, Lay::TX) * gb::ceil_div(ny, TTY),
-                             (long long)per_sm * gb::sm_count(), 2 * R);
+        tkz = star_chunk(nz, (long long)gb::ceil_div(nx, Lay::TX) * gb::ceil_div(ny, TTY), (long long)per_sm * gb::sm_count());
     }
     dim3 blk(16, TTY / TRY), grd(gb::ceil_div(nx, Lay::TX), gb::ceil_div(ny, TTY), gb::ceil_div(nz, tkz));
     unsigned long long wait_ns = 1000000000ull, test_ns = 0;
@@ -839,8 +1012,8 @@ int run_star_tma(T** buf, int nx, int ny, int nz, int pitch, int iters, int mode
 // kernels write interior points only), then three more times between CUDA events on the
 // caller's stream, and the fastest time per step wins.  Candidates: on 16-byte aligned rows the
 // TMA-staged tiles with 4 or 2 x points per thread (depth 1) and the two-step tiles with 64 x 16
-// or 64 x 8 outputs (depth 2), otherwise the vector and scalar tiles; z chunks of the tile's
-// default and 32 .. 256 planes.  Depths 3 and 4 are not candidates: a depth-D tile keeps D
+// or 64 x 8 outputs (depth 2), otherwise AUTO's own choice and the vector and scalar tiles; z chunks of
+// the tile's default and 32 .. 256 planes.  Depths 3 and 4 are not candidates: a depth-D tile keeps D
 // register queues of 9 planes per point (36 D registers per thread of 4 points) over a region
 // 8 (D - 1) points wider and taller than its output, so at D = 3 a 64 x 8 output tile needs
 // 20 x 24 threads x about 160 registers (77 K > the 64 K register file of an SM), and smaller
@@ -936,8 +1109,8 @@ int tune_star(T* a, T* b, int dtype, int nx, int ny, int nz, int pitch, int mode
     std::vector<int> tiles;
     if (rows16)
         tiles = {APPFIS_GB_STAR_TMA_X4, APPFIS_GB_STAR_TMA_X4R4, APPFIS_GB_STAR_TMA_X2, APPFIS_GB_STAR_TB2, APPFIS_GB_STAR_TB2_8};
-    else if (vec4) tiles = {APPFIS_GB_STAR_VEC, APPFIS_GB_STAR_SCALAR4};
-    else tiles = {APPFIS_GB_STAR_SCALAR4, APPFIS_GB_STAR_SCALAR2};
+    else if (vec4) tiles = {APPFIS_GB_STAR_AUTO, APPFIS_GB_STAR_VEC, APPFIS_GB_STAR_SCALAR4};
+    else tiles = {APPFIS_GB_STAR_AUTO, APPFIS_GB_STAR_SCALAR4, APPFIS_GB_STAR_SCALAR2};
     std::vector<int> chunks = {0};
     for (int c : {32, 48, 64, 96, 128, 256})
         if (c < nz) chunks.push_back(c);
@@ -986,8 +1159,18 @@ int run_star(T* a, T* b, int nx, int ny, int nz, int pitch, int iters, int mode,
     T* buf[2] = {a, b};
     const bool rows16 = (pitch * sizeof(T)) % 16 == 0 && gb::aligned16(a) && gb::aligned16(b);
     const bool vec4 = pitch % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % (sizeof(T) * 4)) == 0;
-    if (tile == APPFIS_GB_STAR_AUTO)  // TMA-staged when rows are 16-byte aligned, else vectors, else scalar
-        tile = rows16 ? APPFIS_GB_STAR_TMA_X4 : (vec4 ? APPFIS_GB_STAR_VEC : APPFIS_GB_STAR_SCALAR4);
+    // AUTO: TMA-staged when rows are 16-byte aligned; else the tile with plain asynchronous copies where the
+    // grid fills it (half of its columns, 2 M points, 4 M if FP32 words are copied one by one); else
+    // vectors, else scalar.  Us per step, the smaller tiles (SCALAR2; FP16 260: VEC) / asynchronous:
+    //   FP32 40^3 3.7 / 4.4 (even pitch), 6.6 (odd); 100^3 8.6 / 9.1, 11.1; 130 x 140 x 150 15.0 / 14.0, 16.7;
+    //   250 x 127 x 130 18.1 / 15.6, 18.0; 250^3 71 / 57 (odd); 506^3 467 / 358, 433; 20 x 500 x 500 32 / 35, 52
+    //   FP16 100^3 6.7 / 8.2; 130 x 140 x 150 15.3 / 13.0; 250 x 127 x 130 (258) 18.8 / 12.5; 500^3 466 / 277
+    // (with the rows 16-byte aligned the TMA-staged tile takes 11.9 for 250 x 127 x 130, 206 for 512^3)
+    const unsigned long long align = (unsigned long long)pitch * sizeof(T) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
+    const bool one_word = sizeof(T) == 4 && align % 8 != 0;
+    const bool async = tile == APPFIS_GB_STAR_AUTO && !rows16 && align % 4 == 0 && 2 * nx >= 64 * (int)gb::ceil_div(nx, 64) &&
+                       (size_t)nx * ny * nz >= (one_word ? (size_t)4000000 : (size_t)2000000);
+    if (tile == APPFIS_GB_STAR_AUTO && !async) tile = rows16 ? APPFIS_GB_STAR_TMA_X4 : (vec4 ? APPFIS_GB_STAR_VEC : APPFIS_GB_STAR_SCALAR2);
     if ((tile == APPFIS_GB_STAR_TMA_X4 || tile == APPFIS_GB_STAR_TMA_X2 || tile == APPFIS_GB_STAR_TB2 || tile == APPFIS_GB_STAR_TB2_8 ||
          tile == APPFIS_GB_STAR_TMA_X4R4) &&
         !rows16)
@@ -1014,7 +1197,15 @@ int run_star(T* a, T* b, int nx, int ny, int nz, int pitch, int iters, int mode,
     if (tile == APPFIS_GB_STAR_TMA_X4R4)
         return run_star_tma<T, 4, 4>(buf, nx, ny, nz, pitch, iters, mode, coeff, w, kz, cur_index, st);
     if (tile == APPFIS_GB_STAR_TMA_X2) return run_star_tma<T, 2>(buf, nx, ny, nz, pitch, iters, mode, coeff, w, kz, cur_index, st);
-    if (kz <= 0) kz = 32;
+    if (async) {
+        if (align % 8 == 0) return run_star_async<T, 8>(buf, nx, ny, nz, pitch, iters, mode, coeff, w, kz, cur_index, st);
+        return run_star_async<T, 4>(buf, nx, ny, nz, pitch, iters, mode, coeff, w, kz, cur_index, st);
+    }
+    if (kz <= 0) {  // resident CTAs per SM: 2 of the vector tile, 4 of the scalar ones (3 counted: as fast or faster)
+        const bool vec = tile == APPFIS_GB_STAR_VEC;
+        const int ty = vec ? VTY : 8 * (tile == APPFIS_GB_STAR_SCALAR2 ? 2 : 4);
+        kz = star_chunk(nz, (long long)gb::ceil_div(nx, vec ? VTX : TX) * gb::ceil_div(ny, ty), (vec ? 2LL : 3LL) * gb::sm_count());
+    }
     int ci = 0;
     for (int it = 0; it < iters; it++) {
         if (tile == APPFIS_GB_STAR_VEC) {
@@ -1051,7 +1242,7 @@ int appfis_gb_star_r4(void* a, void* b, int dtype, int nx, int ny, int nz, int p
         tile != APPFIS_GB_STAR_TMA_X4 && tile != APPFIS_GB_STAR_TMA_X2 && tile != APPFIS_GB_STAR_VEC && tile != APPFIS_GB_STAR_TB2 &&
         tile != APPFIS_GB_STAR_TB2_8 && tile != APPFIS_GB_STAR_TMA_X4R4)
         return gb::fail(APPFIS_GB_EINVAL, "star_r4: unknown tile %d", tile);
-    int kz = zchunk <= 0 ? 0 : zchunk;  // 0: the tile's default (TMA-staged: 32-64 planes chosen for whole waves; 32 otherwise)
+    int kz = zchunk <= 0 ? 0 : zchunk;  // 0: the tile's default (chosen for whole waves of resident CTAs)
     cudaStream_t st = gb::as_stream(stream);
     if (tile == APPFIS_GB_STAR_AUTO) {  // a tuned choice for this device and shape, if there is one
         int dev = 0;

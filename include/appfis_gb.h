@@ -238,10 +238,11 @@ APPFIS_GB_API int appfis_gb_himeno_job(const float* coef_host, float* p_host, in
  * mode 1: weighted form  v = w[0]*c + sum_a w[a]*((x-a + x+a) + (y-a + y+a) + (z-a + z+a)).
  * dtype: APPFIS_GB_F32 or APPFIS_GB_F16 (storage).  tile selects the kernel (APPFIS_GB_STAR_*;
  * AUTO: the choice appfis_gb_star_r4_tune recorded for this device and shape, else the TMA-staged
- * tile when rows and fields are 16-byte aligned, else the vector tile when 4-element vectors are
- * aligned, else the scalar tile; all give the same results in the reference form and in FP32).  zchunk: z
- * planes per CTA (0 = the tile's default: TMA-staged 32-64 planes balanced over nz, the length that fills the
- * resident CTAs in the most nearly whole waves; 32 otherwise). */
+ * tile when rows and fields are 16-byte aligned, else by size the same tile with plain asynchronous
+ * copies, the vector tile (4-element vectors aligned) or the scalar tile; all give the same results in
+ * the reference form, and in the weighted form up to the rounding of its first two terms).  zchunk: z
+ * planes per CTA (0 = the tile's default: the length whose waves of resident CTAs take the fewest
+ * plane-times). */
 APPFIS_GB_API int appfis_gb_star_r4(void* a, void* b, int dtype, int nx, int ny, int nz, int pitch, int iters, int mode,
                                     float coeff, const float* weights, int tile, int zchunk, int* cur_index,
                                     void* stream);
