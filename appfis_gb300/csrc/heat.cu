@@ -7,10 +7,13 @@
 // contraction), so every point is bit-identical to the reference's CPU path.
 //
 // The 1024^2 workload is 8.4 MB for both buffers, so it lives in L2; one launch per sweep would
-// be launch-bound.  heat2d_regs therefore runs S sweeps per launch on a tile held on chip
-// (overlapped tiling: the tile plus an S-deep halo is loaded once, each sweep shrinks the valid
+// be launch-bound.  heat2d_bands therefore runs 8 sweeps per launch on a tile held on chip
+// (overlapped tiling: the tile plus an 8-deep halo is loaded once, each sweep shrinks the valid
 // region by one cell, the centre tile is written back).  Ghost-ring cells are loaded and held
-// constant, so Dirichlet boundaries are exact for any S.
+// constant, so Dirichlet boundaries are exact for any number of sweeps.
+#include <cmath>
+
+#include "f32x2.cuh"
 #include "gb_common.cuh"
 
 namespace {
@@ -35,125 +38,148 @@ __global__ void __launch_bounds__(256) heat2d_sweep_k(const float* __restrict__ 
                         cx, cy);
 }
 
-// Overlapped tiling: output tile TX x TY, halo S <= SMAX, S sweeps per launch (S is a template
-// argument: launch_heat_regs instantiates 1..SMAX and picks the launch's).  The
-// (TX + 2 SMAX) x (TY + 2 SMAX) region is cut into 4 x 4 blocks, one per thread, held in
-// registers for all S sweeps.  A sweep publishes each block's four edges (top and bottom rows,
-// left and right columns, one 16-byte vector each) into shared memory, synchronises once, reads
-// the facing edges of the four neighbour blocks and updates its 16 points: 8 shared-memory
-// vector operations per 16 point-updates.  Ghost-ring cells and cells outside the field keep
-// their values; every other cell of the region is updated each sweep (those outside the
-// shrinking valid window only feed cells that are not written back).  The point update is
-// heat_point, scalar: packed FP32-pair multiplies feeding pair adds are contracted to pair FMAs
-// by the code generator, which would change the rounding.
-constexpr int RBS = 4;  // block side
-
-template <int BX, int BY>
-struct HeatEdges {  // block edges, by sweep parity
-    float4 t[2][BY][BX], b[2][BY][BX], l[2][BY][BX], r[2][BY][BX];
-};
-
-// One tile, S sweeps (unrolled: the sweep-to-sweep register copies become renaming).  MASK:
-// the region reaches the ghost ring or beyond the field, so loads are guarded and only interior
-// cells are updated; tiles whose whole region is interior take the unmasked form.
-template <int TX, int TY, int SMAX, int S, bool MASK>
-__device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch,
-                                          float cx, float cy, HeatEdges<(TX + 2 * SMAX) / RBS, (TY + 2 * SMAX) / RBS>& e, gb::BlockId bid)
+// Two points of a row at once, each lane's operations those of heat_point: packed additions and
+// subtractions, except the x sums, whose operands straddle register pairs.  2c is c + c (the same value),
+// and the products are scalar, because the code generator contracts a packed product into the packed
+// addition that takes it.  12 instructions for two points instead of 18.
+__device__ __forceinline__ float2 heat_pair(float2 c, float2 l, float2 r, float2 u, float2 d, float cx, float cy)
 {
-    constexpr int BX = (TX + 2 * SMAX) / RBS, BY = (TY + 2 * SMAX) / RBS;
-    constexpr int rw = TX + 2 * S, rh = TY + 2 * S;  // region in use
-    const int t = threadIdx.x, bx = t % BX, by = t / BX;
-    const int ox = 1 + bid.x * TX - S, oy = 1 + bid.y * TY - S;  // padded coords of region (0,0)
-    float v[RBS][RBS];
-    unsigned upd = 0;  // MASK: bit 4r+c set for an interior cell of the region in use
-#pragma unroll
-    for (int r = 0; r < RBS; r++)
-#pragma unroll
-        for (int c = 0; c < RBS; c++) {
-            const int rx = RBS * bx + c, ry = RBS * by + r, gx = ox + rx, gy = oy + ry;
-            if (MASK) {
-                const bool used = rx < rw && ry < rh;
-                v[r][c] = (used && gx >= 0 && gx <= nx + 1 && gy >= 0 && gy <= ny + 1) ? __ldg(cur + (size_t)gy * pitch + gx) : 0.0f;
-                if (used && gx >= 1 && gx <= nx && gy >= 1 && gy <= ny) upd |= 1u << (RBS * r + c);
-            } else {
-                v[r][c] = __ldg(cur + (size_t)gy * pitch + gx);
-            }
-        }
-    const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int s = 1; s <= S; s++) {
-        // one barrier per sweep: a buffer is rewritten two sweeps later, after every thread has
-        // passed the next sweep's barrier and so finished reading it
-        const int q = s & 1;
-        e.t[q][by][bx] = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-        e.b[q][by][bx] = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
-        e.l[q][by][bx] = make_float4(v[0][0], v[1][0], v[2][0], v[3][0]);
-        e.r[q][by][bx] = make_float4(v[0][3], v[1][3], v[2][3], v[3][3]);
-        __syncthreads();
-        const float4 up = by > 0 ? e.b[q][by - 1][bx] : z4;
-        const float4 dn = by < BY - 1 ? e.t[q][by + 1][bx] : z4;
-        const float4 lf = bx > 0 ? e.r[q][by][bx - 1] : z4;
-        const float4 rt = bx < BX - 1 ? e.l[q][by][bx + 1] : z4;
-        const float upv[RBS] = {up.x, up.y, up.z, up.w}, dnv[RBS] = {dn.x, dn.y, dn.z, dn.w};
-        const float lfv[RBS] = {lf.x, lf.y, lf.z, lf.w}, rtv[RBS] = {rt.x, rt.y, rt.z, rt.w};
-        float nv[RBS][RBS];
-#pragma unroll
-        for (int r = 0; r < RBS; r++)
-#pragma unroll
-            for (int c = 0; c < RBS; c++) {
-                const float l = c > 0 ? v[r][c - 1] : lfv[r], rr = c + 1 < RBS ? v[r][c + 1] : rtv[r];
-                const float u = r > 0 ? v[r - 1][c] : upv[c], d = r + 1 < RBS ? v[r + 1][c] : dnv[c];
-                const float h = heat_point(v[r][c], l, rr, u, d, cx, cy);
-                nv[r][c] = !MASK || ((upd >> (RBS * r + c)) & 1u) ? h : v[r][c];
-            }
-#pragma unroll
-        for (int r = 0; r < RBS; r++)
-#pragma unroll
-            for (int c = 0; c < RBS; c++) v[r][c] = nv[r][c];
-    }
-#pragma unroll
-    for (int r = 0; r < RBS; r++)
-#pragma unroll
-        for (int c = 0; c < RBS; c++) {
-            const int x = RBS * bx + c - S, y = RBS * by + r - S;  // output tile coordinates
-            const int gx = 1 + bid.x * TX + x, gy = 1 + bid.y * TY + y;
-            if (x >= 0 && x < TX && y >= 0 && y < TY && (!MASK || (gx <= nx && gy <= ny))) nxt[(size_t)gy * pitch + gx] = v[r][c];
-        }
+    namespace f2 = gb::f2;
+    const float2 two_c = f2::add(c, c);
+    const float2 tx = f2::sub(make_float2(__fadd_rn(l.x, r.x), __fadd_rn(l.y, r.y)), two_c);
+    const float2 ty = f2::sub(f2::add(u, d), two_c);
+    const float2 x = make_float2(__fmul_rn(cx, tx.x), __fmul_rn(cx, tx.y));
+    const float2 y = make_float2(__fmul_rn(cy, ty.x), __fmul_rn(cy, ty.y));
+    return f2::add(f2::add(c, x), y);
 }
 
-template <int TX, int TY, int SMAX, int S>
-__global__ void __launch_bounds__(((TX + 2 * SMAX) / RBS) * ((TY + 2 * SMAX) / RBS))
-    heat2d_regs(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch, float cx, float cy)
+// Overlapped tiling: a CTA of W warps holds a 128 x 8W region in registers for up to 8 sweeps and writes
+// the 112 x (8W - 16) tile in its middle.  A warp owns a band of 8 rows, a lane 4 columns of it, so that the
+// x neighbours at a lane's edges come by shuffle and only a band's first and last row go through shared
+// memory (one 16-byte vector each per lane and sweep, one barrier).  A sweep works down the band and
+// replaces the rows as it goes, keeping one old row.  Ghost-ring cells and cells outside the field
+// keep their values; every other cell of the region is updated each sweep (those outside the shrinking
+// valid window only feed cells that are not written back).
+constexpr int HS = 8;             // sweeps per launch, and halo width
+constexpr int HR = 8;             // rows per band
+constexpr int HTX = 128 - 2 * HS;  // output columns
+
+template <int G> struct HeatVec;  // G floats that are aligned together
+template <> struct HeatVec<1> { typedef float type; };
+template <> struct HeatVec<2> { typedef float2 type; };
+template <> struct HeatVec<4> { typedef float4 type; };
+
+// MASK: the region reaches the ghost ring or beyond the field: loads are guarded and only interior cells
+// are updated and stored.
+template <int W, int G, bool MASK>
+__device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch, int ns, float cx,
+                                          float cy, int bx, int by, float4 (&top)[2][W][32], float4 (&bot)[2][W][32])
+{
+    typedef typename HeatVec<G>::type V;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int x = bx * HTX - HS + 4 * lane, y0 = 1 + by * (HR * W - 2 * HS) - HS + HR * w;  // padded coordinates of the first cell
+    float v[HR][4];
+    bool in[4];  // MASK: an interior column
+#pragma unroll
+    for (int c = 0; c < 4; c++) in[c] = !MASK || (x + c >= 1 && x + c <= nx);
+#pragma unroll
+    for (int r = 0; r < HR; r++) {
+        const float* row = cur + (ptrdiff_t)(y0 + r) * pitch + x;
+        if (MASK) {
+            const bool yin = y0 + r >= 0 && y0 + r <= ny + 1;
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[r][c] = yin && x + c >= 0 && x + c <= nx + 1 ? __ldg(row + c) : 0.0f;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; c += G) *reinterpret_cast<V*>(&v[r][c]) = __ldg(reinterpret_cast<const V*>(row + c));
+        }
+    }
+    const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
+    for (int s = 0; s < ns; s++) {
+        // one barrier per sweep: a half is rewritten two sweeps later, after every thread has passed the
+        // next sweep's barrier and so finished reading it
+        const int q = s & 1;
+        top[q][w][lane] = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+        bot[q][w][lane] = make_float4(v[HR - 1][0], v[HR - 1][1], v[HR - 1][2], v[HR - 1][3]);
+        __syncthreads();
+        const float4 up = w > 0 ? bot[q][w - 1][lane] : z4;
+        const float4 dn = w < W - 1 ? top[q][w + 1][lane] : z4;
+        float2 u01 = make_float2(up.x, up.y), u23 = make_float2(up.z, up.w);  // the row above, before this sweep
+#pragma unroll
+        for (int r = 0; r < HR; r++) {
+            const float lf = __shfl_up_sync(0xffffffffu, v[r][3], 1), rt = __shfl_down_sync(0xffffffffu, v[r][0], 1);
+            const float2 c01 = make_float2(v[r][0], v[r][1]), c23 = make_float2(v[r][2], v[r][3]);
+            const float2 d01 = r < HR - 1 ? make_float2(v[r < HR - 1 ? r + 1 : 0][0], v[r < HR - 1 ? r + 1 : 0][1]) : make_float2(dn.x, dn.y);
+            const float2 d23 = r < HR - 1 ? make_float2(v[r < HR - 1 ? r + 1 : 0][2], v[r < HR - 1 ? r + 1 : 0][3]) : make_float2(dn.z, dn.w);
+            const float2 h01 = heat_pair(c01, make_float2(lf, c01.x), make_float2(c01.y, c23.x), u01, d01, cx, cy);
+            const float2 h23 = heat_pair(c23, make_float2(c01.y, c23.x), make_float2(c23.y, rt), u23, d23, cx, cy);
+            if (!MASK || (y0 + r >= 1 && y0 + r <= ny)) {  // uniform in the warp
+                v[r][0] = in[0] ? h01.x : c01.x;
+                v[r][1] = in[1] ? h01.y : c01.y;
+                v[r][2] = in[2] ? h23.x : c23.x;
+                v[r][3] = in[3] ? h23.y : c23.y;
+            }
+            u01 = c01;
+            u23 = c23;
+        }
+    }
+    if (lane < HS / 4 || lane >= 32 - HS / 4) return;
+#pragma unroll
+    for (int r = 0; r < HR; r++) {
+        if (HR * w + r < HS || HR * w + r >= HR * W - HS) continue;
+        float* row = nxt + (ptrdiff_t)(y0 + r) * pitch + x;
+        if (MASK) {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (in[c] && y0 + r <= ny) row[c] = v[r][c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; c += G) *reinterpret_cast<V*>(row + c) = *reinterpret_cast<V*>(&v[r][c]);
+        }
+    }
+}
+
+template <int W, int G>
+__global__ void __launch_bounds__(32 * W, 24 / W) heat2d_bands(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch,
+                                                            int ns, float cx, float cy)
 {
     const gb::BlockId bid = gb::grid_wait();
-    constexpr int BX = (TX + 2 * SMAX) / RBS, BY = (TY + 2 * SMAX) / RBS;
-    static_assert(BX * RBS == TX + 2 * SMAX && BY * RBS == TY + 2 * SMAX, "region in whole blocks");
-    static_assert(S >= 1 && S <= SMAX, "sweeps per launch");
-    __shared__ HeatEdges<BX, BY> e;
-    // the whole region (TX + 2 SMAX wide, loaded in full) lies on interior cells
-    const bool inner = S == SMAX && (int)bid.x * TX >= S && (int)bid.y * TY >= S &&
-                       ((int)bid.x + 1) * TX + S <= nx && ((int)bid.y + 1) * TY + S <= ny;
-    if (inner)
-        heat_tile<TX, TY, SMAX, S, false>(cur, nxt, nx, ny, pitch, cx, cy, e, bid);
+    __shared__ float4 top[2][W][32], bot[2][W][32];
+    const int bx = (int)bid.x, by = (int)bid.y, x0 = bx * HTX - HS, y0 = 1 + by * (HR * W - 2 * HS) - HS;
+    if (x0 >= 1 && y0 >= 1 && x0 + 127 <= nx && y0 + HR * W - 1 <= ny)  // the whole region lies on interior cells
+        heat_tile<W, G, false>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
     else
-        heat_tile<TX, TY, SMAX, S, true>(cur, nxt, nx, ny, pitch, cx, cy, e, bid);
+        heat_tile<W, G, true>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
 }
 
-template <int TX, int TY, int SMAX, int S = SMAX>
-void launch_heat_regs(int s, dim3 grd, const float* cur, float* nxt, int nx, int ny, int pitch, float cx, float cy,
-                      cudaStream_t st)
+long long heat_tiles(int w, int nx, int ny) { return (long long)gb::ceil_div(nx + 1, HTX) * gb::ceil_div(ny, HR * w - 2 * HS); }
+
+// Warps per CTA: 8 (112 x 48 tiles: 1.5 points computed per point written), unless a small grid's launch is
+// shorter with 4 (112 x 16 tiles, 2.3, but a third as long) or 12 (112 x 80, 1.4).  A launch lasts about
+// 3.2 us and 1.45 / 3.3 us for each tile of the fullest SM; 12 warps 9 us if every SM has one tile at most.
+// Us per 8 sweeps with 4 / 8 / 12 warps: 64^2 4.5 / 5.7 / 7.3; 512^2 5.9 / 6.4 / 8.7; 777 x 900 7.8 / 6.5 / 8.8;
+// 1024^2 10.6 / 9.6 / 8.8; 1500^2 17.1 / 13.4 / 14.9; 2048^2 28.4 / 22.4 / 23.8; 4096^2 97 / 72 / 72.
+// The 4 x 4 register blocks that this replaced (48 x 32 tiles, four edge vectors per thread and sweep through
+// shared memory): 6.4, 8.4, 14.5, 15.7, 26.4, 40.5, 139.  Bound by instruction issue and the sweep's
+// barrier; 16 warps 10.7 and more up to 1024^2.
+int heat_warps(int nx, int ny)
 {
-    if constexpr (S > 1) {
-        if (s < S) return launch_heat_regs<TX, TY, SMAX, S - 1>(s, grd, cur, nxt, nx, ny, pitch, cx, cy, st);
-    }
-    constexpr int threads = ((TX + 2 * SMAX) / RBS) * ((TY + 2 * SMAX) / RBS);
-    gb::launch(heat2d_regs<TX, TY, SMAX, S>, grd, threads, 0, st, cur, nxt, nx, ny, pitch, cx, cy);
+    const double sms = gb::sm_count();
+    auto full = [&](int w) { return std::ceil((double)heat_tiles(w, nx, ny) / sms); };
+    const double c4 = 3.2 + 1.45 * full(4), c8 = 3.2 + 3.3 * full(8), c12 = full(12) <= 1 ? 9.0 : 1e30;
+    return c8 <= c4 && c8 <= c12 ? 8 : (c12 <= c4 ? 12 : 4);
 }
 
-// 48 x 32 output tiles: a 64 x 48 region, 16 x 12 blocks, 192 threads of at most 96 registers,
-// 3 CTAs per SM.  The wider 64 x 32 tile (240 threads, 2 CTAs per SM) and every other shape
-// tried (40-56 wide, 24-40 high) measured slower.
-constexpr int HTX = 48, HTY = 32, HSMAX = 8;
+// The copies' width goes by the alignment of the rows (region rows start on 4-element boundaries).
+template <int W>
+void launch_bands(const float* cur, float* nxt, int nx, int ny, int pitch, int ns, float cx, float cy, cudaStream_t st)
+{
+    const dim3 grd(gb::ceil_div(nx + 1, HTX), gb::ceil_div(ny, HR * W - 2 * HS));
+    const unsigned long long align = (unsigned long long)pitch * sizeof(float) | reinterpret_cast<uintptr_t>(cur) | reinterpret_cast<uintptr_t>(nxt);
+    auto kern = align % 16 == 0 ? heat2d_bands<W, 4> : (align % 8 == 0 ? heat2d_bands<W, 2> : heat2d_bands<W, 1>);
+    gb::launch(kern, grd, 32 * W, 0, st, cur, nxt, nx, ny, pitch, ns, cx, cy);
+}
 
 int check_heat(const void* a, const void* b, int nx, int ny, int pitch)
 {
@@ -180,16 +206,18 @@ int appfis_gb_heat2d(float* a, float* b, int nx, int ny, int pitch, int iters, f
     GB_TRY(check_heat(a, b, nx, ny, pitch));
     if (iters < 0) return gb::fail(APPFIS_GB_EINVAL, "heat2d: negative iteration count");
     cudaStream_t st = gb::as_stream(stream);
-    dim3 grd(gb::ceil_div(nx, HTX), gb::ceil_div(ny, HTY));
+    const int warps = heat_warps(nx, ny);
     float* buf[2] = {a, b};
     int ci = 0;
     for (int done = 0; done < iters;) {
-        const int S = std::min(HSMAX, iters - done);
-        launch_heat_regs<HTX, HTY, HSMAX>(S, grd, buf[ci], buf[1 - ci], nx, ny, pitch, cx, cy, st);
+        const int ns = std::min(HS, iters - done);
+        if (warps == 8) launch_bands<8>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
+        else if (warps == 12) launch_bands<12>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
+        else launch_bands<4>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
         ci = 1 - ci;
-        done += S;
+        done += ns;
     }
-    GB_TRY(gb::launched("heat2d_regs"));
+    GB_TRY(gb::launched("heat2d_bands"));
     if (cur_index) *cur_index = ci;
     return APPFIS_GB_OK;
 }

@@ -994,7 +994,7 @@ def profile_case(name, local):
             (himeno_tma<1>, himeno_correct)
     fdtd:   512^3, 5 FP32 steps then 5 FP16 steps (star_r4_tma), then 2 two-step launches in FP32
             and 2 in FP16 (star_r4_tb2)
-    heat:   1024^2, 16 iterations (2 heat2d_regs launches)
+    heat:   1024^2, 16 iterations (2 heat2d_bands launches)
     himeno-small: 129x129x257, the mixed form with one inner sweep per launch (himeno_mixed2),
             then with two (himeno_mixed_tb2), 4 sweeps each (~0.3 GB)
     flood:  the 32-domain batch (80 M cells, ~2.6 GB), 20 steps (one flood_fused launch)
