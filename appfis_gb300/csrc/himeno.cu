@@ -168,25 +168,40 @@ __device__ __forceinline__ void gosa_end_flat(const SqAcc& acc, const GosaIO& g,
          W1)
 
 // ---------------------------------------------------------------- defect-correction form
-// FP16 copies of the ten neighbour / boundary coefficient fields (over the interior).
-__global__ void himeno_half_coef(Coef12 cf, __half* __restrict__ w, size_t field, int nx, int ny, int nz, int px, int py)
+// The ten neighbour / boundary coefficients among the twelve: a0 a1 a2 b0 b1 b2 c0 c1 c2 bnd.
+__host__ __device__ constexpr int half_of(int n) { return n < 3 ? n : n + 1; }
+
+// The end of a run: P' = P + e over the interior (what the correction pass writes to P', without the new
+// defect, which nothing would read).  Columns as in himeno_flat, FINISH_K planes per thread.
+constexpr int FINISH_K = 4;
+__global__ void __launch_bounds__(256) himeno_finish(const float* __restrict__ P, const __half* __restrict__ e, float* __restrict__ Pn, int nx,
+                                                     int ny, int nz, int px, unsigned plane_blocks)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y;
-    const int k = 1 + blockIdx.z;
-    if (i > nx) return;
-    const size_t c = ((size_t)k * py + j) * px + i;
-    const int map[10] = {0, 1, 2, 4, 5, 6, 7, 8, 9, 10};  // a0 a1 a2 b0 b1 b2 c0 c1 c2 bnd
+    const gb::BlockId bid = gb::grid_wait();
+    const unsigned zc = bid.x / plane_blocks;
+    const size_t q = (size_t)(bid.x - zc * plane_blocks) * 256 + threadIdx.x;
+    const int j = 1 + (int)(q / (unsigned)px), i = (int)(q - (size_t)(j - 1) * px), k0 = 1 + (int)zc * FINISH_K;
+    if (i < 1 || i > nx || j > ny) return;
+    const size_t plane = (size_t)px * (ny + 2), c = (size_t)k0 * plane + (size_t)j * px + i;
+    float v[FINISH_K], d[FINISH_K];
 #pragma unroll
-    for (int n = 0; n < 10; n++) w[n * field + c] = __float2half_rn(cf.c[map[n]][c]);
+    for (int u = 0; u < FINISH_K; u++)
+        if (k0 + u <= nz) {
+            v[u] = __ldcs(P + c + u * plane);
+            d[u] = __half2float(__ldcs(e + c + u * plane));
+        }
+#pragma unroll
+    for (int u = 0; u < FINISH_K; u++)
+        if (k0 + u <= nz) Pn[c + u * plane] = v[u] + d[u];
 }
 
-// Correction pass: P' = P + e, D = omega*ss(P'), e_next = 0.  Reads P and e at neighbours.
-template <int BX, int BY>
+// Correction pass: P' = P + e, D = omega*ss(P'), and the sweep after it, e = D.  Reads P and e at neighbours.  COPY (the first
+// pass of a run): also leaves the ten coefficients it has read in FP16, in the fields at `copy`.
+template <int BX, int BY, bool COPY>
 __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float* __restrict__ P, const __half* __restrict__ e,
                                                           float* __restrict__ Pn, __half* __restrict__ D,
-                                                          __half* __restrict__ enext, int nx, int ny, int nz, int px,
-                                                          int py, int kz, float omega, float inv_omega, int prime, GosaIO gz)
+                                                          __half* __restrict__ enext, __half* __restrict__ copy, size_t field, int nx,
+                                                          int ny, int nz, int px, int py, int kz, float omega, float inv_omega, GosaIO gz)
 {
     const gb::BlockId bid = gb::grid_wait();
     const int i = 1 + bid.x * BX + threadIdx.x;
@@ -209,11 +224,13 @@ __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float*
         const __half dh = __float2half_rn(omega * ss);
         Pn[c] = q0;
         D[c] = dh;
-        enext[c] = prime ? dh : __float2half_rn(0.0f);
-        if (prime) {  // the next sweep from e = 0 gives e = D exactly, with ss = D / omega
-            const float s1 = __half2float(dh) * inv_omega;
-            g = __fmaf_rn(s1, s1, g);
+        if (COPY) {
+#pragma unroll
+            for (int n = 0; n < 10; n++) copy[n * field + c] = __float2half_rn(__ldg(cf.c[half_of(n)] + c));
         }
+        enext[c] = dh;  // the next sweep from e = 0 gives e = D exactly, with ss = D / omega
+        const float s1 = __half2float(dh) * inv_omega;
+        g = __fmaf_rn(s1, s1, g);
         c += plane;
     }
     gosa_end<1>({(double)g}, gz);
@@ -878,11 +895,12 @@ __device__ __forceinline__ void q_box(const unsigned char* pbox, const unsigned 
     }
 }
 
-template <int S>
+template <int S, bool COPY>
 __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_constant__ CorrMaps maps, float* __restrict__ Pn,
-                                                              __half* __restrict__ D, __half* __restrict__ enext, int nx, int ny,
+                                                              __half* __restrict__ D, __half* __restrict__ enext,
+                                                              __half* __restrict__ copy, size_t field, int nx, int ny,
                                                               int nz, int pitch, int py, int kz, float omega, float inv_omega,
-                                                              int prime, GosaIO gz, unsigned* __restrict__ status)
+                                                              GosaIO gz, unsigned* __restrict__ status)
 {
     const gb::BlockId bid = gb::grid_wait();
     typedef TmaLayout Lay;
@@ -957,11 +975,13 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
             const __half dh = __float2half_rn(omega * ss);
             Pn[cc] = q0;
             D[cc] = dh;
-            enext[cc] = prime ? dh : __float2half_rn(0.0f);
-            if (prime) {  // the next sweep from e = 0 gives e = D exactly, with ss = D / omega
-                const float s1 = __half2float(dh) * inv_omega;
-                g = __fmaf_rn(s1, s1, g);
+            if (COPY) {
+#pragma unroll
+                for (int n = 0; n < 10; n++) copy[n * field + cc] = __float2half_rn(co[half_of(n)]);
             }
+            enext[cc] = dh;  // the next sweep from e = 0 gives e = D exactly, with ss = D / omega
+            const float s1 = __half2float(dh) * inv_omega;
+            g = __fmaf_rn(s1, s1, g);
         }
         // everyone is done with stage s, the slot of plane k-1 and the sums of plane k+2
         if (__syncthreads_or(bad)) break;
@@ -1144,9 +1164,10 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     H10 hf;
     for (int n = 0; n < 10; n++) hf.c[n] = Hc + n * field;
     hf.a3 = coef[3];
-    GB_CUDA(cudaMemsetAsync(hw, 0, sizeof(__half) * 13 * field, st));
+    // only e and p_work are read outside the interior (the two-sweep pass reads all fields on its ring)
+    if (sweeps_per_pass == 2) GB_CUDA(cudaMemsetAsync(hw, 0, sizeof(__half) * 13 * field, st));
+    else GB_CUDA(cudaMemsetAsync(E[0], 0, sizeof(__half) * 2 * field, st));
     GB_CUDA(cudaMemsetAsync(p_work, 0, sizeof(float) * field, st));
-    himeno_half_coef<<<dim3(gb::ceil_div(nx, 128), ny, nz), 128, 0, st>>>(cf, Hc, field, nx, ny, nz, pitch, ny + 2);
     dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, HKZ));
     dim3 rblk(RX, RY);
     // TMA-staged inner sweeps (two points per thread) when the FP16 rows are 16-byte aligned
@@ -1220,9 +1241,10 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     constexpr int csmem = corr_smem(CORR_S);
     int ckz = tkz;  // the correction pass's own z chunk: whole waves of its resident CTAs
     if (use_tma) {
-        GB_CUDA(cudaFuncSetAttribute(himeno_correct_tma<CORR_S>, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+        GB_CUDA(cudaFuncSetAttribute(himeno_correct_tma<CORR_S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+        GB_CUDA(cudaFuncSetAttribute(himeno_correct_tma<CORR_S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, himeno_correct_tma<CORR_S>, RX * RY, csmem) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, himeno_correct_tma<CORR_S, false>, RX * RY, csmem) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
         ckz = gb::wave_chunk(nz, 16, 64, (long long)(nx / RX + 1) * gb::ceil_div(ny, RY), (long long)per_sm * gb::sm_count(), 2);
@@ -1258,26 +1280,26 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     }
     int pc = 0, ec = 0;
     const float inv_omega = 1.0f / omega;
-    // The correction pass: P' = P + e into the other P buffer and D; with `prime` it also does
-    // the next period's first inner sweep, which from e = 0 yields e = D exactly (all neighbour
-    // terms vanish), so it writes e = D and that sweep's gosa; otherwise e = 0.
-    auto correct = [&](bool prime, double* g) {
-        const GosaIO gz = gs.next(use_tma ? cgrd : grd, 1, prime ? g : nullptr);
+    // The correction pass that opens a period: P' = P + e into the other P buffer and D; it also does the
+    // period's first inner sweep, which from e = 0 yields e = D exactly (all neighbour terms vanish), so
+    // it writes e = D and that sweep's gosa.  The run's first one leaves the FP16 coefficients on its way:
+    // it has them in hand, and a pass of its own over the FP32 fields cost 396 us at 257 x 257 x 513.
+    bool first = true;
+    auto correct = [&](double* g) {
+        const GosaIO gz = gs.next(use_tma ? cgrd : grd, 1, g);
         if (use_tma)
-            gb::launch(himeno_correct_tma<CORR_S>, cgrd, rblk, csmem, st, cmaps[pc][ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
-                                                                 ckz, omega, inv_omega, prime ? 1 : 0, gz, status);
+            gb::launch(first ? himeno_correct_tma<CORR_S, true> : himeno_correct_tma<CORR_S, false>, cgrd, rblk, csmem, st, cmaps[pc][ec], P[1 - pc],
+                       Dd, E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, ckz, omega, inv_omega, gz, status);
         else
-            gb::launch(himeno_correct<HBX, HBY>, grd, blk, 0, st, cf, P[pc], E[ec], P[1 - pc], Dd, E[1 - ec], nx, ny, nz, pitch, ny + 2,
-                                                          HKZ, omega, inv_omega, prime ? 1 : 0, gz);
+            gb::launch(first ? himeno_correct<HBX, HBY, true> : himeno_correct<HBX, HBY, false>, grd, blk, 0, st, cf, P[pc], E[ec], P[1 - pc], Dd,
+                       E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, HKZ, omega, inv_omega, gz);
+        first = false;
         pc = 1 - pc;
         ec = 1 - ec;
     };
-    // periods of `period` sweeps, each opened by a correction pass that does its first sweep;
-    // the last correction closes the run
-    for (int it = 0;;) {
-        const bool prime = it < iters;
-        correct(prime, dev_gosa ? dev_gosa + it : nullptr);
-        if (!prime) break;
+    // periods of `period` sweeps, each opened by a correction pass that does its first sweep
+    for (int it = 0; it < iters;) {
+        correct(dev_gosa ? dev_gosa + it : nullptr);
         const int end = std::min(iters, it + period);
         it += 1;
         while (it < end) {
@@ -1299,6 +1321,9 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
         }
     }
     GB_TRY(gs.flush(st));
+    const unsigned fpb = gb::ceil_div((size_t)ny * pitch, 256);
+    gb::launch(himeno_finish, fpb * ((nz + FINISH_K - 1) / FINISH_K), 256, 0, st, P[pc], E[ec], P[1 - pc], nx, ny, nz, pitch, fpb);
+    pc = 1 - pc;
     GB_TRY(gb::launched("himeno_mixed"));
     if (cur_index) *cur_index = pc;
     return APPFIS_GB_OK;
