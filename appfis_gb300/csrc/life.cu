@@ -286,23 +286,28 @@ __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restric
 }
 
 // ------------------------------------------------------------------------------ bit-packed, time-blocked
-// Up to TB_STEPS generations per launch on a tile held in shared memory.  A CTA owns output words
-// [30*tx, 30*tx + 30) x rows [R*ty, R*ty + R) and loads a 32-word x (R + 2*steps)-row region
-// around it (periodic wrap at load time, so the region is a consistent periodic window even on
-// the grid's last tiles).  Lane 0 / 31 hold the halo words: their outer bits go stale by one
-// cell per generation, which never reaches the output words for up to 31 generations; rows go
-// stale from the region's top/bottom by one row per generation, which never reaches the R
-// output rows for up to `steps` generations.  Both states (t and t-1) are kept: each
-// generation writes the new state in place over the t-1 plane (new(x) reads only old(x) and
-// the current plane), then the planes swap.  The launch reads two planes and writes two planes
+// Up to TB_STEPS generations per launch on a region held in registers.  A CTA of 8 warps owns a region of
+// 32 words x 8R rows (periodic wrap at load time, so it is a consistent periodic window even on the
+// grid's last tiles) and writes the 30 words x (8R - 32) rows in its middle; a warp owns a band of R
+// rows, a lane a column of words, both states of it (t and t-1) in registers.  x neighbours come by
+// shuffle; of a band only the first and last row of a generation go through shared memory, one barrier a
+// generation.  A generation works down the band and leaves the new state over the t-1 state (new(x) reads
+// only old(x) and the current state), then the two change roles.  Lane 0 / 31 hold the halo words: their
+// outer bits go stale by one cell per generation, which never reaches the output words for up to 31
+// generations; rows go stale from the region's top and bottom by one row per generation, which never
+// reaches the output rows for up to TB_STEPS generations.  The launch reads two planes and writes two planes
 // (the next launch needs both), so global traffic per generation drops by ~TB_STEPS/1.5.
 //
-// RAGGED: rows of nw words whose last word holds only v = nx - 32*(nw - 1) cells (the rest of its
+// Bound by the logic pipe: a word costs its 11 lop3 and two funnel shifts and two shuffles, and no address,
+// load or store.  (With the planes in shared memory, two loads and a store per word and generation and
+// their loop: 17.8 logic instructions executed per word where this has 13, and 256-row tiles even on
+// small grids.)
+//
+// Ragged rows: nw words whose last word holds only v = nx - 32*(nw - 1) cells (the rest of its
 // bits 0).  Interior words are loaded as they are; the words past a row's end are put together
 // from the two words that hold their 32 cells after the periodic wrap.  Needs nx >= 64.
 constexpr int TB_STEPS = 16;  // generations per launch (max)
 constexpr int TB_WARPS = 8;
-constexpr int tb_smem(int rows) { return 2 * (rows + 2 * TB_STEPS) * 32 * 4; }
 
 // One lane's words of a region: word `q` of every row, or (general) the 32 cells that start r bits
 // into word q, of which only `cnt` lie before the row's end and the others are the row's first.
@@ -342,75 +347,89 @@ __device__ __forceinline__ RowBits tile_row(uint32_t w)
     return r;
 }
 
-template <int RULE, int ROWS, bool RAGGED>
-__global__ void __launch_bounds__(TB_WARPS * 32) life_bits_tb(const uint32_t* __restrict__ curG, const uint32_t* __restrict__ oldG,
-                                                               uint32_t* __restrict__ outCur, uint32_t* __restrict__ outOld,
-                                                               int nx, int nw, int ny, int tiles_x, int tiles, int steps)
+// One generation of a band: c = state at t, o = state at t-1 and then at t+1; up / dn: the rows around it.
+template <int RULE, int R>
+__device__ __forceinline__ void band_generation(const uint32_t (&c)[R], uint32_t (&o)[R], uint32_t upw, uint32_t dnw)
+{
+    RowBits up = tile_row(upw), mid = tile_row(c[0]);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const RowBits dn = tile_row(r + 1 < R ? c[r + 1 < R ? r + 1 : 0] : dnw);
+        o[r] = life_combine<RULE>(up, mid, dn, o[r]);
+        up = mid;
+        mid = dn;
+    }
+}
+
+template <int RULE, int R, bool RAGGED>
+__global__ void __launch_bounds__(TB_WARPS * 32, 2) life_bits_tb(const uint32_t* __restrict__ curG, const uint32_t* __restrict__ oldG,
+                                                                 uint32_t* __restrict__ outCur, uint32_t* __restrict__ outOld, int nx, int nw,
+                                                                 int ny, int tiles_x, int steps)
 {
     const gb::BlockId bid = gb::grid_wait();
-    constexpr int RRMAX = ROWS + 2 * TB_STEPS;
-    extern __shared__ uint32_t tbsm[];  // two (RRMAX x 32)-word planes
-    uint32_t(*sA)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm);
-    uint32_t(*sB)[32] = reinterpret_cast<uint32_t(*)[32]>(tbsm + RRMAX * 32);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rr = ROWS + 2 * steps;  // rows of the region
-    for (int tile = bid.x; tile < tiles; tile += gridDim.x) {
-        const int tx = tile % tiles_x, ty = tile / tiles_x;
-        int wx = (tx * 30 - 1 + lane) % nw;
-        if (wx < 0) wx += nw;
-        WordSource src;
-        if (RAGGED) src.at(tx * 30 - 1 + lane, nx, nw);
-        const int row0 = ty * ROWS - steps;
-        for (int r = warp; r < rr; r += TB_WARPS) {
-            int gy = (row0 + r) % ny;
-            if (gy < 0) gy += ny;
-            const size_t g = (size_t)gy * nw + wx;
+    constexpr int W = TB_WARPS, RR = R * W, ROWS = RR - 2 * TB_STEPS;  // rows of the region, of the tile
+    __shared__ uint32_t top[2][W][32], bot[2][W][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int ty = (int)(bid.x / (unsigned)tiles_x), tx = (int)bid.x - ty * tiles_x;
+    int wx = (tx * 30 - 1 + lane) % nw;
+    if (wx < 0) wx += nw;
+    WordSource src;
+    if (RAGGED) src.at(tx * 30 - 1 + lane, nx, nw);
+    const int y0 = ty * ROWS - TB_STEPS + R * w;  // the band's first row
+    uint32_t c[R], o[R];
+    {
+        int gy = y0 % ny;
+        if (gy < 0) gy += ny;
+        size_t g = (size_t)gy * nw;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
             if (RAGGED) {
-                sA[r][lane] = src.load(curG + (size_t)gy * nw);
-                sB[r][lane] = RULE == APPFIS_GB_LIFE_REFERENCE ? src.load(oldG + (size_t)gy * nw) : 0u;
+                c[r] = src.load(curG + g);
+                o[r] = RULE == APPFIS_GB_LIFE_REFERENCE ? src.load(oldG + g) : 0u;
             } else {
-                sA[r][lane] = __ldg(curG + g);
-                sB[r][lane] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(oldG + g) : 0u;
+                c[r] = __ldg(curG + g + wx);
+                o[r] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(oldG + g + wx) : 0u;
+            }
+            g += nw;
+            if (++gy == ny) {
+                gy = 0;
+                g = 0;
             }
         }
+    }
+    const int above = w > 0 ? w - 1 : 0, below = w < W - 1 ? w + 1 : W - 1;  // the region's outer rows go stale
+    int t = 0;
+    for (; t + 2 <= steps; t += 2) {
+        top[0][w][lane] = c[0];
+        bot[0][w][lane] = c[R - 1];
         __syncthreads();
-        uint32_t(*cur)[32] = sA;
-        uint32_t(*old)[32] = sB;
-        for (int t = 1; t <= steps; t++) {
-            // rows valid after generation t: [t, rr - t), split evenly over the warps; each warp
-            // marches its chunk carrying the row summaries (one new row summary per output row)
-            const int lo = t, n = rr - 2 * t, chunk = (n + TB_WARPS - 1) / TB_WARPS;
-            const int r0 = lo + warp * chunk, r1 = min(lo + n, r0 + chunk);
-            if (r0 < r1) {
-                RowBits up = tile_row(cur[r0 - 1][lane]);
-                RowBits mid = tile_row(cur[r0][lane]);
-#pragma unroll 8  // 8 rows per trip: the up/mid/dn rotation becomes register renaming
-                for (int r = r0; r < r1; r++) {
-                    const RowBits dn = tile_row(cur[r + 1][lane]);
-                    const uint32_t o = RULE == APPFIS_GB_LIFE_REFERENCE ? old[r][lane] : 0u;
-                    old[r][lane] = life_combine<RULE>(up, mid, dn, o);
-                    up = mid;
-                    mid = dn;
-                }
-            }
-            __syncthreads();
-            uint32_t(*tmp)[32] = cur;
-            cur = old;
-            old = tmp;
-        }
-        const int wout = tx * 30 - 1 + lane;
-        const uint32_t keep = RAGGED && wout == nw - 1 && (nx & 31) ? (1u << (nx & 31)) - 1u : FULL;
-        if (lane >= 1 && lane <= 30 && wout < nw) {
-            for (int r = steps + warp; r < steps + ROWS; r += TB_WARPS) {
-                const int gy = ty * ROWS + (r - steps);
-                if (gy < ny) {
-                    const size_t g = (size_t)gy * nw + wout;
-                    outCur[g] = RAGGED ? cur[r][lane] & keep : cur[r][lane];
-                    outOld[g] = RAGGED ? old[r][lane] & keep : old[r][lane];
-                }
-            }
-        }
+        band_generation<RULE, R>(c, o, bot[0][above][lane], top[0][below][lane]);
+        top[1][w][lane] = o[0];
+        bot[1][w][lane] = o[R - 1];
         __syncthreads();
+        band_generation<RULE, R>(o, c, bot[1][above][lane], top[1][below][lane]);
+    }
+    const bool odd = t < steps;
+    if (odd) {
+        top[0][w][lane] = c[0];
+        bot[0][w][lane] = c[R - 1];
+        __syncthreads();
+        band_generation<RULE, R>(c, o, bot[0][above][lane], top[0][below][lane]);
+    }
+    // the newest state is in o after an odd number of generations
+    uint32_t* __restrict__ outC = odd ? outOld : outCur;
+    uint32_t* __restrict__ outO = odd ? outCur : outOld;
+    const int wout = tx * 30 - 1 + lane;
+    const uint32_t keep = RAGGED && wout == nw - 1 ? (1u << (nx & 31)) - 1u : FULL;
+    if (lane < 1 || lane > 30 || wout >= nw) return;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int y = R * w + r;
+        if (y >= TB_STEPS && y < RR - TB_STEPS && y0 + r < ny) {
+            const size_t g = (size_t)(y0 + r) * nw + wout;
+            outC[g] = RAGGED ? c[r] & keep : c[r];
+            outO[g] = RAGGED ? o[r] & keep : o[r];
+        }
     }
 }
 
@@ -614,56 +633,65 @@ struct TbPair {
     uint32_t* p[2];  // state at t, state at t-1
 };
 
-template <int RULE, int ROWS, bool RAGGED>
-int launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+#define LIFE_BANDS(F) F(8) F(10) F(12) F(14) F(16) F(18) F(20) F(22) F(24) F(28) F(32) F(36) F(40) F(45)
+
+// Rows per band: the height whose tiles, dealt to the SMs, take the least time; the fullest SM's tiles follow
+// one another on its logic pipe, 0.49 us per band row (and 0.2) for 16 generations, whatever is resident
+// together.  Tall bands compute less halo (45 rows: 10%, 8: half), but a small grid needs many.  Measured, us
+// per 64 generations with 8 / 16 / 24 / 32 / 40 / 45 rows: 1024 x 1000 22 / 37 / 53 / 70 / 86 / 97; 2048^2 38 / 38 / 53 /
+// 70 / 87 / 98; 4096^2 86 / 67 / 54 / 71 / 87 / 98; 8192^2 262 / 192 / 191 / 193 / 163 / 184; 16384^2 985 / 665 / 613 / 573 /
+// 555 / 541.  (Planes in shared memory, tiles of 32 to 256 rows: 49, 66, 107, 211, 706.)
+int tb_band(int nw, int ny)
 {
-    const int tiles_x = (nw + 29) / 30, tiles = tiles_x * ((ny + ROWS - 1) / ROWS);
-    constexpr int smem = tb_smem(ROWS);
-    auto kern = life_bits_tb<RULE, ROWS, RAGGED>;
-    if (smem > 48 * 1024) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TB_WARPS * 32, smem) != cudaSuccess || per_sm < 1) per_sm = 3;
-    const int grid = std::max(1, std::min(tiles, per_sm * gb::sm_count()));
-    gb::launch(kern, grid, TB_WARPS * 32, smem, st, in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, tiles, steps);
-    return APPFIS_GB_OK;
+    const long long tiles_x = (nw + 29) / 30, sms = gb::sm_count();
+    int best = 8;
+    double cost = 1e30;
+#define LIFE_COST(R)                                                                                        \
+    {                                                                                                       \
+        const long long tiles = tiles_x * ((ny + 8 * R - 2 * TB_STEPS - 1) / (8 * R - 2 * TB_STEPS));       \
+        const double c = (double)((tiles + sms - 1) / sms) * (0.49 * R + 0.2);                              \
+        if (c <= cost) {                                                                                    \
+            cost = c;                                                                                       \
+            best = R;                                                                                       \
+        }                                                                                                   \
+    }
+    LIFE_BANDS(LIFE_COST)
+#undef LIFE_COST
+    return best;
 }
 
-// Output rows per tile: the most whose tiles still number 1.5 per SM.  Tall tiles recompute less halo
-// (256 rows: 9% at 16 generations, 32 rows: 50%) but a warp marches rows / 8 of them one after another, and
-// a small grid has too few to go round.  Measured, us per 64 generations with 256 / 128 / 64 / 32
-// rows: 1024 x 1000 172 / 98 / 66 / 49; 2048^2 172 / 98 / 66 / 66; 4096^2 172 / 123 / 107 / 123;
-// 512 x 16384 164 / 98 / 82 / 98; 8192^2 211 / 213 / 238 / 337; 16384^2 706 / 811 / 935 / 1279.
-int tb_rows(int nw, int ny)
+template <int RULE, int R>
+void launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
 {
+    static_assert(TB_WARPS == 8, "bands of 8 warps");
     const int tiles_x = (nw + 29) / 30;
-    for (int rows : {256, 128, 64})
-        if ((long long)tiles_x * ((ny + rows - 1) / rows) * 2 >= 3LL * gb::sm_count()) return rows;
-    return 32;
+    const unsigned tiles = (unsigned)tiles_x * gb::ceil_div(ny, R * TB_WARPS - 2 * TB_STEPS);
+    gb::launch(nx % 32 ? life_bits_tb<RULE, R, true> : life_bits_tb<RULE, R, false>, tiles, TB_WARPS * 32, 0, st, in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, steps);
 }
 
-template <int RULE, bool RAGGED>
-int tb_step(int rows, TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+template <int RULE>
+void tb_step(int band, TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
 {
-    switch (rows) {
-    case 256: return launch_tb<RULE, 256, RAGGED>(in, out, nx, nw, ny, steps, st);
-    case 128: return launch_tb<RULE, 128, RAGGED>(in, out, nx, nw, ny, steps, st);
-    case 64: return launch_tb<RULE, 64, RAGGED>(in, out, nx, nw, ny, steps, st);
-    default: return launch_tb<RULE, 32, RAGGED>(in, out, nx, nw, ny, steps, st);
+    switch (band) {
+#define LIFE_CASE(R) \
+    case R: return launch_tb<RULE, R>(in, out, nx, nw, ny, steps, st);
+        LIFE_BANDS(LIFE_CASE)
+#undef LIFE_CASE
     }
 }
 
 // `gens` generations in `launches` launches of nearly equal length, from pair[0] and back into
 // `last`; a launch cannot write the pair it reads (its tiles read their neighbours' halo rows).
 // An odd number of launches goes round three pairs once, so it needs pair[2].
-template <int RULE, bool RAGGED>
+template <int RULE>
 int run_tb(const TbPair (&pair)[3], TbPair last, int nx, int ny, int gens, int launches, cudaStream_t st)
 {
-    const int nw = (nx + 31) / 32, rows = tb_rows(nw, ny);
+    const int nw = (nx + 31) / 32, band = tb_band(nw, ny);
     int at = 0, done = 0;
     for (int n = 0; n < launches; n++) {
         const int next = (pair[2].p[0] && n < 3) ? (n + 1) % 3 : 1 - at;
         const int upto = (int)((long long)gens * (n + 1) / launches);
-        GB_TRY((tb_step<RULE, RAGGED>(rows, pair[at], n + 1 == launches ? last : pair[next], nx, nw, ny, upto - done, st)));
+        tb_step<RULE>(band, pair[at], n + 1 == launches ? last : pair[next], nx, nw, ny, upto - done, st);
         done = upto;
         at = next;
     }
@@ -679,13 +707,13 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
     // 18.4 us of one CTA's march, which the one-thread-per-cell form takes there too (701 x 700: 5.4)
     const bool bulk = nx % 16 == 0 && cells >= ((size_t)1 << 22);
     // Packed: bytes to words, the time-blocked kernel, words to bytes.  The conversions and launches cost
-    // 14 us and 1.1-1.5 us per M cells, a generation next to nothing; a sweep costs 3.4 us (0.1 M cells),
-    // 18 (4 M, either form), 60 / 23 (17 M, one thread per cell / bulk), 244 / 35-47 (67 M).  So packed
-    // wins from 4 generations on, sooner where one thread per cell is slow, and from 3 on over the
-    // bulk form.  Us for 20 generations, sweeps -> packed: 301 x 300 82 -> 33, 2050 x 1999 366 -> 43,
-    // 8192^2 697 -> 131, 8200 x 8192 4878 -> 186.
-    const bool packed = bulk ? gens >= 3 : gens >= 4 || (size_t)gens * cells >= ((size_t)1 << 23);
-    if (nx >= 64 && packed && !gb::capturing(st)) {
+    // 7-9 us and 0.8-1.6 us per M cells, a generation next to nothing; a sweep costs 3.0 us (0.1 M cells),
+    // 4.6 (1 M), 14 (4 M, either form), 60 / 19 (17 M, one thread per cell / bulk), 244 / 30-47 (67 M).
+    // Us for 20 generations, sweeps -> packed: 301 x 300 82 -> 17, 2050 x 1999 366 -> 26, 8192^2 697 -> 105,
+    // 8200 x 8192 4878 -> 150.
+    const bool packed = bulk ? gens >= 2 || cells < ((size_t)1 << 23)
+                             : gens >= 4 || (gens >= 2 && (size_t)gens * cells >= 3000000) || cells >= 6000000;
+    if (nx >= 64 && gens > 0 && packed && !gb::capturing(st)) {
         const int nw = (nx + 31) / 32;
         const size_t words = (size_t)nw * ny, plane = (words + 63) / 64 * 64;
         void* ws = nullptr;
@@ -700,11 +728,11 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
             int rc;
             if (nx % 32) {
                 gb::launch(life_pack_rows, wgrid, 256, 0, st, buf[0], buf[1], w, w + plane, nx, nw, words, cells);
-                rc = run_tb<RULE, true>(pair, last, nx, ny, gens, launches, st);
+                rc = run_tb<RULE>(pair, last, nx, ny, gens, launches, st);
                 gb::launch(life_unpack_rows, dim3(gb::ceil_div(cells + 15, 4096), 2), 256, 0, st, last.p[0], last.p[1], buf[ci], buf[1 - ci], nx, nw, cells);
             } else {
                 gb::launch(life_pack, wgrid, 256, 0, st, buf[0], buf[1], w, w + plane, words);
-                rc = run_tb<RULE, false>(pair, last, nx, ny, gens, launches, st);
+                rc = run_tb<RULE>(pair, last, nx, ny, gens, launches, st);
                 gb::launch(life_unpack, dim3(wgrid.x, 2), 256, 0, st, last.p[0], last.p[1], buf[ci], buf[1 - ci], words);
             }
             gb::scratch_free(ws, st);
@@ -736,11 +764,10 @@ int run_u8(uint8_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream
     return APPFIS_GB_OK;
 }
 
-// Bit-packed run.  Four or more generations take the time-blocked kernel, at least two launches so that
-// the state comes back into (a, b): 2 / 4 / 8 generations as sweeps against tiles, us: 1024 x 1000 8.2 / 16.4 /
-// 32.8 against 10.8 / 12.3 / 14.3; 4096^2 12.3 / 24.6 / 49.2 against 14.7 / 17.0 / 22.6; 16384^2 61 / 123 / 246
-// against 89 / 102 / 131.  The newest state is in a after an even number of generations, else in b,
-// as it is when every generation is a sweep.
+// Bit-packed run.  Three or more generations take the time-blocked kernel, at least two launches so that
+// the state comes back into (a, b): as sweeps / tiles, us: 1024 x 1000 4 generations 9.3 / 5.7; 4096^2 3
+// 10.7 / 9.8, 8 28 / 12.8; 16384^2 3 84 / 75, 8 226 / 113.  The newest state is in a after an even number of
+// generations, else in b, as it is when every generation is a sweep.
 template <int RULE>
 int run_bits(uint32_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStream_t st)
 {
@@ -762,12 +789,12 @@ int run_bits(uint32_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStr
             GB_TRY(gb::workspace(gb::WS_LIFE_F, bytes, &wf));
         }
         const TbPair pair[3] = {own, {{(uint32_t*)wc, (uint32_t*)wd}}, {{(uint32_t*)we, (uint32_t*)wf}}};
-        return run_tb<RULE, false>(pair, last, nx, ny, gens, launches, st);
+        return run_tb<RULE>(pair, last, nx, ny, gens, launches, st);
     }
     void* ws = nullptr;
-    if (gens >= 4 && !gb::capturing(st) && gb::scratch_alloc(2 * bytes, st, &ws)) {
+    if (gens >= 3 && !gb::capturing(st) && gb::scratch_alloc(2 * bytes, st, &ws)) {
         const TbPair pair[3] = {own, {{(uint32_t*)ws, (uint32_t*)ws + plane}}, {{nullptr, nullptr}}};
-        const int rc = run_tb<RULE, false>(pair, last, nx, ny, gens, 2, st);
+        const int rc = run_tb<RULE>(pair, last, nx, ny, gens, 2, st);
         gb::scratch_free(ws, st);
         return rc;
     }
