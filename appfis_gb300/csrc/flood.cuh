@@ -48,6 +48,7 @@ struct Ctl {
     int error;
     unsigned ticket[2];  // phase A strip hand-out, by step parity
     unsigned ticketb[2];  // phase B strip hand-out, by step parity
+    unsigned wet[2], dry[2];  // strips listed for the next step of that parity (Params::order)
 };
 
 struct Params {
@@ -58,6 +59,8 @@ struct Params {
     long long total_strips;
     double* dtlog;  // [ndom][max_steps] or null
     unsigned char* zc;  // [2][total_strips] dry-step counters (null: every strip every step)
+    unsigned* order;    // [2][total_strips] the strips in the order that steps of each parity take them (null: as numbered)
+    int spread;         // warps' first places go round the CTAs (else: eight in a row to each)
     unsigned long long spin_limit;  // polls before a grid-barrier wait gives up
     int stall_cta;                  // testing: this CTA skips its arrival at the first barrier (-1: none)
     const SrcDev* srcs;             // [ndom] point sources, or null (no source phase)
@@ -366,21 +369,48 @@ struct DomCtl {
     unsigned char flags[MAXD];  // bit 0: state buffer b, bit 1: fix, bit 2: wants dt / runs phase B
 };
 
-// Strips of one phase: warp w first takes strip w, then strips nwarps + k for the tickets k it
-// draws from *ctr (zeroed after the phase's grid barrier, for its next use two steps later).
-// The next ticket is requested before the current strip is processed, so its latency hides
-// behind the work.  Warps without a first strip draw none (a batch smaller than the grid costs
-// no atomics).
-template <class F>
-__device__ __forceinline__ void for_strips(unsigned* ctr, long long first, long long nwarps, long long total, int lane, F&& body)
+// The order of step n (the first step has none listed: as numbered).
+__device__ __forceinline__ const unsigned* step_order(const Params& p, int n)
 {
-    long long s = first;
+    return p.order && n > 0 ? p.order + (size_t)(n & 1) * p.total_strips : nullptr;
+}
+
+// Strips of one phase: warp w first takes the strip in place w, then those in places nwarps + k for the
+// tickets k it draws from *ctr (zeroed after the phase's grid barrier, for its next use two steps later).
+// The strip after next's ticket and the next strip's number are requested before the current strip is
+// processed, so their latency hides behind the work.  Warps without a first strip draw none (a batch
+// smaller than the grid costs no atomics).
+template <class F>
+__device__ __forceinline__ void for_strips(unsigned* ctr, const unsigned* order, long long first, long long nwarps, long long total, int lane, F&& body)
+{
+    if (first >= total) return;
+    unsigned s = order ? __ldcg(order + first) : (unsigned)first;
     unsigned tk = 0;
-    if (s < total && lane == 0) tk = atomicAdd(ctr, 1u);
-    while (s < total) {
-        body(s);
-        s = nwarps + (long long)__shfl_sync(0xffffffffu, tk, 0);
-        if (s < total && lane == 0) tk = atomicAdd(ctr, 1u);
+    if (lane == 0) tk = atomicAdd(ctr, 1u);
+    long long at = nwarps + (long long)__shfl_sync(0xffffffffu, tk, 0);
+    for (;;) {
+        const bool more = at < total;  // uniform in the warp
+        unsigned sn = 0;
+        if (more) {
+            sn = order ? __ldcg(order + at) : (unsigned)at;
+            if (lane == 0) tk = atomicAdd(ctr, 1u);
+        }
+        body((long long)s);
+        if (!more) return;
+        s = sn;
+        at = nwarps + (long long)__shfl_sync(0xffffffffu, tk, 0);
+    }
+}
+
+// Lists strip s for the step of parity `next`: wet ones from the front, dry ones from the back.  A step lasts
+// as long as its slowest warp, and a wet strip takes several times a dry one's time: with the wet ones
+// taken first, the dry ones fill the gaps at the end (wet_first() has the figures).  Only the
+// order depends on it: the strips of a phase are independent.
+__device__ __forceinline__ void list_strip(Ctl* ctl, const Params& p, int next, long long s, bool dry, int lane)
+{
+    if (p.order && lane == 0) {
+        const unsigned at = dry ? (unsigned)p.total_strips - 1u - atomicAdd(&ctl->dry[next], 1u) : atomicAdd(&ctl->wet[next], 1u);
+        p.order[(size_t)next * p.total_strips + at] = (unsigned)s;
     }
 }
 
@@ -439,7 +469,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     __shared__ DomCtl<T> dc;
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
     __syncthreads();
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long warp = p.spread ? (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     const double big = (double)K<T>::big();
@@ -454,7 +484,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (fix ? 2 : 0) | (want ? 4 : 0));
         }
         __syncthreads();
-        for_strips(&ctl->ticket[cur], warp, nwarps, p.total_strips, lane, [&](long long s) {
+        const unsigned* order = step_order(p, n);
+        for_strips(&ctl->ticket[cur], order, warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
             const int f = dc.flags[d];
             if (SKIP && p.zc[(size_t)cur * p.total_strips + s] >= 1) return;  // dry input: no fix, no dt
@@ -474,25 +505,30 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
         }
         if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
         // phase B
-        for_strips(&ctl->ticketb[cur], warp, nwarps, p.total_strips, lane, [&](long long s) {
+        for_strips(&ctl->ticketb[cur], order, warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
             const int f = dc.flags[d];
+            bool dry = true;
             if (SKIP) {
                 const unsigned char* zin = p.zc + (size_t)cur * p.total_strips;
                 unsigned char* zout = p.zc + (size_t)(1 - cur) * p.total_strips;
                 const unsigned char z = zin[s];
                 if (!(f & 4) || strip_idle(doms[d], zin, s, p.rows)) {  // unchanged state
                     if (lane == 0) zout[s] = z;
-                    return;
+                } else {
+                    dry = phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
+                    if (lane == 0) zout[s] = dry ? (unsigned char)(z < 2 ? z + 1 : 2) : 0;
                 }
-                const bool dry = phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
-                if (lane == 0) zout[s] = dry ? (unsigned char)(z < 2 ? z + 1 : 2) : 0;
             } else if (f & 4) {
-                phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
+                dry = phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
             }
+            list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
         if (!grid_barrier(ctl, p.spin_limit)) return;
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ticketb[cur] = 0;  // next used two steps later, past a barrier
+        if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
+            ctl->ticketb[cur] = 0;
+            ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
+        }
         if (p.srcs) {  // the point sources of step n, seen by the next step's wet/dry fix and dt
             if (blockIdx.x == 0 && threadIdx.x < p.ndom)
                 apply_sources<T>(doms[threadIdx.x], p.srcs[threadIdx.x], ctl, cur, threadIdx.x, p, big);
@@ -781,14 +817,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     }
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
     __syncthreads();
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long warp = p.spread ? (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     const double big = (double)K<T>::big();
     // dt of step 0 from the initial state (no fix before the first step)
     if (threadIdx.x < p.ndom) dc.flags[threadIdx.x] = is_active(ctl, 0, threadIdx.x, p) ? 4 : 0;
     __syncthreads();
-    for_strips(&ctl->ticket[0], warp, nwarps, p.total_strips, lane, [&](long long s) {
+    for_strips(&ctl->ticket[0], nullptr, warp, nwarps, p.total_strips, lane, [&](long long s) {
         const int d = find_domain(doms, p.ndom, s);
         if (dc.flags[d] & 4) phase_a<T, FCOLS, 2>(doms[d], ctl, 0, d, s - doms[d].strip0, ctl->steps[0][d] & 1, false, true, p);
     });
@@ -808,26 +844,30 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
         }
         if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
         const int dn = (n + 1) % 3;
-        for_strips(&ctl->ticketb[cur], warp, nwarps, p.total_strips, lane, [&](long long s) {
+        for_strips(&ctl->ticketb[cur], step_order(p, n), warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
             const int f = dc.flags[d];
+            bool dry = true;
             if (SKIP) {  // the two-phase kernel's dry-strip rule (strip_idle), on this kernel's strips
                 const unsigned char* zin = p.zc + (size_t)cur * p.total_strips;
                 unsigned char* zout = p.zc + (size_t)(1 - cur) * p.total_strips;
                 const unsigned char z = zin[s];
                 if (!(f & 4) || strip_idle(doms[d], zin, s, p.rows)) {  // unchanged state, no fix, no dt
                     if (lane == 0) zout[s] = z;
-                    return;
+                } else {
+                    dry = phase_bf<T, STAGED, false>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p, &ctl->dtbits[dn][d], &ring, d, ctl);
+                    if (lane == 0) zout[s] = dry ? (unsigned char)(z < 2 ? z + 1 : 2) : 0;
                 }
-                const bool dry = phase_bf<T, STAGED, false>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p,
-                                                            &ctl->dtbits[dn][d], &ring, d, ctl);
-                if (lane == 0) zout[s] = dry ? (unsigned char)(z < 2 ? z + 1 : 2) : 0;
             } else if (f & 4) {
-                phase_bf<T, STAGED>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p, &ctl->dtbits[dn][d], &ring, d, ctl);
+                dry = phase_bf<T, STAGED>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p, &ctl->dtbits[dn][d], &ring, d, ctl);
             }
+            list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
         if (!grid_barrier(ctl, p.spin_limit)) return;
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ticketb[cur] = 0;  // next used two steps later, past a barrier
+        if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
+            ctl->ticketb[cur] = 0;
+            ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
+        }
     }
 }
 
@@ -841,6 +881,7 @@ static __global__ void flood_init_ctl(Ctl* ctl, int ndom, double big, double t0)
         ctl->error = 0;
         ctl->ticket[0] = ctl->ticket[1] = 0;
         ctl->ticketb[0] = ctl->ticketb[1] = 0;
+        ctl->wet[0] = ctl->wet[1] = ctl->dry[0] = ctl->dry[1] = 0;
     }
     if (d < ndom) {
         ctl->src_lo[d] = 0;

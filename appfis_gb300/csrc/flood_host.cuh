@@ -173,15 +173,16 @@ inline int upload_sources(const appfis_gb_flood_domain* doms, const appfis_gb_fl
 // than the chip has warps.  Us per step with 32 / 16 / 8 / 4 / 2 rows:
 //   FP32 fused: 100^2 50 / 30 / 19 / 14 / 11; 300 x 1100 55 / 32 / 21 / 17 / 21; 1024^2 55 / 34 / 30 / 31 / 32;
 //     six domains of 3.6 M cells 101 / 73 / 63 / 64 / 88; 2 x 3000^2 180 / 174 / 187 / 241; 32 domains of 80 M cells 671 / 708 / 828 / 1085
-//   FP64: 100^2 1442 / 778 / 412 / 223 / 127; 1024^2 2377 / 1621 / 653 / 476 / 347; six 3090 / 1691 / 1141 / 1014 / 1025;
-//     2 x 3000^2 4224 / 3411 / 3214 / 3282 / 3874; 32 domains 14.87 / 14.23 / 14.34 / 15.40 / 18.13 ms
+//   FP64, wet strips first from two strips a warp: 100^2 1442 / 778 / 412 / 223 / 119; 300 x 1100 1410 / 756 / 411 / 245 / 155;
+//     1024^2 1446 / 785 / 454 / 295 / 289; six 1711 / 999 / 807 / 847 / 965; 2048^2 1684 / 1024 / 802 / 868 / 980;
+//     2 x 3000^2 2981 / 3155 / 3145 / 3429 / 4074; 32 domains (as numbered) 14.87 / 14.23 / 14.34 / 15.40 / 18.13 ms
 // FP64 asks for more strips per warp: it has a third of the warps, and each is bound by the FP64 pipe.
 template <class T>
 int strip_rows(const appfis_gb_flood_domain* doms, int ndom, int scols, long long warps)
 {
     constexpr bool f32 = std::is_same<T, float>::value;
     const int rows[4] = {32, 16, 8, 4};
-    const double per_warp[4] = {f32 ? 8.0 : 512.0, f32 ? 8.0 : 64.0, f32 ? 4.0 : 48.0, f32 ? 0.8 : 24.0};
+    const double per_warp[4] = {f32 ? 8.0 : 512.0, f32 ? 8.0 : 64.0, f32 ? 4.0 : 10.0, f32 ? 0.8 : 10.0};
     for (int k = 0; k < 4; k++) {
         long long strips = 0;
         for (int d = 0; d < ndom; d++)
@@ -189,6 +190,20 @@ int strip_rows(const appfis_gb_flood_domain* doms, int ndom, int scols, long lon
         if ((double)strips >= per_warp[k] * (double)warps) return rows[k];
     }
     return 2;
+}
+
+// Whether a batch takes its wet strips first.  As numbered / wet strips first, us per step, full sweep
+// and with dry strips left out:
+//   FP32 700^2 (1.3 strips a warp) 22.3 / 22.7, 16.1 / 17.4; 1024^2 (2.6) 34.3 / 30.7, 28.2 / 23.5; six domains of 3.6 M cells (4.5)
+//     67.0 / 56.6, 49.8 / 36.5; 2 x 3000^2 (11) 189 / 262, 92.7 / 72.3; 32 domains (25) 873 / 1180, 243 / 240
+//   FP64 300^2 (1.2) 133 / 133, 126 / 125; 300 x 1100 (4.6) 292 / 155, 267 / 129; 1024^2 (15) 428 / 290, 382 / 202; six (13, 8 rows)
+//     1174 / 807, 1029 / 606; 2 x 3000^2 (62) 3514 / 3145, 2443 / 2167
+// Below two strips a warp all start at once.  A full FP32 sweep with many strips a warp is bound by
+// memory: its dry strips' traffic then runs beside the wet strips' arithmetic, and neighbours share lines.
+template <class T>
+bool wet_first(long long strips, int rows, long long warps, bool skip)
+{
+    return strips >= 2 * warps && (sizeof(T) == 8 || skip || rows < 16);
 }
 
 // Uploads the table, initialises the control block and launches the persistent kernel.
@@ -232,7 +247,8 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     if (staged) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
     if (per_sm < 1) return gb::fail(APPFIS_GB_ECUDA, "flood: kernel cannot be resident");
-    const int rows = strip_rows<T>(doms, ndom, scols, 8LL * per_sm * gb::sm_count());
+    const long long warps = 8LL * per_sm * gb::sm_count();
+    const int rows = strip_rows<T>(doms, ndom, scols, warps);
     GB_TRY(make_table<T>(doms, ndom, tab, total, scols, rows));
     void *wt, *hs;
     GB_TRY(gb::workspace(gb::WS_REDUCE, sizeof(Ctl) + sizeof(Dom<T>) * MAXD + 256, &wt));
@@ -262,6 +278,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     p.total_strips = total;
     p.dtlog = prm->max_steps > 0 ? dev_dtlog : nullptr;
     p.zc = nullptr;
+    p.order = nullptr;
     p.spin_limit = SPIN_LIMIT;
     p.stall_cta = -1;
     p.maps = nullptr;
@@ -300,6 +317,13 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
         p.zc = reinterpret_cast<unsigned char*>(z);
     }
 
+    void* listed;  // without room for the lists: as numbered
+    if (wet_first<T>(total, rows, warps, skip) &&
+        gb::workspace(gb::WS_FLOOD_ORDER, 2 * sizeof(unsigned) * (size_t)total, &listed) == APPFIS_GB_OK)
+        p.order = reinterpret_cast<unsigned*>(listed);
+    // round the CTAs: strips in a row are wet together, and an SM's warps share its FP64 pipe (FP64 100^2 128 -> 122 us per
+    // step; 300 x 1100 wet first 232 -> 155); FP32 as numbered 300^2 11.6 against 12.9
+    p.spread = p.order || sizeof(T) == 8;
     long long want = (total * 32 + 255) / 256;  // one warp per strip at most
     int grid = (int)std::min<long long>(want, (long long)per_sm * gb::sm_count());
     if (grid < 1) grid = 1;
