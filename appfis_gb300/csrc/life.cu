@@ -185,11 +185,13 @@ struct RowBits {
 //   reference rule (S234 with the stale carry): a live cell keeps o when S is 3, 4 or 5 and dies
 //     otherwise; a dead cell is born when S is 3 and otherwise keeps o;
 //   B3/S23: a live cell survives when S is 3 or 4; a dead cell is born when S is 3.
-// Only S mod 8 is formed (S0..S2): S = 8 and 9 read as 0 and 1, which neither rule distinguishes
-// from the true values (no birth, no survival either way).  Every step is one explicit 3-input
-// logic instruction (lop3): 6 for the count (two full adders and the half adder folded into
-// s2 = y ^ (x & c1)), 3 for the reference rule (the window S in 3..5, narrowed to S == 3 for a
-// dead cell, then the keep/birth select with the stale value) and 2 for B3/S23.
+// Every step is one explicit 3-input logic instruction (lop3).  The reference rule takes 8: 4 for the count,
+// S = s0 + 2 (c1 + x + 2 y), 3 for the rule and 1 for the keep / birth select with the stale value; B3/S23 takes 6 in
+// all.  S in binary is not formed: the tables are what an exhaustive search over networks of such
+// instructions gave for the rule at every S that a cell can have (a live cell counts itself, so a live
+// cell's S is never 0 and a dead one's never 9); it has no shorter one for the reference rule with s0 and c1.
+// With S's bits and a window on them it was one more and two more: 16384^2, 64 generations 541 against 518 us
+// (reference rule); B3/S23 455 with 7, 411 with 6.
 // One 3-input logic instruction; LUT = f(0xF0, 0xCC, 0xAA) for the function f(a, b, c).
 template <unsigned LUT>
 __device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c)
@@ -204,19 +206,21 @@ template <int RULE>
 __device__ __forceinline__ uint32_t life_combine(const RowBits& up, const RowBits& mid, const RowBits& dn, uint32_t o)
 {
     const uint32_t s0 = lop3<XOR3>(up.a0, mid.a0, dn.a0);
-    const uint32_t c1 = lop3<MAJ3>(up.a0, mid.a0, dn.a0);
-    const uint32_t x = lop3<XOR3>(up.a1, mid.a1, dn.a1);
-    const uint32_t y = lop3<MAJ3>(up.a1, mid.a1, dn.a1);
-    const uint32_t s1 = x ^ c1;
-    const uint32_t s2 = lop3<0x78>(y, x, c1);  // y ^ (x & c1)
     const uint32_t c = mid.w;
     if (RULE == APPFIS_GB_LIFE_REFERENCE) {
-        const uint32_t in345 = lop3<0x38>(s2, s1, s0);  // S in 3..5: (~s2 & s1 & s0) | (s2 & ~s1)
-        const uint32_t d = lop3<0xD0>(in345, c, s2);    // live: S in 3..5; dead: S == 3
-        return lop3<0x8E>(c, o, d);                      // c ? o & d : o | d
+        const uint32_t c1 = lop3<MAJ3>(up.a0, mid.a0, dn.a0);
+        const uint32_t x = lop3<XOR3>(up.a1, mid.a1, dn.a1);
+        const uint32_t y = lop3<MAJ3>(up.a1, mid.a1, dn.a1);
+        const uint32_t p = lop3<0x17>(s0, c1, x);  // not the majority
+        const uint32_t q = lop3<0x42>(c1, x, c);   // c1 == x, and c the other way
+        const uint32_t d = lop3<0x81>(y, p, q);    // all equal: live: S in 3..5; dead: S == 3
+        return lop3<0x8E>(c, o, d);                // c ? o & d : o | d
     } else {
-        const uint32_t in34 = lop3<0x18>(s2, s1, s0);   // S in 3..4
-        return lop3<0xD0>(in34, c, s2);                  // live: S in 3..4; dead: S == 3
+        const uint32_t e = lop3<0x7E>(up.a0, mid.a0, dn.a0);  // one or two
+        const uint32_t p = lop3<0x17>(s0, up.a1, dn.a1);
+        const uint32_t q = lop3<0x61>(e, up.a1, dn.a1);
+        const uint32_t r = lop3<0x4A>(mid.a1, p, q);
+        return lop3<0xE0>(r, s0, c);  // r & (s0 | c): live: S in 3..4; dead: S == 3
     }
 }
 struct RawBits {
@@ -298,10 +302,10 @@ __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restric
 // reaches the output rows for up to TB_STEPS generations.  The launch reads two planes and writes two planes
 // (the next launch needs both), so global traffic per generation drops by ~TB_STEPS/1.5.
 //
-// Bound by the logic pipe: a word costs its 11 lop3 and two funnel shifts and two shuffles, and no address,
-// load or store.  (With the planes in shared memory, two loads and a store per word and generation and
-// their loop: 17.8 logic instructions executed per word where this has 13, and 256-row tiles even on
-// small grids.)
+// Bound by the logic pipe (86% of its issue slots; 13.0 instructions executed per word and generation): a
+// word costs its 10 lop3 (B3/S23: 8) and two funnel shifts and two shuffles, and no address, load or
+// store.  (With the planes in shared memory, two loads and a store per word and generation and their
+// loop: 17.8 there for 11 lop3, and 256-row tiles even on small grids.)
 //
 // Ragged rows: nw words whose last word holds only v = nx - 32*(nw - 1) cells (the rest of its
 // bits 0).  Interior words are loaded as they are; the words past a row's end are put together
@@ -380,21 +384,19 @@ __global__ void __launch_bounds__(TB_WARPS * 32, 2) life_bits_tb(const uint32_t*
     {
         int gy = y0 % ny;
         if (gy < 0) gy += ny;
-        size_t g = (size_t)gy * nw;
+        const size_t plane = (size_t)ny * nw;
+        const uint32_t* pc = curG + (size_t)gy * nw + (RAGGED ? 0 : wx);
+        const ptrdiff_t old = oldG - curG;
+        int wrap = ny - gy;  // the band's row at which the grid begins again
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            if (RAGGED) {
-                c[r] = src.load(curG + g);
-                o[r] = RULE == APPFIS_GB_LIFE_REFERENCE ? src.load(oldG + g) : 0u;
-            } else {
-                c[r] = __ldg(curG + g + wx);
-                o[r] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(oldG + g + wx) : 0u;
+            if (r == wrap) {
+                pc -= plane;
+                wrap += ny;
             }
-            g += nw;
-            if (++gy == ny) {
-                gy = 0;
-                g = 0;
-            }
+            c[r] = RAGGED ? src.load(pc) : __ldg(pc);
+            o[r] = RULE != APPFIS_GB_LIFE_REFERENCE ? 0u : RAGGED ? src.load(pc + old) : __ldg(pc + old);
+            pc += nw;
         }
     }
     const int above = w > 0 ? w - 1 : 0, below = w < W - 1 ? w + 1 : W - 1;  // the region's outer rows go stale
@@ -422,14 +424,17 @@ __global__ void __launch_bounds__(TB_WARPS * 32, 2) life_bits_tb(const uint32_t*
     const int wout = tx * 30 - 1 + lane;
     const uint32_t keep = RAGGED && wout == nw - 1 ? (1u << (nx & 31)) - 1u : FULL;
     if (lane < 1 || lane > 30 || wout >= nw) return;
+    const int first = TB_STEPS - R * w, end = min(RR - TB_STEPS - R * w, ny - y0);  // the band's rows to be written
+    uint32_t* pc = outC + (ptrdiff_t)y0 * nw + wout;
+    uint32_t* po = outO + (ptrdiff_t)y0 * nw + wout;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        const int y = R * w + r;
-        if (y >= TB_STEPS && y < RR - TB_STEPS && y0 + r < ny) {
-            const size_t g = (size_t)(y0 + r) * nw + wout;
-            outC[g] = RAGGED ? c[r] & keep : c[r];
-            outO[g] = RAGGED ? o[r] & keep : o[r];
+        if (r >= first && r < end) {
+            *pc = RAGGED ? c[r] & keep : c[r];
+            *po = RAGGED ? o[r] & keep : o[r];
         }
+        pc += nw;
+        po += nw;
     }
 }
 

@@ -457,13 +457,12 @@ def run_ours(args, rank, world, local):
     replay_tb = graph_of(torch, tb_launches)
     bits_ms = _time(torch, stream, replay_tb, reps=4, warmup=2) / TB_LAUNCHES  # per launch
     # its bound is the integer/logic pipe, not HBM: per word (32 cells) and generation the source
-    # issues 11 lop3 on that pipe (2 for the row summary, 6 for the bit-sliced count, 3 for the
-    # reference rule); its 2 funnel shifts run on the FMA pipe (ncu pipe counters: replacing them
-    # by integer multiply-adds left the logic pipe's instruction count unchanged).  The logic pipe
-    # retires 64 lanes per SM and clock
+    # issues 10 lop3 (2 for the row summary, 4 for the bit-sliced count, 4 for the reference rule) and
+    # 2 funnel shifts on that pipe (ncu counts 13.0 of its instructions, loads and stores included).
+    # The logic pipe retires 64 lanes per SM and clock
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     word_gens = (N // 32) * TB_GENS
-    logic_ops = 11 * word_gens
+    logic_ops = 12 * word_gens
     ops_achieved = logic_ops / (bits_ms * 1e-3) / 1e12  # Tops/s
     bits_bytes = N * 3 / 8 * TB_GENS
     bits_achieved = bits_bytes / (bits_ms * 1e-3) / 1e9
