@@ -313,6 +313,16 @@ __global__ void __launch_bounds__(256) life_bits_sweep(const uint32_t* __restric
 constexpr int TB_STEPS = 16;  // generations per launch (max)
 constexpr int TB_WARPS = 8;
 
+// The tiles of a grid of nw words a row: `cols` columns of 30 words, and (rest > 0) one of the `rest` words that
+// are left, `side` tiles of which, one above the other in the grid, stand side by side in a warp, each with its
+// own two halo words: nothing but the lanes' places differs, as a stale outer bit is all that lanes of
+// different tiles give each other.  A column of its own for the rest, us for 64 generations against this:
+// 2080 x 30000 178 / 133, 4096^2 46.2 / 44.3, 6016 x 5000 76.6 / 73.4 (B3/S23 143 / 109, 40.0 / 37.4, 62.9 / 58.2).
+struct LifeTiles {
+    unsigned whole;  // tiles of whole columns, dealt along the rows
+    int cols, rest, side;
+};
+
 // One lane's words of a region: word `q` of every row, or (general) the 32 cells that start r bits
 // into word q, of which only `cnt` lie before the row's end and the others are the row's first.
 struct WordSource {
@@ -326,13 +336,21 @@ struct WordSource {
         r = (int)(s & 31);
         cnt = nx - (int)s;
     }
-    __device__ __forceinline__ uint32_t load(const uint32_t* __restrict__ row) const
+    __device__ __forceinline__ bool whole() const { return r == 0 && cnt >= 32; }  // the word as it is stored
+    struct Parts {
+        uint32_t lo, hi, first;
+    };
+    __device__ __forceinline__ Parts fetch(const uint32_t* __restrict__ row) const
     {
-        const uint32_t lo = __ldg(row + q);
-        if (r == 0 && cnt >= 32) return lo;
-        const uint32_t hi = q + 1 < nw ? __ldg(row + q + 1) : 0u;
-        const uint32_t w = __funnelshift_r(lo, hi, r);
-        return cnt >= 32 ? w : (w & ((1u << cnt) - 1u)) | (__ldg(row) << cnt);
+        Parts v = {__ldg(row + q), 0u, 0u};
+        if (q + 1 < nw) v.hi = __ldg(row + q + 1);
+        if (cnt < 32) v.first = __ldg(row);
+        return v;
+    }
+    __device__ __forceinline__ uint32_t join(const Parts& v) const
+    {
+        const uint32_t w = __funnelshift_r(v.lo, v.hi, r);
+        return cnt >= 32 ? w : (w & ((1u << cnt) - 1u)) | (v.first << cnt);
     }
 };
 
@@ -365,38 +383,77 @@ __device__ __forceinline__ void band_generation(const uint32_t (&c)[R], uint32_t
     }
 }
 
-template <int RULE, int R, bool RAGGED>
+template <int RULE, int R, bool RAGGED, bool BESIDE>
 __global__ void __launch_bounds__(TB_WARPS * 32, 2) life_bits_tb(const uint32_t* __restrict__ curG, const uint32_t* __restrict__ oldG,
                                                                  uint32_t* __restrict__ outCur, uint32_t* __restrict__ outOld, int nx, int nw,
-                                                                 int ny, int tiles_x, int steps)
+                                                                 int ny, LifeTiles tiles, int steps)
 {
     const gb::BlockId bid = gb::grid_wait();
     constexpr int W = TB_WARPS, RR = R * W, ROWS = RR - 2 * TB_STEPS;  // rows of the region, of the tile
     __shared__ uint32_t top[2][W][32], bot[2][W][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int ty = (int)(bid.x / (unsigned)tiles_x), tx = (int)bid.x - ty * tiles_x;
-    int wx = (tx * 30 - 1 + lane) % nw;
+    int ty, word;
+    bool mine;  // this lane's words are written
+    if (!BESIDE || bid.x < tiles.whole) {
+        ty = (int)(bid.x / (unsigned)tiles.cols);
+        word = ((int)bid.x - ty * tiles.cols) * 30 - 1 + lane;
+        mine = lane >= 1 && lane <= 30 && word < nw;
+    } else {  // the words left over
+        const int g = lane / (tiles.rest + 2), at = lane - g * (tiles.rest + 2);
+        ty = (int)(bid.x - tiles.whole) * tiles.side + g;
+        word = 30 * tiles.cols + at - 1;
+        mine = g < tiles.side && at >= 1 && at <= tiles.rest;
+    }
+    int wx = word % nw;
     if (wx < 0) wx += nw;
     WordSource src;
-    if (RAGGED) src.at(tx * 30 - 1 + lane, nx, nw);
+    if (RAGGED) src.at(word, nx, nw);
     const int y0 = ty * ROWS - TB_STEPS + R * w;  // the band's first row
     uint32_t c[R], o[R];
     {
         int gy = y0 % ny;
         if (gy < 0) gy += ny;
         const size_t plane = (size_t)ny * nw;
-        const uint32_t* pc = curG + (size_t)gy * nw + (RAGGED ? 0 : wx);
+        const uint32_t* pc = curG + (size_t)gy * nw;
         const ptrdiff_t old = oldG - curG;
         int wrap = ny - gy;  // the band's row at which the grid begins again
-#pragma unroll
-        for (int r = 0; r < R; r++) {
+        auto at_row = [&](int r) {
             if (r == wrap) {
                 pc -= plane;
                 wrap += ny;
             }
-            c[r] = RAGGED ? src.load(pc) : __ldg(pc);
-            o[r] = RULE != APPFIS_GB_LIFE_REFERENCE ? 0u : RAGGED ? src.load(pc + old) : __ldg(pc + old);
-            pc += nw;
+        };
+        if (!RAGGED || __all_sync(FULL, src.whole())) {
+            pc += RAGGED ? src.q : wx;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                at_row(r);
+                c[r] = __ldg(pc);
+                o[r] = RULE == APPFIS_GB_LIFE_REFERENCE ? __ldg(pc + old) : 0u;
+                pc += nw;
+            }
+        } else {
+            // four rows' loads before their words are put together: row by row, the warps at a row's end took
+            // 90 loads one after the other (3001 x 3000, 64 generations with the bytes' conversion 64 us, now 50)
+            constexpr int B = 4;
+#pragma unroll
+            for (int r0 = 0; r0 < R; r0 += B) {
+                WordSource::Parts a[B], b[B];
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                    if (r0 + k < R) {
+                        at_row(r0 + k);
+                        a[k] = src.fetch(pc);
+                        if (RULE == APPFIS_GB_LIFE_REFERENCE) b[k] = src.fetch(pc + old);
+                        pc += nw;
+                    }
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                    if (r0 + k < R) {
+                        c[r0 + k] = src.join(a[k]);
+                        o[r0 + k] = RULE == APPFIS_GB_LIFE_REFERENCE ? src.join(b[k]) : 0u;
+                    }
+            }
         }
     }
     const int above = w > 0 ? w - 1 : 0, below = w < W - 1 ? w + 1 : W - 1;  // the region's outer rows go stale
@@ -421,12 +478,11 @@ __global__ void __launch_bounds__(TB_WARPS * 32, 2) life_bits_tb(const uint32_t*
     // the newest state is in o after an odd number of generations
     uint32_t* __restrict__ outC = odd ? outOld : outCur;
     uint32_t* __restrict__ outO = odd ? outCur : outOld;
-    const int wout = tx * 30 - 1 + lane;
-    const uint32_t keep = RAGGED && wout == nw - 1 ? (1u << (nx & 31)) - 1u : FULL;
-    if (lane < 1 || lane > 30 || wout >= nw) return;
+    const uint32_t keep = RAGGED && word == nw - 1 ? (1u << (nx & 31)) - 1u : FULL;
+    if (BESIDE ? !mine : lane < 1 || lane > 30 || word >= nw) return;
     const int first = TB_STEPS - R * w, end = min(RR - TB_STEPS - R * w, ny - y0);  // the band's rows to be written
-    uint32_t* pc = outC + (ptrdiff_t)y0 * nw + wout;
-    uint32_t* po = outO + (ptrdiff_t)y0 * nw + wout;
+    uint32_t* pc = outC + (ptrdiff_t)y0 * nw + word;
+    uint32_t* po = outO + (ptrdiff_t)y0 * nw + word;
 #pragma unroll
     for (int r = 0; r < R; r++) {
         if (r >= first && r < end) {
@@ -638,48 +694,70 @@ struct TbPair {
     uint32_t* p[2];  // state at t, state at t-1
 };
 
-#define LIFE_BANDS(F) F(8) F(10) F(12) F(14) F(16) F(18) F(20) F(22) F(24) F(28) F(32) F(36) F(40) F(45)
+#define LIFE_BANDS(F) F(8) F(10) F(12) F(14) F(16) F(18) F(20) F(22) F(24) F(26) F(28) F(30) F(33) F(36) F(39) F(41) F(43) F(45)
 
-// Rows per band: the height whose tiles, dealt to the SMs, take the least time; the fullest SM's tiles follow
-// one another on its logic pipe, 0.49 us per band row (and 0.2) for 16 generations, whatever is resident
-// together.  Tall bands compute less halo (45 rows: 10%, 8: half), but a small grid needs many.  Measured, us
-// per 64 generations with 8 / 16 / 24 / 32 / 40 / 45 rows: 1024 x 1000 22 / 37 / 53 / 70 / 86 / 97; 2048^2 38 / 38 / 53 /
-// 70 / 87 / 98; 4096^2 86 / 67 / 54 / 71 / 87 / 98; 8192^2 262 / 192 / 191 / 193 / 163 / 184; 16384^2 985 / 665 / 613 / 573 /
-// 555 / 541.  (Planes in shared memory, tiles of 32 to 256 rows: 49, 66, 107, 211, 706.)
-int tb_band(int nw, int ny)
+unsigned life_tiles(int nw, int ny, int rows, bool beside, LifeTiles& t)
 {
-    const long long tiles_x = (nw + 29) / 30, sms = gb::sm_count();
-    int best = 8;
+    const unsigned high = gb::ceil_div(ny, rows);
+    t.cols = beside ? nw / 30 : (nw + 29) / 30;
+    t.rest = beside ? nw % 30 : 0;
+    t.side = 32 / (t.rest + 2);
+    t.whole = (unsigned)t.cols * high;
+    return t.whole + (t.rest ? gb::ceil_div(high, t.side) : 0u);
+}
+
+struct LifePlan {
+    int band;
+    bool beside;
+};
+
+// Rows per band, and whether the words left over from whole columns go side by side: what takes the least time
+// with the tiles dealt to the SMs; the fullest SM's tiles follow one another on its logic pipe, 0.47 us per band
+// row (and 0.2) for 16 generations, whatever is resident together.  Tall bands compute less halo (45 rows:
+// 10%, 8: half), but a small grid needs many.  Measured with 11 lop3 a word, us per 64 generations with 8 / 16 / 24 /
+// 32 / 40 / 45 rows: 1024 x 1000 22 / 37 / 53 / 70 / 86 / 97; 2048^2 38 / 38 / 53 / 70 / 87 / 98; 4096^2 86 / 67 / 54 / 71 / 87 / 98;
+// 8192^2 262 / 192 / 191 / 193 / 163 / 184; 16384^2 985 / 665 / 613 / 573 / 555 / 541.  (Planes in shared memory, tiles of
+// 32 to 256 rows: 49, 66, 107, 211, 706.)  Side by side costs its warps scattered loads (1024 x 1000, where whole
+// columns leave most SMs idle anyway: 20.6 against 23.9), so it has to save 5% (16384^2, 4% fewer: 521 against 519), and half a column or more
+// is a column.
+LifePlan tb_plan(int nw, int ny)
+{
+    const unsigned sms = gb::sm_count();
+    LifePlan best = {8, false};
     double cost = 1e30;
-#define LIFE_COST(R)                                                                                        \
-    {                                                                                                       \
-        const long long tiles = tiles_x * ((ny + 8 * R - 2 * TB_STEPS - 1) / (8 * R - 2 * TB_STEPS));       \
-        const double c = (double)((tiles + sms - 1) / sms) * (0.49 * R + 0.2);                              \
-        if (c <= cost) {                                                                                    \
-            cost = c;                                                                                       \
-            best = R;                                                                                       \
-        }                                                                                                   \
+    LifeTiles t;
+    for (int beside = 0; beside < (nw % 30 && nw % 30 <= 14 ? 2 : 1); beside++) {
+#define LIFE_COST(R)                                                                                                             \
+    {                                                                                                                            \
+        const unsigned tiles = life_tiles(nw, ny, 8 * R - 2 * TB_STEPS, beside != 0, t);                                         \
+        const double c = (double)gb::ceil_div(tiles, sms) * (0.47 * R + 0.2) * (beside ? 1.05 : 1.0);                            \
+        if (c < cost || (c == cost && !beside)) {                                                                                \
+            cost = c;                                                                                                            \
+            best = {R, beside != 0};                                                                                             \
+        }                                                                                                                        \
     }
-    LIFE_BANDS(LIFE_COST)
+        LIFE_BANDS(LIFE_COST)
 #undef LIFE_COST
+    }
     return best;
 }
 
 template <int RULE, int R>
-void launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+void launch_tb(TbPair in, TbPair out, int nx, int nw, int ny, int steps, bool beside, cudaStream_t st)
 {
     static_assert(TB_WARPS == 8, "bands of 8 warps");
-    const int tiles_x = (nw + 29) / 30;
-    const unsigned tiles = (unsigned)tiles_x * gb::ceil_div(ny, R * TB_WARPS - 2 * TB_STEPS);
-    gb::launch(nx % 32 ? life_bits_tb<RULE, R, true> : life_bits_tb<RULE, R, false>, tiles, TB_WARPS * 32, 0, st, in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, tiles_x, steps);
+    LifeTiles t;
+    const unsigned tiles = life_tiles(nw, ny, R * TB_WARPS - 2 * TB_STEPS, beside, t);
+    auto kernel = nx % 32 ? life_bits_tb<RULE, R, true, true> : beside ? life_bits_tb<RULE, R, false, true> : life_bits_tb<RULE, R, false, false>;
+    gb::launch(kernel, tiles, TB_WARPS * 32, 0, st, in.p[0], in.p[1], out.p[0], out.p[1], nx, nw, ny, t, steps);
 }
 
 template <int RULE>
-void tb_step(int band, TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
+void tb_step(LifePlan plan, TbPair in, TbPair out, int nx, int nw, int ny, int steps, cudaStream_t st)
 {
-    switch (band) {
+    switch (plan.band) {
 #define LIFE_CASE(R) \
-    case R: return launch_tb<RULE, R>(in, out, nx, nw, ny, steps, st);
+    case R: return launch_tb<RULE, R>(in, out, nx, nw, ny, steps, plan.beside, st);
         LIFE_BANDS(LIFE_CASE)
 #undef LIFE_CASE
     }
@@ -691,12 +769,13 @@ void tb_step(int band, TbPair in, TbPair out, int nx, int nw, int ny, int steps,
 template <int RULE>
 int run_tb(const TbPair (&pair)[3], TbPair last, int nx, int ny, int gens, int launches, cudaStream_t st)
 {
-    const int nw = (nx + 31) / 32, band = tb_band(nw, ny);
+    const int nw = (nx + 31) / 32;
+    const LifePlan plan = tb_plan(nw, ny);
     int at = 0, done = 0;
     for (int n = 0; n < launches; n++) {
         const int next = (pair[2].p[0] && n < 3) ? (n + 1) % 3 : 1 - at;
         const int upto = (int)((long long)gens * (n + 1) / launches);
-        tb_step<RULE>(band, pair[at], n + 1 == launches ? last : pair[next], nx, nw, ny, upto - done, st);
+        tb_step<RULE>(plan, pair[at], n + 1 == launches ? last : pair[next], nx, nw, ny, upto - done, st);
         done = upto;
         at = next;
     }
