@@ -694,7 +694,7 @@ struct TbPair {
     uint32_t* p[2];  // state at t, state at t-1
 };
 
-#define LIFE_BANDS(F) F(8) F(10) F(12) F(14) F(16) F(18) F(20) F(22) F(24) F(26) F(28) F(30) F(33) F(36) F(39) F(41) F(43) F(45)
+#define LIFE_BANDS(F) F(5) F(6) F(7) F(8) F(10) F(12) F(14) F(16) F(18) F(20) F(22) F(24) F(26) F(28) F(30) F(33) F(36) F(39) F(41) F(43) F(45)
 
 unsigned life_tiles(int nw, int ny, int rows, bool beside, LifeTiles& t)
 {
@@ -714,12 +714,13 @@ struct LifePlan {
 // Rows per band, and whether the words left over from whole columns go side by side: what takes the least time
 // with the tiles dealt to the SMs; the fullest SM's tiles follow one another on its logic pipe, 0.47 us per band
 // row (and 0.2) for 16 generations, whatever is resident together.  Tall bands compute less halo (45 rows:
-// 10%, 8: half), but a small grid needs many.  Measured with 11 lop3 a word, us per 64 generations with 8 / 16 / 24 /
+// 10%, 8: half, 5: four fifths), but a small grid needs many: 256^2 16.2 us for 64 generations with 5 rows against
+// 20.1 with 8, 1024 x 1000 18.3 with 6 against 20.6.  Measured with 11 lop3 a word, us per 64 generations with 8 / 16 / 24 /
 // 32 / 40 / 45 rows: 1024 x 1000 22 / 37 / 53 / 70 / 86 / 97; 2048^2 38 / 38 / 53 / 70 / 87 / 98; 4096^2 86 / 67 / 54 / 71 / 87 / 98;
 // 8192^2 262 / 192 / 191 / 193 / 163 / 184; 16384^2 985 / 665 / 613 / 573 / 555 / 541.  (Planes in shared memory, tiles of
 // 32 to 256 rows: 49, 66, 107, 211, 706.)  Side by side costs its warps scattered loads (1024 x 1000, where whole
-// columns leave most SMs idle anyway: 20.6 against 23.9), so it has to save 5% (16384^2, 4% fewer: 521 against 519), and half a column or more
-// is a column.
+// columns leave SMs idle anyway: 20.6 against 23.9), so it has to save 0.8 us and 5% (16384^2, 4% fewer: 521
+// against 519), and half a column or more is a column.
 LifePlan tb_plan(int nw, int ny)
 {
     const unsigned sms = gb::sm_count();
@@ -730,7 +731,8 @@ LifePlan tb_plan(int nw, int ny)
 #define LIFE_COST(R)                                                                                                             \
     {                                                                                                                            \
         const unsigned tiles = life_tiles(nw, ny, 8 * R - 2 * TB_STEPS, beside != 0, t);                                         \
-        const double c = (double)gb::ceil_div(tiles, sms) * (0.47 * R + 0.2) * (beside ? 1.05 : 1.0);                            \
+        double c = (double)gb::ceil_div(tiles, sms) * (0.47 * R + 0.2);                                                          \
+        if (beside) c = std::max(1.05 * c, c + 0.8);                                                                             \
         if (c < cost || (c == cost && !beside)) {                                                                                \
             cost = c;                                                                                                            \
             best = {R, beside != 0};                                                                                             \
