@@ -53,15 +53,14 @@ __device__ __forceinline__ float2 heat_pair(float2 c, float2 l, float2 r, float2
     return f2::add(f2::add(c, x), y);
 }
 
-// Overlapped tiling: a CTA of W warps holds a 128 x 8W region in registers for up to 8 sweeps and writes
-// the 112 x (8W - 16) tile in its middle.  A warp owns a band of 8 rows, a lane 4 columns of it, so that the
+// Overlapped tiling: a CTA of W warps holds a 128 x (HR W) region in registers for up to 8 sweeps and writes
+// the 112 x (HR W - 16) tile in its middle.  A warp owns a band of HR rows, a lane 4 columns of it, so that the
 // x neighbours at a lane's edges come by shuffle and only a band's first and last row go through shared
 // memory (one 16-byte vector each per lane and sweep, one barrier).  A sweep works down the band and
 // replaces the rows as it goes, keeping one old row.  Ghost-ring cells and cells outside the field
 // keep their values; every other cell of the region is updated each sweep (those outside the shrinking
 // valid window only feed cells that are not written back).
 constexpr int HS = 8;             // sweeps per launch, and halo width
-constexpr int HR = 8;             // rows per band
 constexpr int HTX = 128 - 2 * HS;  // output columns
 
 template <int G> struct HeatVec;  // G floats that are aligned together
@@ -71,7 +70,7 @@ template <> struct HeatVec<4> { typedef float4 type; };
 
 // MASK: the region reaches the ghost ring or beyond the field: loads are guarded and only interior cells
 // are updated and stored.
-template <int W, int G, bool MASK>
+template <int W, int HR, int G, bool MASK>
 __device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch, int ns, float cx,
                                           float cy, int bx, int by, float4 (&top)[2][W][32], float4 (&bot)[2][W][32])
 {
@@ -140,44 +139,47 @@ __device__ __forceinline__ void heat_tile(const float* __restrict__ cur, float* 
     }
 }
 
-template <int W, int G>
-__global__ void __launch_bounds__(32 * W, 24 / W) heat2d_bands(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch,
+template <int W, int HR, int G>
+__global__ void __launch_bounds__(32 * W, HR == 8 ? 24 / W : 4) heat2d_bands(const float* __restrict__ cur, float* __restrict__ nxt, int nx, int ny, int pitch,
                                                             int ns, float cx, float cy)
 {
     const gb::BlockId bid = gb::grid_wait();
     __shared__ float4 top[2][W][32], bot[2][W][32];
     const int bx = (int)bid.x, by = (int)bid.y, x0 = bx * HTX - HS, y0 = 1 + by * (HR * W - 2 * HS) - HS;
     if (x0 >= 1 && y0 >= 1 && x0 + 127 <= nx && y0 + HR * W - 1 <= ny)  // the whole region lies on interior cells
-        heat_tile<W, G, false>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
+        heat_tile<W, HR, G, false>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
     else
-        heat_tile<W, G, true>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
+        heat_tile<W, HR, G, true>(cur, nxt, nx, ny, pitch, ns, cx, cy, bx, by, top, bot);
 }
 
-long long heat_tiles(int w, int nx, int ny) { return (long long)gb::ceil_div(nx + 1, HTX) * gb::ceil_div(ny, HR * w - 2 * HS); }
+long long heat_tiles(int rows, int nx, int ny) { return (long long)gb::ceil_div(nx + 1, HTX) * gb::ceil_div(ny, rows - 2 * HS); }
 
-// Warps per CTA: 8 (112 x 48 tiles: 1.5 points computed per point written), unless a small grid's launch is
-// shorter with 4 (112 x 16 tiles, 2.3, but a third as long) or 12 (112 x 80, 1.4).  A launch lasts about
-// 3.2 us and 1.45 / 3.3 us for each tile of the fullest SM; 12 warps 9 us if every SM has one tile at most.
-// Us per 8 sweeps with 4 / 8 / 12 warps: 64^2 4.5 / 5.7 / 7.3; 512^2 5.9 / 6.4 / 8.7; 777 x 900 7.8 / 6.5 / 8.8;
-// 1024^2 10.6 / 9.6 / 8.8; 1500^2 17.1 / 13.4 / 14.9; 2048^2 28.4 / 22.4 / 23.8; 4096^2 97 / 72 / 72.
+// Rows of a CTA's region: 64 (8 warps of 8 rows, 112 x 48 tiles: 1.5 points computed per point written), unless a
+// small grid's launch is shorter with 32 (8 warps of 4 rows: 2.3, but a third as long), 20 (10 warps of 2 rows: 5.7)
+// or 96 (12 warps of 8 rows: 1.4).  A launch lasts about 3.2 us and 3.3 for each tile of the fullest SM, 2.4 and 1.6
+// with 32 rows, 2.1 and 1.15 with 20; 96 rows 9 us if every SM has one tile at most.  Us per 8 sweeps with 20 / 32 / 64 /
+// 96 rows: 64^2 3.2 / 3.7 / 5.7 / 7.3; 250 x 190 3.4 / 3.9; 512^2 7.9 / 5.7 / 6.4 / 8.7; 777 x 900 14.8 / 7.5 / 6.5 / 8.8; 1024^2
+// 21.7 / 9.9 / 9.6 / 8.8; 1500^2 42 / 16.7 / 13.4 / 14.9; 2048^2 75 / 28 / 22.4 / 23.8; 4096^2 283 / 98 / 72 / 72.  32 rows as 4 warps
+// of 8: 4.6, 4.7, 6.0, 7.8, 10.6; 64 rows as 16 warps of 4: 5.8, 6.5, 6.6, 6.7, 10.8.
 // The 4 x 4 register blocks that this replaced (48 x 32 tiles, four edge vectors per thread and sweep through
-// shared memory): 6.4, 8.4, 14.5, 15.7, 26.4, 40.5, 139.  Bound by instruction issue and the sweep's
-// barrier; 16 warps 10.7 and more up to 1024^2.
-int heat_warps(int nx, int ny)
+// shared memory): 64^2 6.4, 512^2 8.4, 777 x 900 14.5, 1024^2 15.7, 1500^2 26.4, 2048^2 40.5, 4096^2 139.  Bound by
+// instruction issue and the sweep's barrier; 16 warps of 8 rows 10.7 and more up to 1024^2.
+int heat_region(int nx, int ny)
 {
     const double sms = gb::sm_count();
-    auto full = [&](int w) { return std::ceil((double)heat_tiles(w, nx, ny) / sms); };
-    const double c4 = 3.2 + 1.45 * full(4), c8 = 3.2 + 3.3 * full(8), c12 = full(12) <= 1 ? 9.0 : 1e30;
-    return c8 <= c4 && c8 <= c12 ? 8 : (c12 <= c4 ? 12 : 4);
+    auto full = [&](int rows) { return std::ceil((double)heat_tiles(rows, nx, ny) / sms); };
+    const int rows[4] = {64, 32, 20, 96};
+    const double cost[4] = {3.2 + 3.3 * full(64), 2.4 + 1.6 * full(32), 2.1 + 1.15 * full(20), full(96) <= 1 ? 9.0 : 1e30};
+    return rows[std::min_element(cost, cost + 4) - cost];
 }
 
 // The copies' width goes by the alignment of the rows (region rows start on 4-element boundaries).
-template <int W>
+template <int W, int HR>
 void launch_bands(const float* cur, float* nxt, int nx, int ny, int pitch, int ns, float cx, float cy, cudaStream_t st)
 {
     const dim3 grd(gb::ceil_div(nx + 1, HTX), gb::ceil_div(ny, HR * W - 2 * HS));
     const unsigned long long align = (unsigned long long)pitch * sizeof(float) | reinterpret_cast<uintptr_t>(cur) | reinterpret_cast<uintptr_t>(nxt);
-    auto kern = align % 16 == 0 ? heat2d_bands<W, 4> : (align % 8 == 0 ? heat2d_bands<W, 2> : heat2d_bands<W, 1>);
+    auto kern = align % 16 == 0 ? heat2d_bands<W, HR, 4> : (align % 8 == 0 ? heat2d_bands<W, HR, 2> : heat2d_bands<W, HR, 1>);
     gb::launch(kern, grd, 32 * W, 0, st, cur, nxt, nx, ny, pitch, ns, cx, cy);
 }
 
@@ -206,14 +208,13 @@ int appfis_gb_heat2d(float* a, float* b, int nx, int ny, int pitch, int iters, f
     GB_TRY(check_heat(a, b, nx, ny, pitch));
     if (iters < 0) return gb::fail(APPFIS_GB_EINVAL, "heat2d: negative iteration count");
     cudaStream_t st = gb::as_stream(stream);
-    const int warps = heat_warps(nx, ny);
+    const int rows = heat_region(nx, ny);
     float* buf[2] = {a, b};
     int ci = 0;
     for (int done = 0; done < iters;) {
         const int ns = std::min(HS, iters - done);
-        if (warps == 8) launch_bands<8>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
-        else if (warps == 12) launch_bands<12>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
-        else launch_bands<4>(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
+        auto launch = rows == 64 ? launch_bands<8, 8> : rows == 32 ? launch_bands<8, 4> : rows == 20 ? launch_bands<10, 2> : launch_bands<12, 8>;
+        launch(buf[ci], buf[1 - ci], nx, ny, pitch, ns, cx, cy, st);
         ci = 1 - ci;
         done += ns;
     }
