@@ -60,7 +60,6 @@ struct Params {
     double* dtlog;  // [ndom][max_steps] or null
     unsigned char* zc;  // [2][total_strips] dry-step counters (null: every strip every step)
     unsigned* order;    // [2][total_strips] the strips in the order that steps of each parity take them (null: as numbered)
-    int spread;         // warps' first places go round the CTAs (else: eight in a row to each)
     unsigned long long spin_limit;  // polls before a grid-barrier wait gives up
     int stall_cta;                  // testing: this CTA skips its arrival at the first barrier (-1: none)
     const SrcDev* srcs;             // [ndom] point sources, or null (no source phase)
@@ -372,34 +371,35 @@ struct DomCtl {
 // The order of step n (the first step has none listed: as numbered).
 __device__ __forceinline__ const unsigned* step_order(const Params& p, int n)
 {
-    return p.order && n > 0 ? p.order + (size_t)(n & 1) * p.total_strips : nullptr;
+    return n > 0 ? p.order + (size_t)(n & 1) * p.total_strips : nullptr;
 }
 
 // Strips of one phase: warp w first takes the strip in place w, then those in places nwarps + k for the
 // tickets k it draws from *ctr (zeroed after the phase's grid barrier, for its next use two steps later).
-// The strip after next's ticket and the next strip's number are requested before the current strip is
-// processed, so their latency hides behind the work.  Warps without a first strip draw none (a batch
-// smaller than the grid costs no atomics).
+// The next ticket is requested before the current strip is processed, so its latency hides
+// behind the work.  Warps without a first strip draw none (a batch smaller than the grid costs
+// no atomics).
 template <class F>
 __device__ __forceinline__ void for_strips(unsigned* ctr, const unsigned* order, long long first, long long nwarps, long long total, int lane, F&& body)
 {
-    if (first >= total) return;
-    unsigned s = order ? __ldcg(order + first) : (unsigned)first;
+    long long at = first;
     unsigned tk = 0;
-    if (lane == 0) tk = atomicAdd(ctr, 1u);
-    long long at = nwarps + (long long)__shfl_sync(0xffffffffu, tk, 0);
-    for (;;) {
-        const bool more = at < total;  // uniform in the warp
-        unsigned sn = 0;
-        if (more) {
-            sn = order ? __ldcg(order + at) : (unsigned)at;
-            if (lane == 0) tk = atomicAdd(ctr, 1u);
-        }
-        body((long long)s);
-        if (!more) return;
-        s = sn;
+    if (at < total && lane == 0) tk = atomicAdd(ctr, 1u);
+    while (at < total) {
+        body(order ? (long long)__ldcg(order + at) : at);
         at = nwarps + (long long)__shfl_sync(0xffffffffu, tk, 0);
+        if (at < total && lane == 0) tk = atomicAdd(ctr, 1u);
     }
+}
+
+// A warp's first place: round the CTAs, as strips in a row are wet together, and an SM's warps share its
+// FP64 pipe (FP64 100^2 128 -> 122 us per step; 300 x 1100 wet first 232 -> 148); FP32 as numbered eight in a row to
+// a CTA (300^2 11.6 us against 12.9).
+template <class T, bool ORDER>
+__device__ __forceinline__ long long first_place()
+{
+    if (ORDER || sizeof(T) == 8) return (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    return ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 }
 
 // Lists strip s for the step of parity `next`: wet ones from the front, dry ones from the back.  A step lasts
@@ -408,7 +408,7 @@ __device__ __forceinline__ void for_strips(unsigned* ctr, const unsigned* order,
 // order depends on it: the strips of a phase are independent.
 __device__ __forceinline__ void list_strip(Ctl* ctl, const Params& p, int next, long long s, bool dry, int lane)
 {
-    if (p.order && lane == 0) {
+    if (lane == 0) {
         const unsigned at = dry ? (unsigned)p.total_strips - 1u - atomicAdd(&ctl->dry[next], 1u) : atomicAdd(&ctl->wet[next], 1u);
         p.order[(size_t)next * p.total_strips + at] = (unsigned)s;
     }
@@ -459,9 +459,9 @@ __device__ void apply_sources(const Dom<T>& D, const SrcDev& S, Ctl* ctl, int cu
 #define FLOOD_F32_MIN_BLOCKS 3
 #endif
 
-// SKIP: dry strips are left out (Params::zc set); a separate instantiation, so the full sweep
-// carries none of the bookkeeping.
-template <class T, bool SKIP>
+// SKIP: dry strips are left out (Params::zc set); ORDER: wet strips first (Params::order set); separate
+// instantiations, so the others carry none of the bookkeeping.
+template <class T, bool SKIP, bool ORDER>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1) flood_persistent(const Dom<T>* __restrict__ gdoms, Ctl* ctl,
                                                                                 Params p)
 {
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     __shared__ DomCtl<T> dc;
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
     __syncthreads();
-    const long long warp = p.spread ? (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long warp = first_place<T, ORDER>();
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     const double big = (double)K<T>::big();
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (fix ? 2 : 0) | (want ? 4 : 0));
         }
         __syncthreads();
-        const unsigned* order = step_order(p, n);
+        const unsigned* order = ORDER ? step_order(p, n) : nullptr;
         for_strips(&ctl->ticket[cur], order, warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
             const int f = dc.flags[d];
@@ -522,12 +522,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             } else if (f & 4) {
                 dry = phase_b<T>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p);
             }
-            list_strip(ctl, p, 1 - cur, s, dry, lane);
+            if (ORDER) list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
             ctl->ticketb[cur] = 0;
-            ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
+            if (ORDER) ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
         }
         if (p.srcs) {  // the point sources of step n, seen by the next step's wet/dry fix and dt
             if (blockIdx.x == 0 && threadIdx.x < p.ndom)
@@ -795,7 +795,7 @@ __device__ bool phase_bf(const Dom<T>& D, long long local, int b, T dt, const Pa
 // step n+2 is reset by block 0 during step n (nobody reads or writes it then).
 // STAGED: the step's rows arrive through each warp's TMA ring (FS_SMEM bytes of dynamic shared
 // memory; FP32 domains whose rows are 16-byte aligned).
-template <class T, bool SKIP, bool STAGED = false>
+template <class T, bool SKIP, bool ORDER, bool STAGED = false>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1) flood_fused(const Dom<T>* __restrict__ gdoms, Ctl* ctl,
                                                                                           Params p)
 {
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     }
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
     __syncthreads();
-    const long long warp = p.spread ? (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long warp = first_place<T, ORDER>();
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     const double big = (double)K<T>::big();
@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
         }
         if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
         const int dn = (n + 1) % 3;
-        for_strips(&ctl->ticketb[cur], step_order(p, n), warp, nwarps, p.total_strips, lane, [&](long long s) {
+        for_strips(&ctl->ticketb[cur], ORDER ? step_order(p, n) : nullptr, warp, nwarps, p.total_strips, lane, [&](long long s) {
             const int d = find_domain(doms, p.ndom, s);
             const int f = dc.flags[d];
             bool dry = true;
@@ -861,12 +861,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             } else if (f & 4) {
                 dry = phase_bf<T, STAGED>(doms[d], s - doms[d].strip0, f & 1, dc.dt[d], p, &ctl->dtbits[dn][d], &ring, d, ctl);
             }
-            list_strip(ctl, p, 1 - cur, s, dry, lane);
+            if (ORDER) list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
             ctl->ticketb[cur] = 0;
-            ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
+            if (ORDER) ctl->wet[1 - cur] = ctl->dry[1 - cur] = 0;
         }
     }
 }

@@ -162,7 +162,6 @@ inline int upload_sources(const appfis_gb_flood_domain* doms, const appfis_gb_fl
         od += (size_t)S.nt * S.n;
     }
     GB_CUDA(cudaMemcpyAsync(dev, host.data(), host.size(), cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaStreamSynchronize(st));  // the host table is a local
     *out = reinterpret_cast<const SrcDev*>(dev);
     return APPFIS_GB_OK;
 }
@@ -194,16 +193,18 @@ int strip_rows(const appfis_gb_flood_domain* doms, int ndom, int scols, long lon
 
 // Whether a batch takes its wet strips first.  As numbered / wet strips first, us per step, full sweep
 // and with dry strips left out:
-//   FP32 700^2 (1.3 strips a warp) 22.3 / 22.7, 16.1 / 17.4; 1024^2 (2.6) 34.3 / 30.7, 28.2 / 23.5; six domains of 3.6 M cells (4.5)
-//     67.0 / 56.6, 49.8 / 36.5; 2 x 3000^2 (11) 189 / 262, 92.7 / 72.3; 32 domains (25) 873 / 1180, 243 / 240
-//   FP64 300^2 (1.2) 133 / 133, 126 / 125; 300 x 1100 (4.6) 292 / 155, 267 / 129; 1024^2 (15) 428 / 290, 382 / 202; six (13, 8 rows)
-//     1174 / 807, 1029 / 606; 2 x 3000^2 (62) 3514 / 3145, 2443 / 2167
+//   FP32 700^2 (1.3 strips a warp) 22.3 / 22.7, 16.1 / 17.4; 1024^2 (2.6) 29.7 / 26.0, 24.0 / 20.1; six domains of 3.6 M cells (4.5)
+//     63.5 / 50.1, 44.9 / 31.5; 2048^2 (5.2) 60.7 / 56.5, 43.6 / 33.1; 2 x 3000^2 (11) 176 / 262, 85.5 / 66.7; 32 domains (25)
+//     672 / 1180, 230 / 235
+//   FP64 300^2 (1.2) 133 / 133, 126 / 125; 300 x 1100 (4.6) 251 / 148, 240 / 129; 1024^2 (15) 350 / 286, 306 / 205; six (13, 8 rows)
+//     1168 / 806, 986 / 599; 2 x 3000^2 (62) 3310 / 3132, 2354 / 2159
 // Below two strips a warp all start at once.  A full FP32 sweep with many strips a warp is bound by
-// memory: its dry strips' traffic then runs beside the wet strips' arithmetic, and neighbours share lines.
+// memory: its dry strips' traffic then runs beside the wet strips' arithmetic, and neighbours share lines; with
+// dry strips left out a batch of tall strips has enough wet ones to even out.
 template <class T>
 bool wet_first(long long strips, int rows, long long warps, bool skip)
 {
-    return strips >= 2 * warps && (sizeof(T) == 8 || skip || rows < 16);
+    return strips >= 2 * warps && (sizeof(T) == 8 || rows < (skip ? 32 : 16));
 }
 
 // Uploads the table, initialises the control block and launches the persistent kernel.
@@ -214,6 +215,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     if (!doms || !prm || ndom < 1 || ndom > MAXD) return gb::fail(APPFIS_GB_EINVAL, "flood: 1..%d domains required", MAXD);
     if (!(prm->dx > 0) || !(prm->courant > 0) || !(prm->print_interval > 0) || prm->max_steps < 0)
         return gb::fail(APPFIS_GB_EINVAL, "flood: bad parameters");
+    if (gb::capturing(st)) return gb::fail(APPFIS_GB_ECUDA, "flood: the batch's tables cannot be copied while the stream is captured");
     // the fused pass for the full sweep without point sources
     if ((prm->flags & APPFIS_GB_FLOOD_TWO_PHASE) && (prm->flags & APPFIS_GB_FLOOD_FUSED))
         return gb::fail(APPFIS_GB_EINVAL, "flood: TWO_PHASE and FUSED are exclusive");
@@ -240,9 +242,9 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
         staged = staged && (D.pitch * sizeof(T)) % 16 == 0;
     }
     int per_sm = 0;
-    auto kern = staged  ? flood_fused<T, false, true>
-                : fused ? (skip ? flood_fused<T, true> : flood_fused<T, false>)
-                        : (skip ? flood_persistent<T, true> : flood_persistent<T, false>);
+    auto kern = staged  ? flood_fused<T, false, false, true>
+                : fused ? (skip ? flood_fused<T, true, false> : flood_fused<T, false, false>)
+                        : (skip ? flood_persistent<T, true, false> : flood_persistent<T, false, false>);
     const int smem = staged ? FS_SMEM : 0;
     if (staged) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
@@ -250,14 +252,14 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     const long long warps = 8LL * per_sm * gb::sm_count();
     const int rows = strip_rows<T>(doms, ndom, scols, warps);
     GB_TRY(make_table<T>(doms, ndom, tab, total, scols, rows));
-    void *wt, *hs;
+    void* wt;
     GB_TRY(gb::workspace(gb::WS_REDUCE, sizeof(Ctl) + sizeof(Dom<T>) * MAXD + 256, &wt));
     Ctl* ctl = reinterpret_cast<Ctl*>(wt);
     Dom<T>* dtab = reinterpret_cast<Dom<T>*>(reinterpret_cast<char*>(wt) + ((sizeof(Ctl) + 255) / 256) * 256);
-    GB_TRY(gb::pinned(1, sizeof(Dom<T>) * ndom, &hs));
-    GB_CUDA(cudaStreamSynchronize(st));  // the pinned staging buffer may still feed an earlier copy
-    std::memcpy(hs, tab.data(), sizeof(Dom<T>) * ndom);
-    GB_CUDA(cudaMemcpyAsync(dtab, hs, sizeof(Dom<T>) * ndom, cudaMemcpyHostToDevice, st));
+    // this table, the sources' and the tensor maps come from pageable memory, which such a copy has read when it
+    // returns: the host goes on while earlier work of the stream runs (100^2, 20 steps
+    // 272 -> 257 us; six domains of 3.6 M cells 1270 -> 1250)
+    GB_CUDA(cudaMemcpyAsync(dtab, tab.data(), sizeof(Dom<T>) * ndom, cudaMemcpyHostToDevice, st));
     const double big = std::is_same<T, float>::value ? 3.402823466e38 : 1.7976931348623157e308;
     gb::launch(flood_init_ctl, 1, MAXD, 0, st, ctl, ndom, big, prm->t_start);
     GB_TRY(gb::launched("flood_init_ctl"));
@@ -297,7 +299,6 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
         void* dm;
         GB_TRY(gb::workspace(gb::WS_FLOOD_MAPS, sizeof(CUtensorMap) * maps.size(), &dm));
         GB_CUDA(cudaMemcpyAsync(dm, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, st));
-        GB_CUDA(cudaStreamSynchronize(st));  // the host copy is a local
         p.maps = reinterpret_cast<const CUtensorMap*>(dm);
         unsigned long long test_ns = 0;
         if (gb::take_test_stall(gb::TEST_TMA_SHORTFALL, &test_ns)) {  // a test runs the first stage's waits out
@@ -319,11 +320,15 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
 
     void* listed;  // without room for the lists: as numbered
     if (wet_first<T>(total, rows, warps, skip) &&
-        gb::workspace(gb::WS_FLOOD_ORDER, 2 * sizeof(unsigned) * (size_t)total, &listed) == APPFIS_GB_OK)
+        gb::workspace(gb::WS_FLOOD_ORDER, 2 * sizeof(unsigned) * (size_t)total, &listed) == APPFIS_GB_OK) {
         p.order = reinterpret_cast<unsigned*>(listed);
-    // round the CTAs: strips in a row are wet together, and an SM's warps share its FP64 pipe (FP64 100^2 128 -> 122 us per
-    // step; 300 x 1100 wet first 232 -> 155); FP32 as numbered 300^2 11.6 against 12.9
-    p.spread = p.order || sizeof(T) == 8;
+        kern = staged  ? flood_fused<T, false, true, true>
+               : fused ? (skip ? flood_fused<T, true, true> : flood_fused<T, false, true>)
+                       : (skip ? flood_persistent<T, true, true> : flood_persistent<T, false, true>);
+        if (staged) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+        if (per_sm < 1) return gb::fail(APPFIS_GB_ECUDA, "flood: kernel cannot be resident");
+    }
     long long want = (total * 32 + 255) / 256;  // one warp per strip at most
     int grid = (int)std::min<long long>(want, (long long)per_sm * gb::sm_count());
     if (grid < 1) grid = 1;
