@@ -475,7 +475,7 @@ def run_ours(args, rank, world, local):
     kernel_avg("appfis_gb_life_u8", ua, ub, 10)
     u8_ms = kernel_avg("appfis_gb_life_u8", ua, ub, 100)
     u8_bytes = N * 3
-    u8_achieved = u8_bytes / (u8_ms * 1e-3) / 1e9
+    u8_achieved = u8_bytes / (u8_ms * 1e-3) / 1e9  # one sweep's compulsory bytes for each generation
 
     # end to end through the C ABI from pinned host buffers
     pop = ctypes.c_int64(0)
@@ -532,8 +532,8 @@ def run_ours(args, rank, world, local):
         "forms": {
             "bits": {"glups": value, "ms_per_step": ms_bits, "kernel_ms": bits_ms, "achieved_gbs": bits_achieved},
             "u8": {"glups": N * gens / (ms_u8 * 1e-3) / 1e9 * world, "ms_per_step": ms_u8, "kernel_ms": u8_ms,
-                   "kernel": "life_u8_bulk", "achieved_gbs": u8_achieved, "frac": u8_achieved / hbm_peak,
-                   "bytes_per_lup": 3, "traffic": profiled_traffic("life_u8_bulk")},
+                   "kernel": "life_bits_tb (bytes to words and back around it)", "effective_gbs": u8_achieved,
+                   "bytes_per_lup": 3},
         },
         "clocks": clocks,
     }
@@ -620,8 +620,8 @@ def bench_heat(torch, gb, W, dev, sp, hbm):
     gbs = lups * 8 / (best * 1e-3) / 1e9
     return {"workload": "heat2d 1024^2 FP32, 1000 iterations, Dirichlet", "glups": lups / (best * 1e-3) / 1e9, "ms": best,
             "ms_stream_launches": ms, "ms_cuda_graph": ms_g, "bytes_per_lup": 8, "effective_gbs": gbs, "frac_of_hbm": gbs / hbm,
-            "note": "8.4 MB working set is L2-resident; 8 sweeps per launch on chip (4x4 point blocks in registers, "
-                    "block edges through shared memory; 125 launches, replayed from a CUDA graph); HBM fraction is nominal",
+            "note": "8.4 MB working set is L2-resident; 8 sweeps per launch on chip (bands of rows in registers, "
+                    "their edges through shared memory; 125 launches, replayed from a CUDA graph); HBM fraction is nominal",
             "form": "plain FP32 (bit-identical to the reference CPU path)",
             "error_vs_fp64": _err(out32, ref64), "l2_norm": float(out32[1:-1, 1:-1].norm().item()),
             "l2_norm_fp64": float(ref64[1:-1, 1:-1].norm().item())}
@@ -712,7 +712,7 @@ def bench_himeno(torch, gb, W, dev, sp, hbm):
     res["plain"] = {"glups": lups / (ms_p * 1e-3) / 1e9, "ms": ms_p, "bytes_per_lup": 56, "sweep_ms": tma_ms,
                     "kernel": "himeno_tma<plain>", "achieved_gbs": gbs, "frac_of_hbm": gbs / hbm,
                     "traffic": profiled_traffic("himeno_tma<plain>"),
-                    "ring_kernel_sweep_ms_dense_rows": ring_ms, "gosa_last": float(g_p[-1].item()),
+                    "flat_kernel_sweep_ms_dense_rows": ring_ms, "gosa_last": float(g_p[-1].item()),
                     "gosa_last_fp64": gosa64_last, "error_vs_fp64": err_p}
     b_m = (19 * 30 + 62) / 20.0
     res["mixed_fp16_defect_correction"] = {
@@ -986,8 +986,8 @@ def profile_small(name, torch, gb, W, dev, sp):
 
 def profile_case(name, local):
     """Short fixed launch sequences for ncu captures.
-    life:   16384^2 GameOfLife, 20 bit-packed generations (one life_bits_tb launch of 16 + 4
-            life_bits_sweep) then 20 u8 sweeps (life_u8_bulk)
+    life:   16384^2 GameOfLife, 32 bit-packed generations (two life_bits_tb launches of 16) then 20 u8
+            generations (bytes to words, two life_bits_tb launches of 10, words to bytes)
     himeno: 257x257x513 (rows padded to 264), 5 plain sweeps (himeno_tma<0>), 5 mixed sweeps
             (himeno_tma<1>, himeno_correct)
     fdtd:   512^3, 5 FP32 steps then 5 FP16 steps (star_r4_tma), then 2 two-step launches in FP32
@@ -1028,7 +1028,7 @@ def profile_case(name, local):
     ci = ctypes.c_int(0)
     sp = torch.cuda.current_stream(dev).cuda_stream
     gb.call("appfis_gb_life_pack", cells.data_ptr(), wa.data_ptr(), GOL_NX, GOL_NY, sp)
-    gb.call("appfis_gb_life_bits", wa.data_ptr(), wb.data_ptr(), GOL_NX, GOL_NY, 20, 0, ctypes.byref(ci), sp)
+    gb.call("appfis_gb_life_bits", wa.data_ptr(), wb.data_ptr(), GOL_NX, GOL_NY, 32, 0, ctypes.byref(ci), sp)
     gb.call("appfis_gb_life_u8", cells.data_ptr(), ub.data_ptr(), GOL_NX, GOL_NY, 20, 0, ctypes.byref(ci), sp)
     torch.cuda.synchronize(dev)
     print("profile case %s done" % name)

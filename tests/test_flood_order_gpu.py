@@ -73,3 +73,24 @@ def test_fields_do_not_depend_on_the_order(gb, torch_cuda, dtype, beside, flags,
         for a, b in zip(alone[k], batch[k]):
             assert torch_cuda.equal(a, b), k
     assert all(f[0].abs().sum() > 0 for f in batch)
+
+
+def test_capturing_stream_is_refused(gb, torch_cuda):
+    """A run copies tables from the caller's memory, which a graph could not replay: an error, and the
+    stream and the next run are none the worse."""
+    torch = torch_cuda
+    domains = [W.triton_domain(20, 30, 5)]
+    want, _ = _run(gb, torch, domains, _lib.F32, 0, False)
+    table, prm = (_lib.FloodDomain * 1)(), _lib.FloodParams(10.0, 0.5, 1e-3, 600.0, 600.0, 1.0, 0.0, STEPS)
+    f = torch.zeros((8, 22, 32), device="cuda")
+    table[0].nx, table[0].ny, table[0].pitch = 30, 20, 32
+    table[0].h[0], table[0].h[1], table[0].qx[0], table[0].qx[1], table[0].qy[0], table[0].qy[1] = [f[m].data_ptr() for m in range(6)]
+    table[0].dem, table[0].n2 = f[6].data_ptr(), f[7].data_ptr()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(_lib.AppfisError):
+            gb.call("appfis_gb_flood_run", table, 1, _lib.F32, ctypes.byref(prm), None, None, None, None, torch.cuda.current_stream().cuda_stream)
+    got, _ = _run(gb, torch, domains, _lib.F32, 0, False)
+    for a, b in zip(got[0], want[0]):
+        assert torch.equal(a, b)
