@@ -13,8 +13,9 @@
 // The byte-per-cell sweep (life_u8_bulk) stages its rows in shared memory with bulk copies; the
 // one-generation bit-packed sweep (life_bits_sweep) marches down a strip of rows per warp,
 // keeping the row above / at / below in registers and exchanging the words at lane boundaries
-// with warp shuffles.  Runs of 16 or more bit-packed generations use life_bits_tb, which
-// advances a tile held in shared memory by 16 generations per launch.
+// with warp shuffles.  Runs of 4 or more bit-packed generations, and byte runs that are worth the
+// conversion to words and back, use life_bits_tb, which advances a region held in registers by up to 16
+// generations per launch.
 #include "gb_common.cuh"
 #include "tma.cuh"
 
