@@ -150,13 +150,13 @@ __device__ __forceinline__ bool is_active(const Ctl* ctl, int cur, int d, const 
 // no step) into the other half, and resets dtbits[slot], which the steps around this one do not use.
 // Block 0 does it at the step's start, one thread per domain: nobody reads that half before the next
 // grid barrier (in one thread at the step's end, domain after domain, it held up every step:
-// about 1 us a domain).
+// about 1 us a domain).  A collapsed step is no business of its: the error word is read on the way out of
+// every grid barrier, and a CTA that is slow to leave the one before this step would see it and go
+// without its strips (DomCtl::collapsed).
 __device__ __forceinline__ void commit(Ctl* ctl, int cur, int slot, int d, bool active, double dt, const Params& p, double big)
 {
     const double t = ctl->simtime[cur][d];
     const int id = ctl->pid[cur][d], n = ctl->steps[cur][d];
-    // a collapsed (below 1e-9 of the step scale) or NaN time step stops the run
-    if (active && !(dt > 1e-9 * p.time_step)) atomicExch(&ctl->error, 2);
     const double st = active ? t + dt : t;
     if (active && p.dtlog) p.dtlog[(size_t)d * p.max_steps + n] = dt;
     ctl->simtime[1 - cur][d] = st;
@@ -366,7 +366,16 @@ template <class T>
 struct DomCtl {
     T dt[MAXD];
     unsigned char flags[MAXD];  // bit 0: state buffer b, bit 1: fix, bit 2: wants dt / runs phase B
+    int collapsed;              // a domain's time step has collapsed: this step is the run's last
 };
+
+// The end of a step in which a domain's time step has collapsed (below 1e-9 of the step scale, or NaN): the other
+// domains have taken it, nothing follows.  Every CTA finds the collapse by itself, from the same minima
+// and scalars, so all leave here, each after its own strips and without a barrier.
+__device__ __forceinline__ void end_collapsed(Ctl* ctl)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&ctl->error, 0, 2);
+}
 
 // The order of step n (the first step has none listed: as numbered).
 __device__ __forceinline__ const unsigned* step_order(const Params& p, int n)
@@ -468,6 +477,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     __shared__ Dom<T> doms[MAXD];
     __shared__ DomCtl<T> dc;
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
+    if (threadIdx.x == 0) dc.collapsed = 0;
     __syncthreads();
     const long long warp = first_place<T, ORDER>();
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -501,6 +511,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             const bool run = active && dt > 1e-9 * p.time_step;
             dc.dt[d] = (T)dt;
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (run ? 4 : 0));
+            if (active && !run) dc.collapsed = 1;  // below 1e-9 of the step scale, or NaN
             if (blockIdx.x == 0) commit(ctl, cur, 1 - cur, d, active, dt, p, big);
         }
         if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
@@ -524,6 +535,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             }
             if (ORDER) list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
+        if (dc.collapsed) return end_collapsed(ctl);
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
             ctl->ticketb[cur] = 0;
@@ -816,6 +828,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
         }
     }
     for (int k = threadIdx.x; k < p.ndom; k += blockDim.x) doms[k] = gdoms[k];
+    if (threadIdx.x == 0) dc.collapsed = 0;
     __syncthreads();
     const long long warp = first_place<T, ORDER>();
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -840,6 +853,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             const bool run = active && dt > 1e-9 * p.time_step;
             dc.dt[d] = (T)dt;
             dc.flags[d] = (unsigned char)((ctl->steps[cur][d] & 1) | (run ? 4 : 0));
+            if (active && !run) dc.collapsed = 1;  // below 1e-9 of the step scale, or NaN
             if (blockIdx.x == 0) commit(ctl, cur, (n + 2) % 3, d, active, dt, p, big);
         }
         if (!__syncthreads_or(active)) return;  // commit() has left the final scalars in both halves
@@ -863,6 +877,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
             }
             if (ORDER) list_strip(ctl, p, 1 - cur, s, dry, lane);
         });
+        if (dc.collapsed) return end_collapsed(ctl);
         if (!grid_barrier(ctl, p.spin_limit)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {  // next used two steps later, past a barrier
             ctl->ticketb[cur] = 0;
