@@ -13,15 +13,16 @@
 // second launch folds them in block order (a box of up to 4096 elements is one block and one
 // launch): fixed grid, fixed order, deterministic, and nothing kept between calls.
 // This part has 2 FP64 lanes per SM and clock, so FP32 elements are compared as floats, and summed
-// as two or three floats (FloatSum) that reach a double once per 16 or 64 elements: FP32 SUM of 200 x 190 x 180
-// 38 us with a double add and conversion per element, 11.7 so (MAX 38 -> 9.8); 514^3 547 -> 129 us.
-// Bound there by the index arithmetic (a third of the instructions) and HBM (5.1 TB/s MAX); FP64 by
-// its pipe (272 us at 514^3).  The input is never written.
+// as three floats in packed pairs (FloatSum) that reach a double once per 128 elements: FP32 SUM of 200 x 190 x 180
+// 38 us with a double add and conversion per element, 12.1 so (MAX 38 -> 10.2); 512^3 547 -> 135 us.
+// Bound there by the index arithmetic (a third of the instructions) and HBM (4.7 TB/s MAX); FP64 by
+// its pipe (272 us at 512^3).  The input is never written.
 #include <cfloat>
 #include <climits>
 #include <mutex>
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "gb_common.cuh"
 
 namespace {
@@ -71,43 +72,46 @@ __device__ __forceinline__ A block_reduce(A v, A neutral, A* sh)
     return v;
 }
 
-// a + b == sum + err exactly, |err| at most half a unit in the last place of sum (Knuth's two-sum).
+// a + b == sum + err exactly, |err| at most half a unit in the last place of sum (Knuth's two-sum); two at once.
 __device__ __forceinline__ float two_sum(float a, float b, float& err)
 {
     const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
     err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
     return s;
 }
+__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& err)
+{
+    namespace f2 = gb::f2;
+    const float2 s = f2::add(a, b), bb = f2::sub(s, a);
+    err = f2::add(f2::sub(a, f2::sub(s, bb)), f2::sub(b, bb));
+    return s;
+}
 
-// A thread's running sum of floats.  hi takes the element, mid what hi rounds off and (EXACT) lo what mid
-// rounds off.  EXACT: 64 elements reach the double within 2^-60 of their magnitude, so no more is
-// lost than by adding each to a double.  Otherwise 16 elements do within ~2^-47 of theirs, at half the
-// instructions: for boxes of 2^20 elements and more, where those errors, of either sign, come to
-// less than 2^-56 of the sum of magnitudes, under the rounding of the double tree that follows.
+// A thread's running sum of floats, in two lanes: hi takes the element, mid what hi rounds off and lo what mid
+// rounds off.  Of n elements of a lane (n <= 64) and the sum S of their magnitudes, mid holds at most n 2^-24 S and
+// lo n^2 2^-48 S, so only lo's own roundings are lost, at most n^3 2^-72 S <= 2^-54 S, whatever the values: less
+// than one rounding of a double sum, and 128 elements reach the thread's double in one addition.
 // Infinities, NaN and sums beyond the float range leave a component that is not finite: the thread
 // then starts again in doubles.
-template <bool EXACT>
 struct FloatSum {
-    static constexpr int BATCH = EXACT ? 64 : 16;
-    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
+    static constexpr int BATCH = 128;
+    float2 hi = {0.0f, 0.0f}, mid = {0.0f, 0.0f}, lo = {0.0f, 0.0f};
     double total = 0.0;
     bool finite = true;
-    __device__ __forceinline__ void add(float v)
+    __device__ __forceinline__ void add(float2 v)
     {
-        float e, r;
+        float2 e, r;
         hi = two_sum(hi, v, e);
-        if (EXACT) {
-            mid = two_sum(mid, e, r);
-            lo = __fadd_rn(lo, r);
-        } else {
-            mid = __fadd_rn(mid, e);
-        }
+        mid = two_sum(mid, e, r);
+        lo = gb::f2::add(lo, r);
     }
     __device__ __forceinline__ void flush()
     {
-        finite = finite && fabsf(hi) <= FLT_MAX && fabsf(mid) <= FLT_MAX;
-        total += (double)hi + (EXACT ? (double)mid + (double)lo : (double)mid);
-        hi = mid = lo = 0.0f;
+        float e, f, g;
+        const float h = two_sum(hi.x, hi.y, e), m = two_sum(two_sum(mid.x, mid.y, f), e, g);
+        finite = finite && fabsf(h) <= FLT_MAX && fabsf(m) <= FLT_MAX;
+        total += (double)h + ((double)m + (double)__fadd_rn(__fadd_rn(lo.x, lo.y), __fadd_rn(f, g)));
+        hi = mid = lo = make_float2(0.0f, 0.0f);
     }
 };
 
@@ -160,8 +164,7 @@ __device__ __forceinline__ void put_result(void* result, W w)
     *reinterpret_cast<W*>(result) = w;
 }
 
-// EXACT: see FloatSum (FP32 SUM only).
-template <class T, int OP, class Off, bool EXACT>
+template <class T, int OP, class Off>
 __global__ void __launch_bounds__(RED_THREADS, RED_PER_SM) reduce_part(const T* __restrict__ field, Box b, int px, size_t plane,
                                                           typename Wide<T>::type* __restrict__ partials, void* __restrict__ result)
 {
@@ -178,8 +181,7 @@ __global__ void __launch_bounds__(RED_THREADS, RED_PER_SM) reduce_part(const T* 
         c.to(b, e0, px, plane);
         size_t left = (b.n - e0 + stride - 1) / stride;  // this thread's elements
         if constexpr (std::is_same<T, float>::value && OP == APPFIS_GB_SUM) {
-            typedef FloatSum<EXACT> Sum;
-            Sum t;
+            FloatSum t;
             int m = 0;
             size_t q = left;
             for (; q >= U; q -= U) {
@@ -190,14 +192,14 @@ __global__ void __launch_bounds__(RED_THREADS, RED_PER_SM) reduce_part(const T* 
                     c.next(b);
                 }
 #pragma unroll
-                for (int u = 0; u < U; u++) t.add(x[u]);
-                if ((m += U) == Sum::BATCH) {
+                for (int u = 0; u < U; u += 2) t.add(make_float2(x[u], x[u + 1]));
+                if ((m += U) == FloatSum::BATCH) {
                     t.flush();
                     m = 0;
                 }
             }
             for (; q > 0; q--) {
-                t.add(__ldg(f + c.at));
+                t.add(make_float2(__ldg(f + c.at), 0.0f));
                 c.next(b);
             }
             t.flush();
@@ -285,10 +287,7 @@ int launch_op(const T* f, int px, int py, const int* x, int grid, void* partials
     Wd* part = reinterpret_cast<Wd*>(partials);
     // the last offset a cursor can reach: one stride past the box
     const bool small = (double)plane * (x[5] - x[4] + 2) + (double)b.step < 2147483647.0;
-    constexpr bool fsum = std::is_same<T, float>::value && OP == APPFIS_GB_SUM;
-    const bool exact = fsum && b.n < ((size_t)1 << 20);
-    auto kern = exact ? reduce_part<T, OP, int, fsum> : (small ? reduce_part<T, OP, int, false> : reduce_part<T, OP, long long, false>);
-    if (exact && !small) kern = reduce_part<T, OP, long long, fsum>;
+    auto kern = small ? reduce_part<T, OP, int> : reduce_part<T, OP, long long>;
     gb::launch(kern, grid, RED_THREADS, 0, st, f, b, px, plane, part, grid == 1 ? res : nullptr);
     if (grid > 1) gb::launch(reduce_fold<T, OP>, 1, RED_THREADS, 0, st, part, grid, res);
     return gb::launched("reduce");
