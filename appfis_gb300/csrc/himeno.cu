@@ -24,6 +24,7 @@
 // per thread) when the FP16 rows are 16-byte aligned, else (and on small grids without gosa) himeno_flat.
 #include <cuda_fp16.h>
 
+#include <cfloat>
 #include <type_traits>
 
 #include "gb_common.cuh"
@@ -126,28 +127,46 @@ struct SqAcc {
 };
 
 // The end of a flat sweep's block: as gosa_end, for kernels whose threads have only a few points each.
-// The warps add their threads' two-float sums as such (relative error under 2^-45 for these
-// positive terms) and one warp takes the warps' sums to double: a double shuffle tree per warp costs
-// 8 FP64 instructions of 16 cycles each on this part, more than the sweep itself at few planes per
-// thread (65 x 65 x 129: see himeno_flat).
+// The warps add their threads' two-float sums in three floats (every rounding of hi and of mid is kept: what lo rounds
+// off is under 2^-65 of these positive terms' sum), and one warp takes the warps' sums to double: a double
+// shuffle tree per warp costs 8 FP64 instructions of 16 cycles each on this part, more than the sweep itself at
+// few planes per thread (65 x 65 x 129, us per sweep: 8.25, so 6.0).  Sums beyond the float range take it.
+__device__ __forceinline__ float two_sum(float a, float b, float& err)
+{
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+
 __device__ __forceinline__ void gosa_end_flat(const SqAcc& acc, const GosaIO& g, unsigned block)
 {
     if (g.part) {
-        __shared__ float2 sh[32];
-        float hi = acc.hi, lo = acc.lo;
+        __shared__ float4 sh[8];  // hi, mid, lo, whether they hold the sum
+        __shared__ double wide[8];
+        float hi = acc.hi, mid = acc.lo, lo = 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            const float h2 = __shfl_down_sync(0xffffffffu, hi, o), l2 = __shfl_down_sync(0xffffffffu, lo, o);
-            const float s = __fadd_rn(hi, h2), bb = __fsub_rn(s, hi);
-            const float e = __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(h2, bb)), __fadd_rn(lo, l2));
-            hi = __fadd_rn(s, e);
-            lo = __fsub_rn(e, __fsub_rn(hi, s));
+            const float h2 = __shfl_down_sync(0xffffffffu, hi, o), m2 = __shfl_down_sync(0xffffffffu, mid, o);
+            const float l2 = __shfl_down_sync(0xffffffffu, lo, o);
+            float e, f, r;
+            hi = two_sum(hi, h2, e);
+            mid = two_sum(mid, m2, f);
+            mid = two_sum(mid, e, r);
+            lo = __fadd_rn(__fadd_rn(lo, l2), __fadd_rn(f, r));
         }
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_float2(hi, lo);
+        const int w = threadIdx.x >> 5;
+        const bool held = fabsf(hi) <= FLT_MAX && fabsf(mid) <= FLT_MAX;
+        if (!__shfl_sync(0xffffffffu, held, 0)) {
+            double v = acc.value();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if ((threadIdx.x & 31) == 0) wide[w] = v;
+        }
+        if ((threadIdx.x & 31) == 0) sh[w] = make_float4(hi, mid, lo, held ? 1.0f : 0.0f);
         __syncthreads();
         if (threadIdx.x < 32) {
-            const float2 w = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : make_float2(0.0f, 0.0f);
-            double v = (double)w.x + (double)w.y;
+            const float4 q = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+            double v = q.w != 0.0f ? (double)q.x + ((double)q.y + (double)q.z) : wide[threadIdx.x];
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);  // at most 8 warps
             if (threadIdx.x == 0) g.part[block] = v;
