@@ -197,9 +197,9 @@ __global__ void __launch_bounds__(256) himeno_finish(const float* __restrict__ P
                                                      int ny, int nz, int px, unsigned plane_blocks)
 {
     const gb::BlockId bid = gb::grid_wait();
-    const unsigned zc = bid.x / plane_blocks;
+    const unsigned zc = bid.x / plane_blocks, w = (unsigned)nx + 2;
     const size_t q = (size_t)(bid.x - zc * plane_blocks) * 256 + threadIdx.x;
-    const int j = 1 + (int)(q / (unsigned)px), i = (int)(q - (size_t)(j - 1) * px), k0 = 1 + (int)zc * FINISH_K;
+    const int j = 1 + (int)(q / w), i = (int)(q - (size_t)(j - 1) * w), k0 = 1 + (int)zc * FINISH_K;
     if (i < 1 || i > nx || j > ny) return;
     const size_t plane = (size_t)px * (ny + 2), c = (size_t)k0 * plane + (size_t)j * px + i;
     float v[FINISH_K], d[FINISH_K];
@@ -257,9 +257,10 @@ __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float*
 
 // ---------------------------------------------------------------- flat form
 // One column of FK planes per thread, the columns of a plane numbered along its rows (ghost columns
-// and padding included, so a warp reads consecutive addresses whatever the row length); neighbours
-// come through L1.  Going up a column, the five values of plane k+1 that plane k needs serve again as
-// plane k+1's own, so a point costs 9 loads of the field and 12 of the coefficients.
+// included, so a warp reads consecutive addresses whatever the row length; the padding of a row not: rows of 30
+// at a pitch of 4096 185 us a sweep with it, 16.6 without, and at pitches close to the row as fast or
+// faster); neighbours come through L1.  Going up a column, the five values of plane k+1 that plane k needs
+// serve again as plane k+1's own, so a point costs 9 loads of the field and 12 of the coefficients.
 //
 // It is the form for rows that are not 16-byte aligned, and for grids too small to give every SM the
 // long z-march of the TMA-staged forms.  Us per sweep against a 2.5-D march with a shared-memory plane
@@ -288,16 +289,16 @@ __global__ void __launch_bounds__(FT, 4) himeno_flat(Coef12 cf, H10 hf, const vo
     const gb::BlockId bid = gb::grid_wait();
     typedef typename std::conditional<MODE == 0, float, __half>::type L;
     const L* __restrict__ f = reinterpret_cast<const L*>(pin);
-    const unsigned zc = bid.x / plane_blocks, pb = bid.x - zc * plane_blocks;
+    const unsigned zc = bid.x / plane_blocks, pb = bid.x - zc * plane_blocks, w = (unsigned)nx + 2;
     unsigned row, col;
-    if (plane_blocks < 1u << 24) {  // uniform: a plane of fewer than 2^32 elements
+    if (plane_blocks < 1u << 24) {  // uniform: a plane of fewer than 2^32 columns
         const unsigned q = pb * FT + threadIdx.x;
-        row = q / (unsigned)px;
-        col = q - row * (unsigned)px;
+        row = q / w;
+        col = q - row * w;
     } else {
         const size_t q = (size_t)pb * FT + threadIdx.x;
-        row = (unsigned)(q / (unsigned)px);
-        col = (unsigned)(q - (size_t)row * px);
+        row = (unsigned)(q / w);
+        col = (unsigned)(q - (size_t)row * w);
     }
     const int i = (int)col, j = 1 + (int)row, k0 = 1 + (int)zc * FK;
     const size_t plane = (size_t)px * (ny + 2);
@@ -388,9 +389,9 @@ template <int MODE>
 struct FlatPlan {
     decltype(&himeno_flat<MODE, 4>) kernel;
     unsigned plane_blocks, blocks;
-    FlatPlan(int ny, int nz, int pitch)
+    FlatPlan(int nx, int ny, int nz)
     {
-        plane_blocks = gb::ceil_div((size_t)ny * pitch, FT);
+        plane_blocks = gb::ceil_div((size_t)ny * (nx + 2), FT);
         auto grid = [&](int fk) { return (size_t)plane_blocks * ((nz + fk - 1) / fk); };
         const size_t sms = gb::sm_count();
         const int fk = grid(8) >= 10 * sms ? 8 : (grid(4) >= 2 * sms ? 4 : 2);
@@ -1109,7 +1110,7 @@ int appfis_gb_himeno(const float* const* coef, float* p, float* wrk2, int nx, in
     int ci = 0;
     // the flat sweep below ~6 M points or without 16-byte rows (measured lines at himeno_flat)
     if (!plain_tma_ok(coef, p, wrk2, pitch) || (size_t)nx * ny * nz <= FLAT_POINTS) {
-        const FlatPlan<0> fp(ny, nz, pitch);
+        const FlatPlan<0> fp(nx, ny, nz);
         const dim3 fgrd(fp.blocks);
         GB_TRY(gs.init(dev_gosa, fgrd.x, 1));
         H10 none = {};
@@ -1273,8 +1274,8 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     // its squares in single floats: a better sum would be another one, in the ninth digit).  Us per sweep,
     // staged / flat: 65 x 65 x 129 26 / 6.2, 100 x 100 x 200 29 / 21, 129 x 129 x 257 35.9 / 35.9, 160 x 160 x 300 46 / 60
     const bool flat = !use_tma || (!dev_gosa && !two && (size_t)nx * ny * nz <= FLAT_MIXED_POINTS);
-    const FlatPlan<1> aligned_plan(ny, nz, pitch);
-    const FlatPlan<2> fplan(ny, nz, pitch);
+    const FlatPlan<1> aligned_plan(nx, ny, nz);
+    const FlatPlan<2> fplan(nx, ny, nz);
     auto fkern = use_tma ? aligned_plan.kernel : fplan.kernel;
     const dim3 fgrd(fplan.blocks);
     GosaSeq gs;  // block sums of the sweeps and of the correction passes (which do a sweep each)
@@ -1340,7 +1341,7 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
         }
     }
     GB_TRY(gs.flush(st));
-    const unsigned fpb = gb::ceil_div((size_t)ny * pitch, 256);
+    const unsigned fpb = gb::ceil_div((size_t)ny * (nx + 2), 256);
     gb::launch(himeno_finish, fpb * ((nz + FINISH_K - 1) / FINISH_K), 256, 0, st, P[pc], E[ec], P[1 - pc], nx, ny, nz, pitch, fpb);
     pc = 1 - pc;
     GB_TRY(gb::launched("himeno_mixed"));
