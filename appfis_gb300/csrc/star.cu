@@ -1166,9 +1166,15 @@ int run_star(T* a, T* b, int nx, int ny, int nz, int pitch, int iters, int mode,
     //   250 x 127 x 130 18.1 / 15.6, 18.0; 250^3 71 / 57 (odd); 506^3 467 / 358, 433; 20 x 500 x 500 32 / 35, 52
     //   FP16 100^3 6.7 / 8.2; 130 x 140 x 150 15.3 / 13.0; 250 x 127 x 130 (258) 18.8 / 12.5; 500^3 466 / 277
     // (with the rows 16-byte aligned the TMA-staged tile takes 11.9 for 250 x 127 x 130, 206 for 512^3)
+    // Its ring is filled with 8 planes before the first is computed, so a flat grid is the smaller tiles': 3000 x 3000 x
+    //   1 / 2 / 4 / 8 / 12 / 16 planes FP32 86 / 116 / 176 / 300 / 423 / 547 against 135 / 157 / 204 / 296 / 385 / 470 (even),
+    //   136 / 159 / 209 / 318 / 425 / 527 (odd); FP16 1500 x 1500 x 1 / 2 16.7 / 26.5 against 17.9 / 21.4
+    // and rows whose odd FP32 words it copies for a third more columns than the scalar tile: 90 x 700 x 120 35 against 40
     const unsigned long long align = (unsigned long long)pitch * sizeof(T) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b);
     const bool one_word = sizeof(T) == 4 && align % 8 != 0;
-    const bool async = tile == APPFIS_GB_STAR_AUTO && !rows16 && align % 4 == 0 && 2 * nx >= 64 * (int)gb::ceil_div(nx, 64) &&
+    const size_t cols = (size_t)64 * gb::ceil_div(nx, 64), scalar_cols = (size_t)TX * gb::ceil_div(nx, TX);
+    const bool fills = 2 * (size_t)nx >= cols && nz >= (sizeof(T) == 2 ? 2 : one_word ? 16 : 8) && (!one_word || 4 * cols <= 5 * scalar_cols);
+    const bool async = tile == APPFIS_GB_STAR_AUTO && !rows16 && align % 4 == 0 && fills &&
                        (size_t)nx * ny * nz >= (one_word ? (size_t)4000000 : (size_t)2000000);
     if (tile == APPFIS_GB_STAR_AUTO && !async) tile = rows16 ? APPFIS_GB_STAR_TMA_X4 : (vec4 ? APPFIS_GB_STAR_VEC : APPFIS_GB_STAR_SCALAR2);
     if ((tile == APPFIS_GB_STAR_TMA_X4 || tile == APPFIS_GB_STAR_TMA_X2 || tile == APPFIS_GB_STAR_TB2 || tile == APPFIS_GB_STAR_TB2_8 ||
