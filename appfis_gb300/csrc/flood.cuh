@@ -886,7 +886,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FLOOD_F32_MIN_BLOCKS : 1
     }
 }
 
-static __global__ void flood_init_ctl(Ctl* ctl, int ndom, double big, double t0)
+template <class T>
+struct Table {
+    Dom<T> d[MAXD];
+};
+
+// The control block's first state, and the domain table, which comes as an argument (5.6 KB) and so needs no copy.
+template <class T>
+__global__ void flood_init_ctl(Ctl* ctl, Dom<T>* doms, const __grid_constant__ Table<T> table, int ndom, double big, double t0)
 {
     gb::grid_wait();
     const int d = threadIdx.x;  // one block
@@ -899,6 +906,7 @@ static __global__ void flood_init_ctl(Ctl* ctl, int ndom, double big, double t0)
         ctl->wet[0] = ctl->wet[1] = ctl->dry[0] = ctl->dry[1] = 0;
     }
     if (d < ndom) {
+        doms[d] = table.d[d];
         ctl->src_lo[d] = 0;
         ctl->dtbits[2][d] = (unsigned long long)__double_as_longlong(big);
         for (int k = 0; k < 2; k++) {

@@ -2,6 +2,7 @@
 // host-buffer job (upload + padding, run, mass, download).  Included once per precision.
 #pragma once
 
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -161,7 +162,7 @@ inline int upload_sources(const appfis_gb_flood_domain* doms, const appfis_gb_fl
         std::memcpy(dv + od, S.flows, sizeof(double) * S.nt * S.n);
         od += (size_t)S.nt * S.n;
     }
-    GB_CUDA(cudaMemcpyAsync(dev, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+    GB_TRY(gb::upload(dev, host.data(), host.size(), st));
     *out = reinterpret_cast<const SrcDev*>(dev);
     return APPFIS_GB_OK;
 }
@@ -256,12 +257,10 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
     GB_TRY(gb::workspace(gb::WS_REDUCE, sizeof(Ctl) + sizeof(Dom<T>) * MAXD + 256, &wt));
     Ctl* ctl = reinterpret_cast<Ctl*>(wt);
     Dom<T>* dtab = reinterpret_cast<Dom<T>*>(reinterpret_cast<char*>(wt) + ((sizeof(Ctl) + 255) / 256) * 256);
-    // this table, the sources' and the tensor maps come from pageable memory, which such a copy has read when it
-    // returns: the host goes on while earlier work of the stream runs (100^2, 20 steps
-    // 272 -> 257 us; six domains of 3.6 M cells 1270 -> 1250)
-    GB_CUDA(cudaMemcpyAsync(dtab, tab.data(), sizeof(Dom<T>) * ndom, cudaMemcpyHostToDevice, st));
+    Table<T> table;
+    std::copy(tab.begin(), tab.end(), table.d);
     const double big = std::is_same<T, float>::value ? 3.402823466e38 : 1.7976931348623157e308;
-    gb::launch(flood_init_ctl, 1, MAXD, 0, st, ctl, ndom, big, prm->t_start);
+    gb::launch(flood_init_ctl<T>, 1, MAXD, 0, st, ctl, dtab, table, ndom, big, prm->t_start);
     GB_TRY(gb::launched("flood_init_ctl"));
 
     Params p;
@@ -298,7 +297,7 @@ int run(const appfis_gb_flood_domain* doms, int ndom, const appfis_gb_flood_para
         }
         void* dm;
         GB_TRY(gb::workspace(gb::WS_FLOOD_MAPS, sizeof(CUtensorMap) * maps.size(), &dm));
-        GB_CUDA(cudaMemcpyAsync(dm, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, st));
+        GB_TRY(gb::upload(dm, maps.data(), sizeof(CUtensorMap) * maps.size(), st));
         p.maps = reinterpret_cast<const CUtensorMap*>(dm);
         unsigned long long test_ns = 0;
         if (gb::take_test_stall(gb::TEST_TMA_SHORTFALL, &test_ns)) {  // a test runs the first stage's waits out

@@ -76,8 +76,11 @@ bool scratch_alloc(size_t bytes, cudaStream_t st, void** out);
 void scratch_free(void* p, cudaStream_t st);
 // True while `st` records a graph (or cannot tell): a call then allocates nothing of its own.
 bool capturing(cudaStream_t st);
-// Pinned host staging buffer, grow-only, per slot (0..1).
-int pinned(int slot, size_t bytes, void** out);
+// Copies a host table to the device on `st`; the source may go as soon as it returns, and the host does not wait
+// for earlier work of the stream.  Through pinned memory of the library's own: whether a copy from
+// pageable memory has been read when the call returns is the platform's choice, and one whose GPU reads pageable
+// memory itself need not have.  Up to 6 copies a device are under way, then the oldest is waited for.
+int upload(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
 inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 

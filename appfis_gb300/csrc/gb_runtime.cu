@@ -3,6 +3,7 @@
 // The reference keeps one CUDA stream in a singleton (Appfis/Topology.hpp:104-151) and ignores
 // CUDA return codes after initialisation; here every call returns a status and the message of
 // the last failure is kept per host thread.
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -56,11 +57,23 @@ struct Buf {
 };
 std::mutex g_mu;
 std::vector<std::vector<Buf>> g_dev;  // [device][slot]
-Buf g_pinned[2];
 std::vector<int> g_sms;
 std::vector<unsigned*> g_status;  // [device]
 std::vector<cudaStream_t> g_job_streams;  // [device]
 std::vector<cudaMemPool_t> g_pools;  // [device]
+// Pinned staging of upload(): a device's buffers in turn, each free again once its event has passed.
+constexpr int STAGES = 6;
+struct Stage {
+    void* p = nullptr;
+    size_t n = 0;
+    cudaEvent_t copied = nullptr;
+};
+struct StageRing {
+    Stage stage[STAGES];
+    unsigned next = 0;
+};
+std::mutex g_stage_mu;
+std::vector<StageRing> g_stage;  // [device]
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 std::once_flag g_encode_once;
 }  // namespace
@@ -131,22 +144,29 @@ bool capturing(cudaStream_t st)
     return true;
 }
 
-int pinned(int slot, size_t bytes, void** out)
+int upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
 {
-    if (slot < 0 || slot > 1) return fail(APPFIS_GB_EINVAL, "pinned slot %d", slot);
-    std::lock_guard<std::mutex> lk(g_mu);
-    Buf& b = g_pinned[slot];
-    if (b.n < bytes) {
-        if (b.p) {
-            cudaFreeHost(b.p);
-            b.p = nullptr;
-            b.n = 0;
-        }
-        GB_TRY(cuda_status(cudaMallocHost(&b.p, bytes), "cudaMallocHost(staging)"));
-        b.n = bytes;
+    int dev = 0;
+    GB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if ((int)g_stage.size() <= dev) g_stage.resize(dev + 1);
+    StageRing& ring = g_stage[dev];
+    Stage& s = ring.stage[ring.next++ % STAGES];
+    if (!s.copied) GB_CUDA(cudaEventCreateWithFlags(&s.copied, cudaEventDisableTiming));
+    GB_CUDA(cudaEventSynchronize(s.copied));  // its last copy has been made (or none was)
+    if (s.n < bytes) {
+        if (s.p) cudaFreeHost(s.p);
+        s.p = nullptr;
+        s.n = 0;
+        const size_t want = bytes < (64u << 10) ? 64u << 10 : bytes;
+        GB_TRY(cuda_status(cudaMallocHost(&s.p, want), "cudaMallocHost(staging)"));
+        s.n = want;
     }
-    *out = b.p;
-    return APPFIS_GB_OK;
+    std::memcpy(s.p, src, bytes);
+    GB_CUDA(cudaMemcpyAsync(dst, s.p, bytes, cudaMemcpyHostToDevice, st));
+    const cudaError_t e = cudaEventRecord(s.copied, st);
+    if (e != cudaSuccess) cudaStreamSynchronize(st);
+    return cuda_status(e, "cudaEventRecord(staging)");
 }
 
 int sm_count()
