@@ -50,7 +50,7 @@ __global__ void flood_extract(Dom<T> D, int b, double* __restrict__ h, double* _
     qy[o] = (double)D.qy[b][c];
 }
 
-static __global__ void flood_results(const Ctl* __restrict__ ctl, int ndom, int* steps, double* simtime, int* status)
+static __global__ void flood_results(const Ctl* ctl, int ndom, int* steps, double* simtime, int* status)
 {
     gb::grid_wait();
     const int d = threadIdx.x;

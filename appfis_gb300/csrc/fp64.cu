@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(NT) himeno_f64(CoefF64 cf, const double* __res
 }
 
 // One block folds n partials: each thread a contiguous run in order, then the runs in thread order.
-__global__ void __launch_bounds__(1024) fold_f64(const double* __restrict__ part, size_t n, double* __restrict__ out)
+__global__ void __launch_bounds__(1024) fold_f64(const double* part, size_t n, double* out)
 {
     gb::grid_wait();
     __shared__ double sh[1024];

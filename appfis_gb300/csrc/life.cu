@@ -672,7 +672,7 @@ __global__ void popcount_words(const uint32_t* __restrict__ words, size_t n, uns
 }
 
 // tail of a byte array whose length is not a multiple of 4
-__global__ void popcount_tail(const uint8_t* __restrict__ p, int n, unsigned long long* __restrict__ out)
+__global__ void popcount_tail(const uint8_t* p, int n, unsigned long long* out)
 {
     gb::grid_wait();
     unsigned long long s = 0;

@@ -248,15 +248,14 @@ __global__ void __launch_bounds__(RED_THREADS, RED_PER_SM) reduce_part(const T* 
 }
 
 template <class T, int OP>
-__global__ void __launch_bounds__(RED_THREADS) reduce_fold(const typename Wide<T>::type* __restrict__ partials, int n, void* __restrict__ result)
+__global__ void __launch_bounds__(RED_THREADS) reduce_fold(const typename Wide<T>::type* partials, int n, void* result)
 {
     gb::grid_wait();
     typedef typename Wide<T>::type Wd;
     __shared__ Wd sh[32];
-    const volatile Wd* part = partials;  // written by the launch before: read behind the wait
     const Wd neutral = (Wd)seed<T, OP>();
     Wd v = neutral;
-    for (int k = threadIdx.x; k < n; k += RED_THREADS) v = combine<OP>(v, (Wd)part[k]);
+    for (int k = threadIdx.x; k < n; k += RED_THREADS) v = combine<OP>(v, partials[k]);
     v = block_reduce<OP>(v, neutral, sh);
     if (threadIdx.x == 0) put_result(result, v);
 }
