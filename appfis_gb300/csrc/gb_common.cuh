@@ -70,6 +70,8 @@ enum Slot { WS_REDUCE = 0, WS_JOB_A, WS_JOB_B, WS_JOB_C, WS_JOB_D, WS_JOB_E, WS_
 int workspace(int slot, size_t bytes, void** out);
 // True if that slot holds at least `bytes` already, so that workspace() will not allocate.
 bool workspace_holds(int slot, size_t bytes);
+// Gives that slot's memory back.
+void workspace_drop(int slot);
 // Device memory for one call, ordered on `st` (allocated and freed by the stream, so calls on other
 // streams and threads never share it): from a pool per device that keeps up to 256 MB between
 // calls and gives back what is over that when the device is next synchronised.  False, with no error

@@ -109,6 +109,16 @@ bool workspace_holds(int slot, size_t bytes)
     return (int)g_dev.size() > dev && g_dev[dev][slot].n >= bytes;
 }
 
+void workspace_drop(int slot)
+{
+    int dev = 0;
+    if (slot < 0 || slot >= WS_SLOTS || cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> lk(g_mu);
+    if ((int)g_dev.size() <= dev || !g_dev[dev][slot].p) return;
+    cudaFree(g_dev[dev][slot].p);
+    g_dev[dev][slot] = Buf();
+}
+
 bool scratch_alloc(size_t bytes, cudaStream_t st, void** out)
 {
     int dev = 0;

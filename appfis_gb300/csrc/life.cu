@@ -864,16 +864,22 @@ int run_bits(uint32_t* buf[2], int nx, int ny, int gens, int* cur_index, cudaStr
     if (cur_index) *cur_index = ci;
     if (gens >= TB_STEPS) {
         // the long runs' pairs stay in the workspace, so that a run can be recorded in a graph after a
-        // first one has sized them; a recording that would need more takes one more, shorter, launch
+        // first one has sized them; a recording that would need more, or a full device, takes one more, shorter,
+        // launch and no third pair
         int launches = std::max(2, (gens + TB_STEPS - 1) / TB_STEPS);
         void *wc, *wd, *we = nullptr, *wf = nullptr;
         GB_TRY(gb::workspace(gb::WS_LIFE_C, bytes, &wc));
         GB_TRY(gb::workspace(gb::WS_LIFE_D, bytes, &wd));
-        if (launches % 2 && gb::capturing(st) && !(gb::workspace_holds(gb::WS_LIFE_E, bytes) && gb::workspace_holds(gb::WS_LIFE_F, bytes)))
-            launches++;
         if (launches % 2) {
-            GB_TRY(gb::workspace(gb::WS_LIFE_E, bytes, &we));
-            GB_TRY(gb::workspace(gb::WS_LIFE_F, bytes, &wf));
+            const bool held = gb::workspace_holds(gb::WS_LIFE_E, bytes) && gb::workspace_holds(gb::WS_LIFE_F, bytes);
+            int rc = !held && gb::capturing(st) ? (int)APPFIS_GB_ENOMEM : gb::workspace(gb::WS_LIFE_E, bytes, &we);
+            if (rc == APPFIS_GB_OK && (rc = gb::workspace(gb::WS_LIFE_F, bytes, &wf)) == APPFIS_GB_ENOMEM) gb::workspace_drop(gb::WS_LIFE_E);
+            if (rc == APPFIS_GB_ENOMEM) {
+                launches++;
+                we = wf = nullptr;
+            } else if (rc != APPFIS_GB_OK) {
+                return rc;
+            }
         }
         const TbPair pair[3] = {own, {{(uint32_t*)wc, (uint32_t*)wd}}, {{(uint32_t*)we, (uint32_t*)wf}}};
         return run_tb<RULE>(pair, last, nx, ny, gens, launches, st);
