@@ -119,8 +119,8 @@ struct FloatSum {
 // all threads moves a position by.
 struct Box {
     size_t first, n;          // elements
-    int W, ny;                // row length, rows per plane
-    int dcol, drow;           // the stride's columns, rows within a plane
+    unsigned W, ny;           // row length, rows per plane
+    unsigned dcol, drow;      // the stride's columns, rows within a plane
     long long step;           // and as an element offset
     long long row_end, plane_end;  // offsets added when a row or a plane is passed
 };
@@ -129,12 +129,12 @@ struct Box {
 template <class Off>
 struct Cursor {
     Off at;
-    int col, row;
+    unsigned col, row;  // their sums with the stride's may pass 2^31
     __device__ __forceinline__ void to(const Box& b, size_t e, int px, size_t plane)
     {
-        const size_t r = e / (unsigned)b.W, k = r / (unsigned)b.ny;
-        col = (int)(e - r * b.W);
-        row = (int)(r - k * b.ny);
+        const size_t r = e / b.W, k = r / b.ny;
+        col = (unsigned)(e - r * b.W);
+        row = (unsigned)(r - k * b.ny);
         at = (Off)(k * plane + (size_t)row * px + col);
     }
     __device__ __forceinline__ void next(const Box& b)
@@ -277,10 +277,10 @@ int launch_op(const T* f, int px, int py, const int* x, int grid, void* partials
     b.first = x[4] * plane + (size_t)x[2] * px + x[0];
     b.n = (size_t)b.W * b.ny * (x[5] - x[4]);
     const size_t stride = (size_t)grid * RED_THREADS, srow = stride / b.W;
-    b.dcol = (int)(stride % b.W);
-    b.drow = (int)(srow % b.ny);
+    b.dcol = (unsigned)(stride % b.W);
+    b.drow = (unsigned)(srow % b.ny);
     b.step = (long long)(srow / b.ny * plane) + (long long)b.drow * px + b.dcol;
-    b.row_end = px - b.W;
+    b.row_end = px - (long long)b.W;
     b.plane_end = (long long)plane - (long long)b.ny * px;
     typedef typename Wide<T>::type Wd;
     Wd* part = reinterpret_cast<Wd*>(partials);
