@@ -216,6 +216,11 @@ __global__ void __launch_bounds__(256) himeno_finish(const float* __restrict__ P
 
 // Correction pass: P' = P + e, D = omega*ss(P'), and the sweep after it, e = D.  Reads P and e at neighbours.  COPY (the first
 // pass of a run): also leaves the ten coefficients it has read in FP16, in the fields at `copy`.
+// Rows that are not 16-byte aligned (else himeno_correct_tma).  Bound by latency on small grids, by HBM and L1 on large ones
+// (257 x 257 x 513: 0.75 of the copy rate).  Nothing is kept from plane to plane, so a CTA takes only CKZ = 6 of them,
+// and a point's coefficients are asked for before its sums.  Us per pass with 32 planes / 6 / 6 and the
+// coefficients first: 33 x 33 x 65 42 / 10 / 5.8; 65 x 65 x 129 47 / 12 / 9.4; 129 x 129 x 257 115 / 74 / 59; 257 x 257 x 513 498 / 496 / 414;
+// so with 2 / 4 / 8 / 16 planes: 65 x 65 x 129 8.7 / 9.7 / 9.9 / 14.0, with gosa 13.3 / 10.9 / 11.3 / 15.3; 257 x 257 x 513 434 / 418 / 415 / 422.
 template <int BX, int BY, bool COPY>
 __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float* __restrict__ P, const __half* __restrict__ e,
                                                           float* __restrict__ Pn, __half* __restrict__ D,
@@ -234,18 +239,19 @@ __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float*
 #define QF(di, dj, dk)                                                                                      \
     (__ldg(P + c + (ptrdiff_t)(di) + (ptrdiff_t)(dj) * px + (ptrdiff_t)(dk) * (ptrdiff_t)plane) +          \
      __half2float(e[c + (ptrdiff_t)(di) + (ptrdiff_t)(dj) * px + (ptrdiff_t)(dk) * (ptrdiff_t)plane]))
+        float co[12];
+#pragma unroll
+        for (int n = 0; n < 12; n++) co[n] = __ldg(cf.c[n] + c);
         const float q0 = QF(0, 0, 0);
-        const float s0 = HIMENO_S0(QF, __ldg(cf.c[0] + c), __ldg(cf.c[1] + c), __ldg(cf.c[2] + c), __ldg(cf.c[4] + c),
-                                   __ldg(cf.c[5] + c), __ldg(cf.c[6] + c), __ldg(cf.c[7] + c), __ldg(cf.c[8] + c),
-                                   __ldg(cf.c[9] + c), __ldg(cf.c[11] + c));
+        const float s0 = HIMENO_S0(QF, co[0], co[1], co[2], co[4], co[5], co[6], co[7], co[8], co[9], co[11]);
 #undef QF
-        const float ss = (s0 * __ldg(cf.c[3] + c) - q0) * __ldg(cf.c[10] + c);
+        const float ss = (s0 * co[3] - q0) * co[10];
         const __half dh = __float2half_rn(omega * ss);
         Pn[c] = q0;
         D[c] = dh;
         if (COPY) {
 #pragma unroll
-            for (int n = 0; n < 10; n++) copy[n * field + c] = __float2half_rn(__ldg(cf.c[half_of(n)] + c));
+            for (int n = 0; n < 10; n++) copy[n * field + c] = __float2half_rn(co[half_of(n)]);
         }
         enext[c] = dh;  // the next sweep from e = 0 gives e = D exactly, with ss = D / omega
         const float s1 = __half2float(dh) * inv_omega;
@@ -1015,8 +1021,8 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
     gosa_end<1>({k < k1 ? __longlong_as_double(0x7ff8000000000000ll) : (double)g}, gz);
 }
 
-// HKZ: z planes per CTA (nz is split into equal chunks of at most HKZ planes)
-constexpr int HBX = 32, HBY = 4, HKZ = 32;
+constexpr int HBX = 32, HBY = 4, CKZ = 6;  // himeno_correct: threads and z planes per CTA
+constexpr int HKZ = 32;  // z planes per CTA elsewhere (nz is split into equal chunks of at most HKZ planes)
 constexpr int TMA_S_PLAIN = 3;
 constexpr size_t FLAT_POINTS = 6000000;        // grids up to this take the flat FP32 sweep
 constexpr size_t FLAT_MIXED_POINTS = 3000000;  // ... and the flat FP16 sweep where no gosa is asked for
@@ -1188,7 +1194,7 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     if (sweeps_per_pass == 2) GB_CUDA(cudaMemsetAsync(hw, 0, sizeof(__half) * 13 * field, st));
     else GB_CUDA(cudaMemsetAsync(E[0], 0, sizeof(__half) * 2 * field, st));
     GB_CUDA(cudaMemsetAsync(p_work, 0, sizeof(float) * field, st));
-    dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, HKZ));
+    dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, CKZ));
     dim3 rblk(RX, RY);
     // TMA-staged inner sweeps (two points per thread) when the FP16 rows are 16-byte aligned
     // (pitch a multiple of 8)
@@ -1312,7 +1318,7 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
                        Dd, E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, ckz, omega, inv_omega, gz, status);
         else
             gb::launch(first ? himeno_correct<HBX, HBY, true> : himeno_correct<HBX, HBY, false>, grd, blk, 0, st, cf, P[pc], E[ec], P[1 - pc], Dd,
-                       E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, HKZ, omega, inv_omega, gz);
+                       E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, CKZ, omega, inv_omega, gz);
         first = false;
         pc = 1 - pc;
         ec = 1 - ec;
