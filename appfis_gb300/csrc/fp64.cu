@@ -14,7 +14,7 @@
 // their rows and dealt to threads in that order, so every lane has a point whatever the row length (a
 // 32-wide block left a quarter of them idle at nx = 65), and nothing that can be done exactly in
 // integers is done in FP64.  Neighbours come through the read-only cache.  G points/s before and now: heat
-// 1000 x 777 45.4 / 57.5 (8 FP64 instructions a point), Himeno 65 x 65 x 129 7.1 / 11.1 with gosa, 8.3 / 12.9
+// 1000 x 777 45.4 / 57.5 (8 FP64 instructions a point), Himeno 65 x 65 x 129 7.1 / 11.6 with gosa, 8.3 / 13.9
 // without, 257 x 257 x 129 11.6 / 14.4, star 100^3 15.1 / 19.7, 255 x 256 x 200 18.0 / 18.1.
 #include "gb_common.cuh"
 
@@ -65,13 +65,12 @@ struct CoefF64 {
     const double* f[12];  // a0 a1 a2 a3 b0 b1 b2 c0 c1 c2 bnd wrk1
 };
 
-// Himeno/src/himeno_appfis.hpp:178-198 in double, HK planes per thread; ss^2 summed per thread and block
+// Himeno/src/himeno_appfis.hpp:178-198 in double, hk planes per thread; ss^2 summed per thread and block
 // (fixed order) where gosa is asked for, the block partials folded in block order by fold_f64 into
 // gosa[it].  The sum over a warp takes 5 FP64 instructions, as many as 5 points' operations: one plane per
-// thread spent 39 instructions per point, 33 without the sum, this 35.5.
-constexpr int HK = 4;
+// thread spent 39 instructions per point, 33 without the sum, this 35.5 with 4.
 __global__ void __launch_bounds__(NT) himeno_f64(CoefF64 cf, const double* __restrict__ p, double* __restrict__ w2, int nx, int ny, int nz, int px,
-                                                 int py, unsigned plane_blocks, double omega, double* __restrict__ partials)
+                                                 int py, int hk, unsigned plane_blocks, double omega, double* __restrict__ partials)
 {
     const gb::BlockId bid = gb::grid_wait();
     const unsigned zc = bid.x / plane_blocks;
@@ -81,9 +80,9 @@ __global__ void __launch_bounds__(NT) himeno_f64(CoefF64 cf, const double* __res
         unsigned row, col;
         place(q, nx, points, &row, &col);
         const long long sy = px, sz = (long long)px * py;
-        size_t c = (size_t)(1 + zc * HK) * sz + (size_t)(row + 1) * sy + col + 1;
+        size_t c = (size_t)(1 + zc * hk) * sz + (size_t)(row + 1) * sy + col + 1;
 #pragma unroll 1
-        for (int k = 1 + (int)zc * HK; k < 1 + (int)(zc + 1) * HK && k <= nz; k++, c += sz) {
+        for (int k = 1 + (int)zc * hk; k < 1 + (int)(zc + 1) * hk && k <= nz; k++, c += sz) {
             auto P = [&](int di, int dj, int dk) { return __ldg(p + c + di + dj * sy + dk * sz); };
             auto C = [&](int n) { return __ldg(cf.f[n] + c); };
             double s0 = __dmul_rn(C(0), P(1, 0, 0));
@@ -116,6 +115,27 @@ __global__ void __launch_bounds__(NT) himeno_f64(CoefF64 cf, const double* __res
         for (int o = NT / 64; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(0xffffffffu, s, o));
         if (t == 0) partials[bid.x] = s;
     }
+}
+
+// Planes per thread: more share a sum, but a small grid then has too few blocks.  The fullest SM's blocks follow one
+// another on its FP64 pipe, 2.5 us for a plane of a block and 0.5 for its sum.  Us per sweep with 1 / 2 / 3 / 4 planes,
+// with gosa (without, 1 is the fastest or as fast): 24^3 9.3 / 12.0 / 14.6 / 17.2; 33 x 33 x 65 15.3 / 17.1 / 14.7 / 17.3;
+// 300 x 24 x 24 21.8 / 23.0 / 22.4 / 27.3; 65^3 30.5 / 28.8 / 30.6 / 27.5; 64 x 64 x 128 48.5 / 45.4 / 46.8 / 48.7;
+// 100^3 84.6 / 81.2 / 81.6 / 82.7; 257 x 257 x 129 656 / 608 / 597 / 588; without 552 / 553 / 559 / 558.
+int planes_per_thread(size_t plane_blocks, int nz, bool gosa)
+{
+    const size_t sms = gb::sm_count();
+    int best = 1;
+    double cost = 1e30;
+    for (int hk = 1; hk <= 4; hk++) {
+        const size_t blocks = plane_blocks * ((nz + hk - 1) / hk);
+        const double c = (double)((blocks + sms - 1) / sms) * (2.5 * hk + (gosa ? 0.5 : 0.0));
+        if (c < cost) {
+            cost = c;
+            best = hk;
+        }
+    }
+    return best;
 }
 
 // One block folds n partials: each thread a contiguous run in order, then the runs in thread order.
@@ -198,7 +218,9 @@ int appfis_gb_himeno_f64(const double* const* coef, double* p, double* wrk2, int
         cf.f[n] = coef[n];
     }
     cudaStream_t st = gb::as_stream(stream);
-    const size_t pb = ((size_t)nx * ny + NT - 1) / NT, nblk = pb * ((nz + HK - 1) / HK);
+    const size_t pb = ((size_t)nx * ny + NT - 1) / NT;
+    const int hk = planes_per_thread(pb, nz, dev_gosa != nullptr);
+    const size_t nblk = pb * ((nz + hk - 1) / hk);
     if (nblk > 0x7fffffffu) return gb::fail(APPFIS_GB_EINVAL, "himeno_f64: grid too large");
     void* ws = nullptr;
     if (dev_gosa) GB_TRY(gb::workspace(gb::WS_F64_PARTIALS, sizeof(double) * nblk, &ws));
@@ -206,7 +228,7 @@ int appfis_gb_himeno_f64(const double* const* coef, double* p, double* wrk2, int
     double* buf[2] = {p, wrk2};
     int ci = 0;
     for (int it = 0; it < iters; it++, ci = 1 - ci) {
-        gb::launch(himeno_f64, (unsigned)nblk, NT, 0, st, cf, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, (unsigned)pb, omega, part);
+        gb::launch(himeno_f64, (unsigned)nblk, NT, 0, st, cf, buf[ci], buf[1 - ci], nx, ny, nz, pitch, ny + 2, hk, (unsigned)pb, omega, part);
         if (dev_gosa) gb::launch(fold_f64, 1, 1024, 0, st, part, nblk, dev_gosa + it);
     }
     GB_TRY(gb::launched("himeno_f64"));
