@@ -18,7 +18,7 @@
  *   - after the sweep, the grids named by GridsToUpdate get their periodic ghosts refreshed on
  *     the device (no pack / host copy / MPI round trip) and are swapped; with one rank and no
  *     periodic axis there is nothing to exchange, as in the reference.
- * Reductions run on the device in one deterministic launch (appfis_gb_reduce) and return the
+ * Reductions run on the device, deterministically (appfis_gb_reduce), and return the
  * value to the host like the reference's Execute*DReduceGPU (Runtime_CUDA.hpp:554-740), seeds
  * included (MAX starts from numeric_limits<T>::min()); the input grid is never overwritten.
  * The reference's GPU 1-D executor swaps the updated grids twice (Runtime_CUDA.hpp:295-296), a

@@ -10,7 +10,8 @@
 // (fluxes + update into the other state buffer), separated by grid barriers whose spin waits
 // are bounded (on timeout the kernel records an error and returns).  Per-domain scalars
 // (dt bits, simulated time, print index, step count) are double-buffered by step parity so no
-// block ever reads a value another block is writing in the same phase; one thread commits them.
+// block ever reads a value another block is writing in the same phase; one thread of block 0 per domain
+// commits them.
 #pragma once
 
 #include "flood_core.cuh"

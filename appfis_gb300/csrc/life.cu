@@ -13,9 +13,9 @@
 // The byte-per-cell sweep (life_u8_bulk) stages its rows in shared memory with bulk copies; the
 // one-generation bit-packed sweep (life_bits_sweep) marches down a strip of rows per warp,
 // keeping the row above / at / below in registers and exchanging the words at lane boundaries
-// with warp shuffles.  Runs of 4 or more bit-packed generations, and byte runs that are worth the
-// conversion to words and back, use life_bits_tb, which advances a region held in registers by up to 16
-// generations per launch.
+// with warp shuffles.  Runs of 3 or more bit-packed generations (while a stream is recorded: 16), and byte
+// runs that are worth the conversion to words and back, use life_bits_tb, which advances a region held in
+// registers by up to 16 generations per launch.
 #include "gb_common.cuh"
 #include "tma.cuh"
 
@@ -715,13 +715,26 @@ struct LifePlan {
 // Rows per band, and whether the words left over from whole columns go side by side: what takes the least time
 // with the tiles dealt to the SMs; the fullest SM's tiles follow one another on its logic pipe, 0.47 us per band
 // row (and 0.2) for 16 generations, whatever is resident together.  Tall bands compute less halo (45 rows:
-// 10%, 8: half, 5: four fifths), but a small grid needs many: 256^2 16.2 us for 64 generations with 5 rows against
-// 20.1 with 8, 1024 x 1000 18.3 with 6 against 20.6.  Measured with 11 lop3 a word, us per 64 generations with 8 / 16 / 24 /
-// 32 / 40 / 45 rows: 1024 x 1000 22 / 37 / 53 / 70 / 86 / 97; 2048^2 38 / 38 / 53 / 70 / 87 / 98; 4096^2 86 / 67 / 54 / 71 / 87 / 98;
-// 8192^2 262 / 192 / 191 / 193 / 163 / 184; 16384^2 985 / 665 / 613 / 573 / 555 / 541.  (Planes in shared memory, tiles of
-// 32 to 256 rows: 49, 66, 107, 211, 706.)  Side by side costs its warps scattered loads (1024 x 1000, where whole
-// columns leave SMs idle anyway: 20.6 against 23.9), so it has to save 0.8 us and 5% (16384^2, 4% fewer: 521
-// against 519), and half a column or more is a column.
+// 10%, 8: half, 5: four fifths), but a small grid needs many tiles, and a step in the fullest SM's tiles separates
+// neighbouring heights: us per 64 generations (four launches of 16), reference rule, in columns of their own,
+//   rows             5    6    7    8   10   12   14   16   18   20   22   24   26   28   30   33   36   39   41   43   45
+//   256^2           17   18   19   20   23   26   30   33   36   39   43   46   49   53   57   67   71   77   84   85   92
+//   1024 x 1000     26   19   19   21   24   28   31   35   38   41   45   48   51   56   60   70   74   82   89   90   98
+//   1440 x 1500     36   30   20   21   24   28   32   35   39   42   46   49   52   57   61   71   75   83   90   91   98
+//   2048^2          66   41   32   36   24   28   32   36   39   43   46   50   53   57   61   72   76   83   90   91   99
+//   3072 x 3000    106   65   58   50   42   49   33   36   39   43   46   50   53   58   62   72   76   84   91   92   99
+//   4096^2         177  112   85   80   60   71   57   64   71   78   48   51   54   58   62   73   77   84   92   93  100
+//   5760 x 6000    306  182  138  125   97   94   83   93  102   79   86   92   98  106  114  129   78   85   92   93  100
+//   8192^2         615  367  282  242  203  179  181  175  165  148  163  171  145  157  169  187  142  155  164  169  179
+//   11520 x 12000 1194  705  531  448  365  330  308  289  291  286  279  257  279  256  277  307  272  295  311  319  264
+//   15904 x 12000 1683  986  742  626  509  478  432  401  414  390  394  379  371  397  384  371  399  367  388  403  423
+//   16384^2       2431 1426 1070  906  743  675  632  595  573  562  550  542  547  546  545  553  537  517  545  565  519
+// (planes in shared memory, tiles of 32 to 256 rows: 1024 x 1000 49, 2048^2 66, 4096^2 107, 8192^2 211, 16384^2 706).
+// The rule takes the fastest of them, 45 rows at 11520 x 12000 within 3% of it; a run of 8 generations (two
+// launches of 4, more load than generations) within 9% (1024 x 1000 6.6 against 6.1 us, 4096^2 11.4 against 10.9).
+// Side by side costs its warps scattered loads (1024 x 1000, where whole columns leave SMs idle anyway: 20.6 against
+// 18.6 with 6 rows; 4096^2 with 20 rows 45.5, the fastest), so it has to save 0.8 us and 5% (16384^2, 4% fewer tiles with
+// 45 rows: 546 against 519; with 30 rows 510), and half a column or more is a column.
 LifePlan tb_plan(int nw, int ny)
 {
     const unsigned sms = gb::sm_count();

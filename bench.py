@@ -477,6 +477,13 @@ def run_ours(args, rank, world, local):
     u8_bytes = N * 3
     u8_achieved = u8_bytes / (u8_ms * 1e-3) / 1e9  # one sweep's compulsory bytes for each generation
 
+    def one_u8():  # a single generation is one sweep (what a recorded run takes for each, too)
+        gb.call("appfis_gb_life_u8", ua.data_ptr(), ub.data_ptr(), GOL_NX, GOL_NY, 1, 0, ctypes.byref(ci),
+                torch.cuda.current_stream(dev).cuda_stream)
+
+    sweep_ms = _time(torch, stream, one_u8, reps=20, warmup=3)
+    sweep_gbs = u8_bytes / (sweep_ms * 1e-3) / 1e9
+
     # end to end through the C ABI from pinned host buffers
     pop = ctypes.c_int64(0)
 
@@ -533,7 +540,10 @@ def run_ours(args, rank, world, local):
             "bits": {"glups": value, "ms_per_step": ms_bits, "kernel_ms": bits_ms, "achieved_gbs": bits_achieved},
             "u8": {"glups": N * gens / (ms_u8 * 1e-3) / 1e9 * world, "ms_per_step": ms_u8, "kernel_ms": u8_ms,
                    "kernel": "life_bits_tb (bytes to words and back around it)", "effective_gbs": u8_achieved,
-                   "bytes_per_lup": 3},
+                   "bytes_per_lup": 3,
+                   "one_generation": {"kernel": "life_u8_bulk", "ms": sweep_ms, "glups": N / (sweep_ms * 1e-3) / 1e9,
+                                      "achieved_gbs": sweep_gbs, "frac": sweep_gbs / hbm_peak,
+                                      "traffic": profiled_traffic("life_u8_bulk")}},
         },
         "clocks": clocks,
     }
@@ -986,8 +996,9 @@ def profile_small(name, torch, gb, W, dev, sp):
 
 def profile_case(name, local):
     """Short fixed launch sequences for ncu captures.
-    life:   16384^2 GameOfLife, 32 bit-packed generations (two life_bits_tb launches of 16) then 20 u8
-            generations (bytes to words, two life_bits_tb launches of 10, words to bytes)
+    life:   16384^2 GameOfLife, 32 bit-packed generations (two life_bits_tb launches of 16), 20 u8
+            generations (bytes to words, two life_bits_tb launches of 10, words to bytes), one u8
+            generation (life_u8_bulk)
     himeno: 257x257x513 (rows padded to 264), 5 plain sweeps (himeno_tma<0>), 5 mixed sweeps
             (himeno_tma<1>, himeno_correct)
     fdtd:   512^3, 5 FP32 steps then 5 FP16 steps (star_r4_tma), then 2 two-step launches in FP32
@@ -1030,6 +1041,7 @@ def profile_case(name, local):
     gb.call("appfis_gb_life_pack", cells.data_ptr(), wa.data_ptr(), GOL_NX, GOL_NY, sp)
     gb.call("appfis_gb_life_bits", wa.data_ptr(), wb.data_ptr(), GOL_NX, GOL_NY, 32, 0, ctypes.byref(ci), sp)
     gb.call("appfis_gb_life_u8", cells.data_ptr(), ub.data_ptr(), GOL_NX, GOL_NY, 20, 0, ctypes.byref(ci), sp)
+    gb.call("appfis_gb_life_u8", cells.data_ptr(), ub.data_ptr(), GOL_NX, GOL_NY, 1, 0, ctypes.byref(ci), sp)
     torch.cuda.synchronize(dev)
     print("profile case %s done" % name)
 

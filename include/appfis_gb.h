@@ -120,7 +120,8 @@ APPFIS_GB_API int appfis_gb_reduce_host(const void* field, int dtype, int px, in
 /* ----------------------------------------------------------------------------- halo */
 /* Periodic ghost refresh of a dense padded field (row pitch = padded_dims[0]) in place: the
  * single-rank form of Exchange for periodic grids (Appfis/Communication.hpp:612-678 with the
- * pack/unpack of Appfis/Runtime.hpp:916-1173), axis by axis over full faces so corners match.
+ * pack/unpack of Appfis/Runtime.hpp:916-1173); edges and corners as its axis-by-axis refresh over full
+ * faces leaves them, in one launch.
  * elem_size 1, 2, 4 or 8 bytes; each padded axis must be >= 3*ghost. */
 APPFIS_GB_API int appfis_gb_ghost_periodic(void* field, int elem_size, int ndim, const int* padded_dims, int ghost,
                                            void* stream);
@@ -268,8 +269,8 @@ APPFIS_GB_API int appfis_gb_star_r4_f64(double* a, double* b, int nx, int ny, in
 
 /* Autotuner of the radius-4 star (no counterpart in the reference): times every candidate kernel
  * for this shape on `stream` — on 16-byte rows the TMA-staged tiles (4 or 2 x points per thread,
- * one step per launch) and the two-step time-blocked tiles (64 x 16 / 64 x 8 outputs), else the
- * vector / scalar tiles — with z chunks of the tile's default and 32 .. 256 planes, each run
+ * one step per launch) and the two-step time-blocked tiles (64 x 16 / 64 x 8 outputs), else AUTO's
+ * own choice and the vector / scalar tiles — with z chunks of the tile's default and 32 .. 256 planes, each run
  * from a into b (b's interior is overwritten; a and the halos are not), and keeps the fastest
  * per device and shape (dtype, form, nx, ny, nz, pitch) for the process; later calls with
  * tile = APPFIS_GB_STAR_AUTO use it (zchunk 0 = the tuned chunk).  With APPFIS_GB_TUNE_FILE set
