@@ -55,6 +55,21 @@ __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c)
     return unpack(r);
 }
 
+// a + b == sum + err exactly, |err| at most half a unit in the last place of sum (Knuth's two-sum); one, and two at once.
+__device__ __forceinline__ float two_sum(float a, float b, float& err)
+{
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+
+__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& err)
+{
+    const float2 s = add(a, b), bb = sub(s, a);
+    err = add(sub(a, sub(s, bb)), sub(b, bb));
+    return s;
+}
+
 __device__ __forceinline__ float2 splat(float s) { return make_float2(s, s); }
 
 __device__ __forceinline__ float2 from_half2(__half2 h) { return __half22float2(h); }

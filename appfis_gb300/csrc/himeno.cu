@@ -131,45 +131,40 @@ struct SqAcc {
 // off is under 2^-65 of these positive terms' sum), and one warp takes the warps' sums to double: a double
 // shuffle tree per warp costs 8 FP64 instructions of 16 cycles each on this part, more than the sweep itself at
 // few planes per thread (65 x 65 x 129, us per sweep: 8.25, so 6.0).  Sums beyond the float range take it.
-__device__ __forceinline__ float two_sum(float a, float b, float& err)
-{
-    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    return s;
-}
-
 __device__ __forceinline__ void gosa_end_flat(const SqAcc& acc, const GosaIO& g, unsigned block)
 {
     if (g.part) {
         __shared__ float4 sh[8];  // hi, mid, lo, whether they hold the sum
         __shared__ double wide[8];
-        float hi = acc.hi, mid = acc.lo, lo = 0.0f;
+        float2 v = make_float2(acc.hi, acc.lo);  // hi, mid
+        float lo = 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            const float h2 = __shfl_down_sync(0xffffffffu, hi, o), m2 = __shfl_down_sync(0xffffffffu, mid, o);
-            const float l2 = __shfl_down_sync(0xffffffffu, lo, o);
-            float e, f, r;
-            hi = two_sum(hi, h2, e);
-            mid = two_sum(mid, m2, f);
-            mid = two_sum(mid, e, r);
-            lo = __fadd_rn(__fadd_rn(lo, l2), __fadd_rn(f, r));
+            const float2 v2 = make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o));
+            float2 e;
+            float r;
+            v = gb::f2::two_sum(v, v2, e);
+            v.y = gb::f2::two_sum(v.y, e.x, r);
+            const float rest = __fadd_rn(e.y, r);
+            lo = o == 16 ? rest : __fadd_rn(__fadd_rn(lo, __shfl_down_sync(0xffffffffu, lo, o)), rest);
         }
+        const float hi = v.x, mid = v.y;
         const int w = threadIdx.x >> 5;
         const bool held = fabsf(hi) <= FLT_MAX && fabsf(mid) <= FLT_MAX;
         if (!__shfl_sync(0xffffffffu, held, 0)) {
-            double v = acc.value();
+            double d = acc.value();
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((threadIdx.x & 31) == 0) wide[w] = v;
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
+            if ((threadIdx.x & 31) == 0) wide[w] = d;
         }
         if ((threadIdx.x & 31) == 0) sh[w] = make_float4(hi, mid, lo, held ? 1.0f : 0.0f);
         __syncthreads();
         if (threadIdx.x < 32) {
             const float4 q = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-            double v = q.w != 0.0f ? (double)q.x + ((double)q.y + (double)q.z) : wide[threadIdx.x];
+            double d = q.w != 0.0f ? (double)q.x + ((double)q.y + (double)q.z) : wide[threadIdx.x];
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);  // at most 8 warps
-            if (threadIdx.x == 0) g.part[block] = v;
+            for (int o = 4; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);  // at most 8 warps
+            if (threadIdx.x == 0) g.part[block] = d;
         }
     }
     if (g.prev && block == 0) gosa_fold(g);

@@ -72,20 +72,7 @@ __device__ __forceinline__ A block_reduce(A v, A neutral, A* sh)
     return v;
 }
 
-// a + b == sum + err exactly, |err| at most half a unit in the last place of sum (Knuth's two-sum); two at once.
-__device__ __forceinline__ float two_sum(float a, float b, float& err)
-{
-    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    return s;
-}
-__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& err)
-{
-    namespace f2 = gb::f2;
-    const float2 s = f2::add(a, b), bb = f2::sub(s, a);
-    err = f2::add(f2::sub(a, f2::sub(s, bb)), f2::sub(b, bb));
-    return s;
-}
+using gb::f2::two_sum;
 
 // A thread's running sum of floats, in two lanes: hi takes the element, mid what hi rounds off and lo what mid
 // rounds off.  Of n elements of a lane (n <= 64) and the sum S of their magnitudes, mid holds at most n 2^-24 S and
