@@ -250,6 +250,10 @@ int tensor_map_3d(CUtensorMap* map, CUtensorMapDataType type, size_t esize, cons
         cudaGetLastError();
     });
     if (!g_encode) return fail(APPFIS_GB_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    // a driver call: in a host thread that has made no runtime call yet there is no current context for it
+    int dev = 0;
+    GB_CUDA(cudaGetDevice(&dev));
+    GB_CUDA(cudaSetDevice(dev));
     if (!aligned16(base) || (pitch * esize) % 16 != 0)
         return fail(APPFIS_GB_EINVAL, "tensor map: base or row stride not 16-byte aligned");
     const cuuint64_t dims[3] = {dx, dy, dz};
