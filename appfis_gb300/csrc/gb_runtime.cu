@@ -119,8 +119,19 @@ void workspace_drop(int slot)
     g_dev[dev][slot] = Buf();
 }
 
+namespace {
+// While one lives, this thread's calls on streams that are not captured do not break a capture under way on
+// another stream, in this thread or in others (a capture in the default mode forbids allocations anywhere).
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
 bool scratch_alloc(size_t bytes, cudaStream_t st, void** out)
 {
+    BesideCaptures guard;
     int dev = 0;
     cudaMemPool_t pool = nullptr;
     if (cudaGetDevice(&dev) == cudaSuccess) {
@@ -144,7 +155,11 @@ bool scratch_alloc(size_t bytes, cudaStream_t st, void** out)
     return false;
 }
 
-void scratch_free(void* p, cudaStream_t st) { cudaFreeAsync(p, st); }
+void scratch_free(void* p, cudaStream_t st)
+{
+    BesideCaptures guard;
+    cudaFreeAsync(p, st);
+}
 
 bool capturing(cudaStream_t st)
 {
