@@ -46,7 +46,8 @@ struct Ctl {
     int steps[2][MAXD];
     unsigned bar_count;
     unsigned bar_gen;
-    int error;
+    int error;      // a wait that gave up (1) or misaligned staging memory (3): read on the way out of every barrier
+    int collapsed;  // a time step collapsed: read after the run only
     unsigned ticket[2];  // phase A strip hand-out, by step parity
     unsigned ticketb[2];  // phase B strip hand-out, by step parity
     unsigned wet[2], dry[2];  // strips listed for the next step of that parity (Params::order)
@@ -151,9 +152,7 @@ __device__ __forceinline__ bool is_active(const Ctl* ctl, int cur, int d, const 
 // no step) into the other half, and resets dtbits[slot], which the steps around this one do not use.
 // Block 0 does it at the step's start, one thread per domain: nobody reads that half before the next
 // grid barrier (in one thread at the step's end, domain after domain, it held up every step:
-// about 1 us a domain).  A collapsed step is no business of its: the error word is read on the way out of
-// every grid barrier, and a CTA that is slow to leave the one before this step would see it and go
-// without its strips (DomCtl::collapsed).
+// about 1 us a domain).
 __device__ __forceinline__ void commit(Ctl* ctl, int cur, int slot, int d, bool active, double dt, const Params& p, double big)
 {
     const double t = ctl->simtime[cur][d];
@@ -372,10 +371,12 @@ struct DomCtl {
 
 // The end of a step in which a domain's time step has collapsed (below 1e-9 of the step scale, or NaN): the other
 // domains have taken it, nothing follows.  Every CTA finds the collapse by itself, from the same minima
-// and scalars, so all leave here, each after its own strips and without a barrier.
+// and scalars, so all leave here, each after its own strips and without a barrier.  Ctl::error does not say so: it is
+// read on the way out of every grid barrier, and a CTA slow to leave the one before this step would see it
+// and go without its strips, however late in the step another sets it.
 __device__ __forceinline__ void end_collapsed(Ctl* ctl)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&ctl->error, 0, 2);
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->collapsed = 1;
 }
 
 // The order of step n (the first step has none listed: as numbered).
@@ -902,6 +903,7 @@ __global__ void flood_init_ctl(Ctl* ctl, Dom<T>* doms, const __grid_constant__ T
         ctl->bar_count = 0;
         ctl->bar_gen = 0;
         ctl->error = 0;
+        ctl->collapsed = 0;
         ctl->ticket[0] = ctl->ticket[1] = 0;
         ctl->ticketb[0] = ctl->ticketb[1] = 0;
         ctl->wet[0] = ctl->wet[1] = ctl->dry[0] = ctl->dry[1] = 0;

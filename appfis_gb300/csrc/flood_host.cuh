@@ -59,8 +59,7 @@ static __global__ void flood_results(const Ctl* ctl, int ndom, int* steps, doubl
         if (simtime) simtime[d] = ctl->simtime[0][d];
     }
     if (d == 0 && status)
-        *status = ctl->error == 0   ? APPFIS_GB_OK
-                  : ctl->error == 2 ? APPFIS_GB_ENUMERIC
+        *status = ctl->error == 0   ? (ctl->collapsed ? APPFIS_GB_ENUMERIC : APPFIS_GB_OK)
                   : ctl->error == 3 ? APPFIS_GB_ECUDA  // staging buffers misaligned: no step was taken
                                     : APPFIS_GB_ETIMEOUT;
 }

@@ -91,6 +91,21 @@ def test_collapse_by_a_source_after_a_step(gb, torch_cuda, dtype, flags):
             assert torch_cuda.equal(got[0][m], want[0][m]), m
 
 
+@pytest.mark.parametrize("side", [50, 300])
+@pytest.mark.parametrize("dtype,flags", FORMS)
+def test_the_collapsing_domain_first(gb, torch_cuda, dtype, flags, side):
+    """The first CTAs' strips are the collapsing domain's, so they are done at once, while others may still
+    be leaving the barrier before the step."""
+    two_phase = flags & _lib.FLOOD_TWO_PHASE or (dtype == _lib.F64 and not flags & _lib.FLOOD_FUSED)
+    want, _, _ = _run(gb, torch_cuda, [_healthy(side)], dtype, flags, 1)
+    dem, h, qx = [np.kron(a, np.ones((15, 20))) for a in _bad(1e13)]
+    for _ in range(10):
+        got, _, status = _run(gb, torch_cuda, [(dem, h, qx), _healthy(side)], dtype, flags, 5)
+        assert status == ENUMERIC
+        for m in ((0, 1, 2, 4) if two_phase else range(6)):
+            assert torch_cuda.equal(got[1][m], want[0][m]), m
+
+
 def test_the_next_run_is_none_the_worse(gb, torch_cuda):
     want, _, _ = _run(gb, torch_cuda, [_healthy(120)], _lib.F32, 0, 7)
     _run(gb, torch_cuda, [_healthy(120), _bad(1e13)], _lib.F32, 0, 5)
