@@ -74,10 +74,12 @@ constexpr unsigned long long SPIN_LIMIT = 1ull << 25;
 constexpr int STEP_CAP = 1000000;  // steps per domain when the caller sets no limit
 
 // Grid-wide barrier of the cooperative launch.  Every wait is bounded (`limit` polls, each with
-// a short sleep); a wait that gives up records error 1 and every CTA leaves its loop.  `skip`
+// a short sleep); a wait that gives up records error 1 and every CTA leaves its loop, all threads of a CTA
+// by the one look that its thread 0 takes.  `skip`
 // (testing only) makes this CTA wait without arriving, so that the barrier cannot complete.
 __device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned long long limit, bool skip = false)
 {
+    __shared__ int error;
     __syncthreads();
     if (threadIdx.x == 0) {
         volatile unsigned* vgen = &ctl->bar_gen;
@@ -99,9 +101,10 @@ __device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned long long limit,
             }
         }
         __threadfence();
+        error = *(volatile int*)&ctl->error;
     }
     __syncthreads();
-    return *(volatile int*)&ctl->error == 0;
+    return error == 0;
 }
 
 template <class T>

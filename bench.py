@@ -654,7 +654,7 @@ def _pad_x(t, pitch):
 
 def bench_himeno(torch, gb, W, dev, sp, hbm):
     """Both forms on rows padded to 264 elements (16-byte aligned FP16 and FP32 rows: the
-    TMA-staged kernels), plus one-sweep times of the register-prefetch kernels on the dense
+    TMA-staged kernels), plus one-sweep times of the flat sweep on the dense
     259-element rows for comparison."""
     c = W.HIMENO
     nx, ny, nz, it, om = c["nx"], c["ny"], c["nz"], c["iters"], c["omega"]
