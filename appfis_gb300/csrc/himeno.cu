@@ -215,7 +215,9 @@ __global__ void __launch_bounds__(256) himeno_finish(const float* __restrict__ P
 // (257 x 257 x 513: 0.75 of the copy rate).  Nothing is kept from plane to plane, so a CTA takes only CKZ = 6 of them,
 // and a point's coefficients are asked for before its sums.  Us per pass with 32 planes / 6 / 6 and the
 // coefficients first: 33 x 33 x 65 42 / 10 / 5.8; 65 x 65 x 129 47 / 12 / 9.4; 129 x 129 x 257 115 / 74 / 59; 257 x 257 x 513 498 / 496 / 414;
-// so with 2 / 4 / 8 / 16 planes: 65 x 65 x 129 8.7 / 9.7 / 9.9 / 14.0, with gosa 13.3 / 10.9 / 11.3 / 15.3; 257 x 257 x 513 434 / 418 / 415 / 422.
+// so with 2 / 4 / 8 / 16 planes: 65 x 65 x 129 8.7 / 9.7 / 9.9 / 14.0; 257 x 257 x 513 434 / 418 / 415 / 422.  Where gosa is asked
+// for it takes CKZ_GOSA = 32: a thread sums its squares in one float, and another number of them is another sum, in the
+// eighth digit: 33 x 33 x 65 24, 65 x 65 x 129 25, 129 x 129 x 257 69, 257 x 257 x 513 434.
 template <int BX, int BY, bool COPY>
 __global__ void __launch_bounds__(BX* BY) himeno_correct(Coef12 cf, const float* __restrict__ P, const __half* __restrict__ e,
                                                           float* __restrict__ Pn, __half* __restrict__ D,
@@ -1016,7 +1018,7 @@ __global__ void __launch_bounds__(RX* RY) himeno_correct_tma(const __grid_consta
     gosa_end<1>({k < k1 ? __longlong_as_double(0x7ff8000000000000ll) : (double)g}, gz);
 }
 
-constexpr int HBX = 32, HBY = 4, CKZ = 6;  // himeno_correct: threads and z planes per CTA
+constexpr int HBX = 32, HBY = 4, CKZ = 6, CKZ_GOSA = 32;  // himeno_correct: threads and z planes per CTA
 constexpr int HKZ = 32;  // z planes per CTA elsewhere (nz is split into equal chunks of at most HKZ planes)
 constexpr int TMA_S_PLAIN = 3;
 constexpr size_t FLAT_POINTS = 6000000;        // grids up to this take the flat FP32 sweep
@@ -1189,7 +1191,8 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
     if (sweeps_per_pass == 2) GB_CUDA(cudaMemsetAsync(hw, 0, sizeof(__half) * 13 * field, st));
     else GB_CUDA(cudaMemsetAsync(E[0], 0, sizeof(__half) * 2 * field, st));
     GB_CUDA(cudaMemsetAsync(p_work, 0, sizeof(float) * field, st));
-    dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, CKZ));
+    const int pkz = dev_gosa ? CKZ_GOSA : CKZ;
+    dim3 blk(HBX, HBY), grd(gb::ceil_div(nx, HBX), gb::ceil_div(ny, HBY), gb::ceil_div(nz, pkz));
     dim3 rblk(RX, RY);
     // TMA-staged inner sweeps (two points per thread) when the FP16 rows are 16-byte aligned
     // (pitch a multiple of 8)
@@ -1313,7 +1316,7 @@ int appfis_gb_himeno_mixed_ex(const float* const* coef, float* p, float* p_work,
                        Dd, E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, ckz, omega, inv_omega, gz, status);
         else
             gb::launch(first ? himeno_correct<HBX, HBY, true> : himeno_correct<HBX, HBY, false>, grd, blk, 0, st, cf, P[pc], E[ec], P[1 - pc], Dd,
-                       E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, CKZ, omega, inv_omega, gz);
+                       E[1 - ec], Hc, field, nx, ny, nz, pitch, ny + 2, pkz, omega, inv_omega, gz);
         first = false;
         pc = 1 - pc;
         ec = 1 - ec;

@@ -56,4 +56,4 @@ def test_rows_of_any_alignment(gb, torch_cuda, nx, ny, nz):
 def test_time(gb, torch_cuda):
     _, _, plain = _call(gb, torch_cuda, "plain", 65, 65, 129, 67, 20, 6)
     _, _, passes = _call(gb, torch_cuda, "mixed", 65, 65, 129, 67, 20, 6)
-    assert passes < 5 * plain, (passes, plain)  # 2 times; marching 32 planes 8 times
+    assert passes < 5 * plain, (passes, plain)  # 4 times; with the coefficients asked for one by one 8 times
